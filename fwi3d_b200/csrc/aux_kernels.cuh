@@ -387,15 +387,20 @@ __global__ void rbc_blobs_kernel(float *__restrict__ vp, int nzz, int nxx, int n
     }
 }
 
-// Stencil coefficient dt^2 v^2 / dh^2 of every cell, evaluated as
-// (v * v) * cvel exactly as the stencil kernels would, so reading it instead
-// of the velocity changes no result bit.
-__global__ void coeff_kernel(const float *__restrict__ vp, float *__restrict__ out, long long n, float cvel)
+// Stencil coefficient (v * v) * cvel = dt^2 v^2 / dh^2 of every updated cell of
+// the velocity slots, 0 on the 4-cell shell that is never updated.
+__global__ void coeff_kernel(const float *__restrict__ vp, float *__restrict__ out, int nzz, int nxx, int nyy,
+                             int ldz, int nslot, float cvel)
 {
+    const long long n = (long long)ldz * nxx * nyy * nslot;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
          c += (long long)gridDim.x * blockDim.x) {
+        const int i = (int)(c % ldz);
+        const long long r = c / ldz;
+        const int j = (int)(r % nxx), k = (int)(r / nxx % nyy);
+        const bool upd = i >= 4 && i < nzz - 4 && j >= 4 && j < nxx - 4 && k >= 4 && k < nyy - 4;
         const float v = vp[c];
-        out[c] = v * v * cvel;
+        out[c] = upd ? v * v * cvel : 0.0f;
     }
 }
 

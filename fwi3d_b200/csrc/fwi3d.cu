@@ -37,8 +37,13 @@ constexpr int kTileTX[kNumTiles] = {8, 16, 8, 8, 8, 8, 8, 16, 4, 4};
 constexpr int SHF = 8, SCF = 3;  // forward rings: halo slots, centre slots
 constexpr int SHB = 7, SCB = 3;  // backward rings
 
+// x rows per thread: two in the forward kernel, which shares the eight x
+// neighbour rows of a cell between both (10 instead of 14 shared-memory loads
+// per 4 cells); the backward kernel has no registers for it
 template <int I>
-using TileOf = Tile<kTileTZ4[I], kTileTX[I]>;
+using FwdTile = Tile<kTileTZ4[I], kTileTX[I], 2>;
+template <int I>
+using BwdTile = Tile<kTileTZ4[I], kTileTX[I], 1>;
 
 struct KInfo {
     const void *fn = nullptr;
@@ -49,7 +54,7 @@ struct KInfo {
 template <int I>
 KInfo fwd_info(bool abc)
 {
-    using T = TileOf<I>;
+    using T = FwdTile<I>;
     KInfo k;
     k.threads = T::NT;
     k.tz = T::TZ;
@@ -63,7 +68,7 @@ KInfo fwd_info(bool abc)
 template <int I>
 KInfo bwd_info(bool grad, bool dy)
 {
-    using T = TileOf<I>;
+    using T = BwdTile<I>;
     KInfo k;
     k.threads = T::NT;
     k.tz = T::TZ;
@@ -604,7 +609,7 @@ FwdLaunch make_fwd(fwi_ctx *c, int n, int tile, int nchunk, bool record)
         L.mh[b] = make_map(c->F[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz + 8, L.k.tx + 8);
         L.mq[b] = make_map(c->F[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz, L.k.tx);
     }
-    L.mv = make_map(c->vp.p, c->nzz, c->nxx, c->nyy, c->ldz, c->vel_slots, L.k.tz, L.k.tx);
+    L.mv = make_map(c->vc.p, c->nzz, c->nxx, c->nyy, c->ldz, c->vel_slots, L.k.tz, L.k.tx);
     FwdArgs &a = L.a;
     memset(&a, 0, sizeof a);
     a.nzz = c->nzz;
@@ -855,8 +860,8 @@ void update_coeff(fwi_ctx *c)
         c->vc.ensure(n);
         ++c->generation;
     }
-    coeff_kernel<<<grid_blocks((long long)n), 256, 0, c->stream>>>(c->vp.p, c->vc.p, (long long)n,
-                                                                  c->p.dt * c->p.dt * c->idh2);
+    coeff_kernel<<<grid_blocks((long long)n), 256, 0, c->stream>>>(c->vp.p, c->vc.p, c->nzz, c->nxx, c->nyy, c->ldz,
+                                                                   c->vel_slots, c->p.dt * c->p.dt * c->idh2);
     CK(cudaGetLastError());
     ++c->launches;
 }
@@ -874,6 +879,7 @@ void model_impl(fwi_ctx *c, const int *shots, int nshots, float *out, bool out_i
         upload_batch(c, t);
         if (c->shot_rbc)
             shot_pads(c, shots + s0, n, shots + s0 + n, std::min(c->B, nshots - s0 - n));
+        update_coeff(c);
         const int R = t.info.R;
         if (R) CK(cudaMemsetAsync(c->seis_tm.p, 0, (size_t)c->p.nt * R * sizeof(float), c->stream));
         start_forward(c, n);

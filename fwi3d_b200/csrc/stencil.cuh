@@ -20,6 +20,9 @@
 //
 // Tiling: a CTA owns a TZ x TX (z, x) column of one shot and walks a chunk of
 // y planes.  Thread (lz, lx) owns 4 consecutive z cells of row lx.
+//   - The forward kernel works on packed pairs of z cells and two x rows per
+//     thread, and keeps the y derivative as eight partial sums instead of a
+//     queue of nine values (push_y).
 //   - Stencil fields arrive plane by plane as (TZ+8) x (TX+8) halo tiles,
 //     TMA-loaded into a ring of SH shared-memory slots (plane y needs slots
 //     y..y+4 resident; the rest is prefetch).  z and x neighbours come from the
@@ -40,10 +43,11 @@ namespace fwi {
 
 __device__ unsigned int g_status;
 
-template <int TZ4_, int TX_>
+template <int TZ4_, int TX_, int R_>
 struct Tile {
-    static constexpr int TZ4 = TZ4_, TX = TX_;
-    static constexpr int NT = TZ4 * TX;          // threads
+    static constexpr int TZ4 = TZ4_, TX = TX_, R = R_;
+    static constexpr int NT = TZ4 * TX / R;      // threads: 4 z cells of R x rows each
+    static_assert(TX % R == 0, "a thread owns R whole rows");
     static constexpr int TZ = 4 * TZ4;           // z cells
     static constexpr int HZ = TZ + 8, HX = TX + 8;
     static constexpr int HALO_BYTES = HZ * HX * 4;
@@ -115,11 +119,149 @@ __global__ void bounded_wait_probe_kernel(uint64_t limit_ns)
 }
 
 // ---------------------------------------------------------------------------
+// Stencil on packed pairs of z cells (fma.rn.f32x2).
+// ---------------------------------------------------------------------------
+struct f2 {
+    unsigned long long v;
+};
+
+__device__ __forceinline__ f2 pk(float lo, float hi)
+{
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float lo(f2 a) { return __uint_as_float((unsigned)a.v); }
+__device__ __forceinline__ float hi(f2 a) { return __uint_as_float((unsigned)(a.v >> 32)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c)
+{
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b)
+{
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b)
+{
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f2 dup2(float x) { return pk(x, x); }
+
+// Four consecutive z cells.
+struct q4 {
+    f2 a, b;
+};
+__device__ __forceinline__ q4 ldq(const float *p)
+{
+    const ulonglong2 u = *reinterpret_cast<const ulonglong2 *>(p);
+    q4 r;
+    r.a.v = u.x;
+    r.b.v = u.y;
+    return r;
+}
+__device__ __forceinline__ void stq(float *p, const q4 &x)
+{
+    *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(x.a.v, x.b.v);
+}
+__device__ __forceinline__ q4 fma4(f2 w, const q4 &x, const q4 &c) { return {fma2(w, x.a, c.a), fma2(w, x.b, c.b)}; }
+__device__ __forceinline__ q4 fma4(const q4 &w, const q4 &x, const q4 &c)
+{
+    return {fma2(w.a, x.a, c.a), fma2(w.b, x.b, c.b)};
+}
+__device__ __forceinline__ q4 mul4(f2 w, const q4 &x) { return {mul2(w, x.a), mul2(w, x.b)}; }
+__device__ __forceinline__ q4 add4(const q4 &x, const q4 &y) { return {add2(x.a, y.a), add2(x.b, y.b)}; }
+__device__ __forceinline__ float get(const q4 &x, int e)
+{
+    return e == 0 ? lo(x.a) : (e == 1 ? hi(x.a) : (e == 2 ? lo(x.b) : hi(x.b)));
+}
+__device__ __forceinline__ q4 mk4(float e0, float e1, float e2, float e3) { return {pk(e0, e1), pk(e2, e3)}; }
+
+// The y derivatives of the planes in the making: when plane p arrives, its
+// value v enters the sums of planes p-4 .. p+4 with their tap weights.  s[k]
+// is the sum of plane p-4+k so far; the call returns the finished plane p-4
+// and moves every sum down by one plane, which costs nothing: each
+// multiply-add reads s[k+1] and writes s[k].
+__device__ __forceinline__ q4 push_y(q4 (&s)[8], const q4 &v)
+{
+    const q4 done = fma4(dup2(-W4), v, s[0]);
+    s[0] = fma4(dup2(W3), v, s[1]);
+    s[1] = fma4(dup2(-W2), v, s[2]);
+    s[2] = fma4(dup2(W1), v, s[3]);
+    s[3] = fma4(dup2(-W0), v, s[4]);
+    s[4] = fma4(dup2(W1), v, s[5]);
+    s[5] = fma4(dup2(-W2), v, s[6]);
+    s[6] = fma4(dup2(W3), v, s[7]);
+    s[7] = mul4(dup2(-W4), v);
+    return done;
+}
+
+// d += the z derivative of 4 cells c whose neighbours are m (4 below) and p (4
+// above).  Even distances are packed; odd distances straddle the pairs and
+// stay scalar, since building the straddling pairs would cost as many moves.
+__device__ __forceinline__ void add_dz(q4 &d, const q4 &m, const q4 &c, const q4 &p)
+{
+    q4 x = fma4(dup2(-W4), m, d);
+    x = fma4(dup2(-W4), p, x);
+    const float w[12] = {lo(m.a), hi(m.a), lo(m.b), hi(m.b), lo(c.a), hi(c.a),
+                         lo(c.b), hi(c.b), lo(p.a), hi(p.a), lo(p.b), hi(p.b)};
+    float y[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y[e] = fmaf(W3, w[e + 7], fmaf(W3, w[e + 1], get(x, e)));
+    x = mk4(y[0], y[1], y[2], y[3]);
+    x.a = fma2(dup2(-W2), c.b, fma2(dup2(-W2), m.b, x.a));
+    x.b = fma2(dup2(-W2), p.a, fma2(dup2(-W2), c.a, x.b));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y[e] = fmaf(W1, w[e + 5], fmaf(W1, w[e + 3], get(x, e)));
+    d = fma4(dup2(-W0), c, mk4(y[0], y[1], y[2], y[3]));
+}
+
+// x + z derivatives d of R neighbouring x rows (4 z cells each) of one plane,
+// and the rows' own values c.  H: the thread's first cell in the halo tile.
+template <class T>
+__device__ __forceinline__ void xz_d2(const float *H, q4 (&c)[T::R], q4 (&d)[T::R])
+{
+    constexpr int R = T::R;
+    q4 row[R + 8];  // rows -4 .. R+3
+#pragma unroll
+    for (int r = 0; r < R + 8; ++r) row[r] = ldq(H + (r - 4) * T::HZ);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        c[r] = row[r + 4];
+        q4 x = mul4(dup2(-W4), row[r]);
+        x = fma4(dup2(-W4), row[r + 8], x);
+        x = fma4(dup2(W3), row[r + 1], x);
+        x = fma4(dup2(W3), row[r + 7], x);
+        x = fma4(dup2(-W2), row[r + 2], x);
+        x = fma4(dup2(-W2), row[r + 6], x);
+        x = fma4(dup2(W1), row[r + 3], x);
+        x = fma4(dup2(W1), row[r + 5], x);
+        d[r] = fma4(dup2(-W0), c[r], x);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) add_dz(d[r], ldq(H + r * T::HZ - 4), c[r], ldq(H + r * T::HZ + 4));
+}
+
+// ---------------------------------------------------------------------------
 // Forward leapfrog step.
+// Bound by HBM: 4 shots of 301^3 padded cells take 0.282 ms a step, 6.19 TB/s
+// of 16 B per cell, 94 % of the 6.55 TB/s that a copy reaches (0.324 ms with
+// scalar arithmetic, one row per thread and a nine-deep y queue, which were
+// limited by instruction issue: 285 instead of about 110 instructions per 128
+// cells).  With damping, 201^3 cells take 36 us (73 us with the Cerjan factor
+// branched on per cell; here its z part sits in registers and the branch is on
+// the row).
 //   mh: halo-box map over A (the field read with the stencil)
 //   mq: centre-box map over Q (the field overwritten)
-//   mv: centre-box map over the velocity slots (one slot shared by every
-//       shot, or one slot per shot when every shot has its own random pad)
+//   mv: centre-box map over the stencil coefficients dt^2 v^2 / dh^2 of the
+//       velocity slots (one slot shared by every shot, or one slot per shot
+//       when every shot has its own random pad).  They are 0 on the cells
+//       that are never updated, which keeps those cells at 0.
 // ---------------------------------------------------------------------------
 template <class T, int SH, int SC, bool ABC>
 __global__ void __launch_bounds__(T::NT)
@@ -127,12 +269,12 @@ __global__ void __launch_bounds__(T::NT)
                       const __grid_constant__ CUtensorMap mv, const FwdArgs a)
 {
     static_assert(SH >= 5, "plane y needs halo slots y..y+4");
+    constexpr int R = T::R;
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char *hring = smem;
     unsigned char *cring = smem + SH * T::HSLOT;
     uint64_t *hbar = reinterpret_cast<uint64_t *>(cring + SC * 2 * T::CSLOT);
     uint64_t *cbar = hbar + SH;
-    __shared__ float b1s[ABC ? kMaxPad : 1];
     __shared__ int abort_flag;
 
     const int tid = threadIdx.x;
@@ -143,11 +285,11 @@ __global__ void __launch_bounds__(T::NT)
     // every launched thread takes part).  The reference records P after its
     // in-place damping, i.e. d * A (src/modeling/modeling.cu:378, 391-392).
     if (a.t > a.tlag) {
-        const int R = a.binfo->R;
+        const int nrec = a.binfo->R;
         const long long total = (long long)gridDim.x * gridDim.y * T::NT;
-        for (long long g = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * T::NT + tid; g < R;
+        for (long long g = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * T::NT + tid; g < nrec;
              g += total)
-            a.seis_tm[(long long)(a.t - a.tlag) * R + g] = a.rec_damp[g] * a.A[a.rec_cell[g]];
+            a.seis_tm[(long long)(a.t - a.tlag) * nrec + g] = a.rec_damp[g] * a.A[a.rec_cell[g]];
     }
 
     int b = blockIdx.x;
@@ -160,13 +302,10 @@ __global__ void __launch_bounds__(T::NT)
     const int yb = min(ya + a.ylen, a.nyy - 4);
     if (ya >= yb || shot >= a.binfo->nshot) return;  // uniform per CTA
 
-    const int lz = tid % T::TZ4, lx = tid / T::TZ4;
+    const int lz = tid % T::TZ4, lx = tid / T::TZ4 * R;
     const int zc = z0 + 4 * lz, xc = x0 + lx;
     const int vshot = a.vel_slots > 1 ? shot : 0;
 
-    if constexpr (ABC) {
-        for (int i = tid; i < a.nb; i += T::NT) b1s[i] = a.b1d[i];
-    }
     if (tid == 0) {
         abort_flag = 0;
         prefetch_tmap(&mh);
@@ -180,95 +319,154 @@ __global__ void __launch_bounds__(T::NT)
 
     const int pf = ya - 4, pl = yb + 3;  // halo planes loaded: [pf, pl]
     int h_issued = pf - 1, c_issued = ya - 1;  // meaningful in thread 0 only
-    auto issue_h = [&](int p) {
-        const int s = (p - pf) % SH;
+    auto issue_h = [&](int p, int s) {
         mbar_expect_tx(&hbar[s], T::HALO_BYTES);
         tma_load_4d(hring + s * T::HSLOT, &mh, &hbar[s], z0 - 4, x0 - 4, p, shot);
         h_issued = p;
     };
-    auto issue_c = [&](int y) {
-        const int s = (y - ya) % SC;
+    auto issue_c = [&](int y, int s) {
         mbar_expect_tx(&cbar[s], 2 * T::CTR_BYTES);
         tma_load_4d(cring + (2 * s) * T::CSLOT, &mq, &cbar[s], z0, x0, y, shot);
         tma_load_4d(cring + (2 * s + 1) * T::CSLOT, &mv, &cbar[s], z0, x0, y, vshot);
         c_issued = y;
     };
     if (tid == 0) {
-        for (int p = pf; p < pf + SH && p <= pl; ++p) issue_h(p);
-        for (int y = ya; y < ya + SC && y < yb; ++y) issue_c(y);
+        for (int p = pf; p < pf + SH && p <= pl; ++p) issue_h(p, p - pf);
+        for (int y = ya; y < ya + SC && y < yb; ++y) issue_c(y, y - ya);
+    }
+
+    // Cerjan factors of the thread's z cells, constant over the plane loop.
+    float bz[4] = {1.f, 1.f, 1.f, 1.f};
+    int zpad = 0;
+    if constexpr (ABC) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int d = zc + e < a.nzz ? pad_depth(zc + e, a.nzz, a.nb) : -1;
+            if (d >= 0) {
+                bz[e] = a.b1d[d];
+                zpad |= 1 << e;
+            }
+        }
+    }
+    float bx[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        bx[r] = -1.0f;  // outside the x pad
+        if constexpr (ABC) {
+            const int d = xc + r < a.nxx ? pad_depth(xc + r, a.nxx, a.nb) : -1;
+            if (d >= 0) bx[r] = a.b1d[d];
+        }
     }
 
     const int3 src = make_int3(a.binfo->src[shot][0], a.binfo->src[shot][1], a.binfo->src[shot][2]);
-    const int ro = (lx + 4) * T::HZ, zo = 4 + 4 * lz;
-    const bool row_ok = xc < a.nxx - 4 && zc < a.nzz - 4;
-    const int dx = ABC ? pad_depth(xc, a.nxx, a.nb) : -1;
-    float *Qshot = a.Q + (long long)shot * a.vol;
+    const int se = (src.x >= zc && src.x < zc + 4) ? src.x - zc : -1;  // source cell among this thread's
+    const int sr = (se >= 0 && src.y >= xc && src.y < xc + R) ? src.y - xc : -1;
+    const int ys = sr >= 0 && a.t + 1 < a.nt ? src.z : -1;
+    const int ho = (lx + 4) * T::HZ + 4 + 4 * lz, co = lx * T::TZ + 4 * lz;
+    const int nrow = zc < a.nzz - 4 ? min(R, a.nxx - 4 - xc) : 0;  // rows this thread writes
     const long long plane = (long long)a.ldz * a.nxx;
+    float *Qp = a.Q + (long long)shot * a.vol + (long long)ya * plane + (long long)xc * a.ldz + zc;
 
-    float4 q[9];
+    q4 s[R][8];
 #pragma unroll
-    for (int m = 0; m < 9; ++m) q[m] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int m = 0; m < 8; ++m) s[r][m] = mk4(0.f, 0.f, 0.f, 0.f);
 
+    // Ring positions: hs, hph = slot and phase parity of halo plane p; hy =
+    // slot of plane y = p - 4; cs, cph = slot and phase parity of centre plane y.
+    int hs = 0, hph = 0, hy = 0, cs = 0, cph = 0;
     for (int p = pf; p <= pl; ++p) {
         const int y = p - 4;
-        bool ok = mbar_wait(&hbar[(p - pf) % SH], ((p - pf) / SH) & 1);
-        if (y >= ya) ok = mbar_wait(&cbar[(y - ya) % SC], ((y - ya) / SC) & 1) && ok;
+        bool ok = mbar_wait(&hbar[hs], hph);
+        if (y >= ya) ok = mbar_wait(&cbar[cs], cph) && ok;
         if (!ok) abort_flag = 1;
 
-        const float *Hp = reinterpret_cast<const float *>(hring + ((p - pf) % SH) * T::HSLOT);
+        const float *Hp = reinterpret_cast<const float *>(hring + hs * T::HSLOT) + ho;
+        q4 dy[R];
 #pragma unroll
-        for (int m = 0; m < 8; ++m) q[m] = q[m + 1];
-        q[8] = lds4(Hp + ro + zo);
+        for (int r = 0; r < R; ++r) dy[r] = push_y(s[r], ldq(Hp + r * T::HZ));
 
         if (y >= ya) {
-            const float *Hy = reinterpret_cast<const float *>(hring + ((y - pf) % SH) * T::HSLOT);
-            const int cs = (y - ya) % SC;
-            const float *Cq = reinterpret_cast<const float *>(cring + (2 * cs) * T::CSLOT);
-            const float *Cv = reinterpret_cast<const float *>(cring + (2 * cs + 1) * T::CSLOT);
-            float ax[4], ay[4], az[4];
-            axis_d2<T>(Hy, ro, zo, q, ax, ay, az);
-            const float4 qo = lds4(Cq + lx * T::TZ + 4 * lz);
-            const float4 vv = lds4(Cv + lx * T::TZ + 4 * lz);
-            const int dy = ABC ? pad_depth(y, a.nyy, a.nb) : -1;
-            float4 out;
+            const float *Hy = reinterpret_cast<const float *>(hring + hy * T::HSLOT) + ho;
+            const float *Cq = reinterpret_cast<const float *>(cring + (2 * cs) * T::CSLOT) + co;
+            const float *Cv = reinterpret_cast<const float *>(cring + (2 * cs + 1) * T::CSLOT) + co;
+            q4 c[R], d[R];
+            xz_d2<T>(Hy, c, d);
+            float by = -1.0f;
+            if constexpr (ABC) {
+                const int dep = pad_depth(y, a.nyy, a.nb);
+                if (dep >= 0) by = a.b1d[dep];
+            }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float v = comp(vv, e);
-                const float cv = v * v * a.cvel;
-                const float lap = ax[e] + ay[e] + az[e];
-                const float p0 = comp(q[4], e);
-                float old = comp(qo, e);
-                float d = 1.0f;
+            for (int r = 0; r < R; ++r) {
+                const q4 lap = add4(d[r], dy[r]);
+                const q4 old = ldq(Cq + r * T::TZ), cv = ldq(Cv + r * T::TZ);
+                q4 out;
                 if constexpr (ABC) {
-                    d = cerjan(b1s, pad_depth(zc + e, a.nzz, a.nb), dx, dy);
-                    old = __fmul_rn(d, old);
+                    // b2d / b3d of the reference (modeling.cu:101-127) from
+                    // the 1-D table; which axes are in the pad is the same
+                    // for the whole row except along z
+                    float f[4];
+                    const bool px = bx[r] >= 0.0f, py = by >= 0.0f;
+                    if (px && py) {
+                        const float bxy = __fadd_rn(bx[r], by), n2 = __fsub_rn(bxy, 1.0f);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            f[e] = (zpad >> e) & 1
+                                       ? __fsub_rn(__fadd_rn(__fadd_rn(__fadd_rn(bz[e], bx[r]), bxy),
+                                                             __fadd_rn(bz[e], by)), 5.0f)
+                                       : n2;
+                    } else if (px || py) {
+                        const float b1 = px ? bx[r] : by;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            f[e] = (zpad >> e) & 1 ? __fsub_rn(__fadd_rn(bz[e], b1), 1.0f) : b1;
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) f[e] = bz[e];
+                    }
+                    const q4 f4 = mk4(f[0], f[1], f[2], f[3]), n4 = mk4(-f[0], -f[1], -f[2], -f[3]);
+                    out = fma4(cv, lap, fma4(n4, old, add4(c[r], c[r])));
+                    out = {mul2(f4.a, out.a), mul2(f4.b, out.b)};
+                } else {
+                    out = fma4(cv, lap, fma4(dup2(-1.0f), old, add4(c[r], c[r])));
                 }
-                float nv = fmaf(cv, lap, 2.0f * p0 - old);
-                if constexpr (ABC) nv = __fmul_rn(d, nv);
-                if (zc + e >= a.nzz - 4) nv = comp(qo, e);
-                set_comp(out, e, nv);
+                // Source sample t+1 goes into the new field, which is exactly where
+                // the reference adds it at the start of the next step
+                // (src/modeling/modeling.cu:347-348).
+                if (y == ys && r == sr) {
+                    const float add = a.idh3 * a.wavelet[a.t + 1];
+                    out = mk4(lo(out.a) + (se == 0 ? add : 0.f), hi(out.a) + (se == 1 ? add : 0.f),
+                              lo(out.b) + (se == 2 ? add : 0.f), hi(out.b) + (se == 3 ? add : 0.f));
+                }
+                if (r < nrow) stq(Qp + (long long)r * a.ldz, out);
             }
-            // Source sample t+1 goes into the new field, which is exactly where
-            // the reference adds it at the start of the next step
-            // (src/modeling/modeling.cu:347-348).
-            if (y == src.z && xc == src.y) {
-                const int e = src.x - zc;
-                if (e >= 0 && e < 4 && a.t + 1 < a.nt)
-                    set_comp(out, e, comp(out, e) + a.idh3 * a.wavelet[a.t + 1]);
-            }
-            if (row_ok)
-                *reinterpret_cast<float4 *>(Qshot + y * plane + (long long)xc * a.ldz + zc) = out;
+            Qp += plane;
         }
         __syncthreads();
         if (abort_flag) break;
         if (tid == 0) {
             fence_proxy_async();
             if (p < ya) {
-                if (p + SH <= pl) issue_h(p + SH);
+                if (p + SH <= pl) issue_h(p + SH, hs);
             } else if (y >= ya) {
-                if (y + SH <= pl) issue_h(y + SH);
-                if (y + SC < yb) issue_c(y + SC);
+                if (y + SH <= pl) issue_h(y + SH, hy);
+                if (y + SC < yb) issue_c(y + SC, cs);
             }
+        }
+        if (++hs == SH) {
+            hs = 0;
+            hph ^= 1;
+        }
+        if (y >= ya) {
+            if (++hy == SH) hy = 0;
+            if (++cs == SC) {
+                cs = 0;
+                cph ^= 1;
+            }
+        } else if (y == ya - 1) {
+            hy = 4 % SH;
         }
     }
 
