@@ -34,49 +34,68 @@ struct BatchInfo {
     int src[kMaxBatch][3];        // source cell (i=z, j=x, k=y), padded indices
 };
 
-// Forward step arguments (one leapfrog step of every shot of a batch).
+// Receivers of a batch by the column of the tiling that owns their cells:
+// entry u of column (shot, col) is one distinct cell, sorted by y plane; its
+// receivers are rid[first[u]] .. rid[first[u+1]-1].
+struct CellLists {
+    const int *col_first;         // [shots * columns + 1] first entry of each column
+    const long long *cell;        // batch-flat cell index
+    const int *y;                 // y plane of the cell
+    const int *first;             // [entries + 1]
+    const int *rid;
+};
+
+// Progress of the items of a time-loop kernel: an item is one step of one
+// column of one shot; it publishes the y planes it has stored.
+struct LoopProgress {
+    unsigned long long *ticket;   // next item
+    long long *done;              // [shot][step % ring][column]: step * nyy + planes stored
+    int ring;
+    int shots;                    // shots whose steps interleave in the ticket order
+};
+
+// Forward time loop arguments (all leapfrog steps of every shot of a batch).
 struct FwdArgs {
     int nzz, nxx, nyy, ldz;
     long long vol;                // device elements of one shot's field (pitched)
-    int ntz, ntx, ylen;           // z tiles, x tiles, planes per y chunk
-    int t, nt, tlag;              // step index, wavelet length, recording lag
-    float cvel;                   // dt^2 / dh^2
+    int ntz, ncol;                // z tiles, columns (z tiles x x tiles)
+    int nsteps, nt, tlag;         // steps, wavelet length, recording lag
     float idh3;                   // source / adjoint scaling 1/dh^3
     int nb;                       // pad width (damper tables)
     int vel_slots;                // 1: every shot reads velocity slot 0; B: shot s reads slot s
-    float *Q;                     // field written this step (batch base)
-    const float *A;               // field read with the stencil (batch base)
+    float *F[2];                  // field pair (batch base): step t reads F[t & 1], overwrites the other
     const float *b1d;             // Cerjan 1-D table (ABC only)
     const float *wavelet;         // [nt]
     const BatchInfo *binfo;
-    const long long *rec_cell;    // [R] batch-flat cell index of each receiver
+    CellLists rec;
     const float *rec_damp;        // [R] damping at the receiver (1 without ABC)
     float *seis_tm;               // [nt][R] time-major seismograms
+    LoopProgress prog;
 };
 
-// Fused backward step arguments (source rebuild + adjoint + imaging).
+// Backward time loop arguments (source rebuild + adjoint + imaging).
 struct BwdArgs {
     int nzz, nxx, nyy, ldz;
     long long vol;
-    int ntz, ntx, ylen;
-    int t, nt, nsteps;            // backward step index, wavelet length, N = nt + tlag
-    float cvel;                   // dt^2 / dh^2
-    float gscale;                 // dt / dh^2 (gradient imaging condition)
+    int ntz, ncol;
+    int nsteps, nt;               // N = nt + tlag, wavelet and data length
+    float gscale;                 // 1/dt (gradient imaging condition)
     float idh3;
     int subtract_src;             // remove the source while rebuilding Ps
     int vel_slots;                // 1: every shot reads velocity slot 0; B: shot s reads slot s
     int acc_z0, acc_z1;           // box [acc_z0, acc_z1) x [acc_x0, acc_x1) x [acc_y0, acc_y1)
     int acc_x0, acc_x1;           // of the cells whose image and illumination accumulate;
-    int acc_y0, acc_y1;           // the accumulators of every other cell are neither read nor written
-    int acc_zbox;                 // z extent of the accumulator tiles, from z = floor4(max(z0, acc_z0))
-    float *Ps;                    // rebuilt source field (written)
-    const float *Psold;           // source field read with the stencil
-    float *Prold;                 // adjoint field written
-    const float *Pr;              // adjoint field read with the stencil
+    int acc_y0, acc_y1;           // the accumulators of every other cell keep their values
+    int s0;                       // F[s0] holds the older of the two forward levels
+    float *F[2];                  // source field: step t reads F[(s0 + t) & 1], overwrites the other
+    float *Rf[2];                 // adjoint field: step t reads Rf[t & 1], overwrites the other
     float *image;                 // image or gradient accumulator (batch base)
     float *illum;                 // illumination accumulator (batch base)
     const float *wavelet;
     const BatchInfo *binfo;
+    CellLists inj;
+    const float *data_tm;         // [nt][R] observed data or residuals, time-major
+    LoopProgress prog;
 };
 
 // ---------------------------------------------------------------------------
@@ -102,6 +121,48 @@ __device__ __forceinline__ void fence_mbar_init()
 __device__ __forceinline__ void fence_proxy_async()
 {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// Generic-proxy accesses of global memory (another CTA's stores, made visible
+// by an acquire) before the TMA copies that follow.
+__device__ __forceinline__ void fence_proxy_async_global()
+{
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+}
+
+__device__ __forceinline__ long long ld_acquire_gpu(const long long *p)
+{
+    long long v;
+    asm volatile("ld.acquire.gpu.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void red_add(float *p, float v)
+{
+    asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+
+__device__ __forceinline__ void red_add4(float *p, float a, float b, float c, float d)
+{
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
+                 : "memory");
+}
+
+__device__ __forceinline__ void st_release_gpu(long long *p, long long v)
+{
+    asm volatile("st.release.gpu.global.s64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ int ld_acquire_cta(const int *p)
+{
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void st_release_cta(int *p, int v)
+{
+    asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_addr(p)), "r"(v) : "memory");
 }
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
@@ -283,21 +344,6 @@ __device__ __forceinline__ bool bar_and(int id, int count, bool pred)
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap *map)
 {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-}
-
-__device__ __forceinline__ float4 lds4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
-
-__device__ __forceinline__ float comp(const float4 &v, int e)
-{
-    return e == 0 ? v.x : (e == 1 ? v.y : (e == 2 ? v.z : v.w));
-}
-
-__device__ __forceinline__ void set_comp(float4 &v, int e, float s)
-{
-    if (e == 0) v.x = s;
-    else if (e == 1) v.y = s;
-    else if (e == 2) v.z = s;
-    else v.w = s;
 }
 
 // Distance into the pad along one axis, -1 inside (src/modeling/modeling.cu:408-431).

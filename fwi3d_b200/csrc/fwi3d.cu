@@ -2,7 +2,7 @@
 //
 // One translation unit: the stencil kernels (stencil.cuh), the small kernels
 // (aux_kernels.cuh) and the host runtime (context, device buffers, TMA
-// descriptors, shot batches, CUDA-graph time loops, tile autotuner).
+// descriptors, shot batches, time loops, tile autotuner).
 #include "../../include/fwi3d.h"
 
 #include <cudaTypedefs.h>
@@ -28,22 +28,26 @@ using namespace fwi;
 namespace {
 
 // ---------------------------------------------------------------------------
-// Tile table (z cells = 4*TZ4, x rows = TX).  The autotuner picks one entry
-// per context and kernel; every entry is compiled for both kernels.
+// Tile tables: z quads (cells = 4*TZ4), x rows, halo slots of the ring, CTAs per
+// SM, and the picoseconds a step takes per cell that the tiles cover on a busy
+// GPU (measured on 201^3 .. 483 x 483 x 283 cells).  A thread owns two x rows,
+// which share their eight x neighbours: 10 instead of 14 shared-memory loads
+// per 4 cells.  16 warps of 128 registers fill an SM, so the large tiles take
+// 14 compute warps or less and all the shared memory: halo slots beyond the
+// five in use are load-ahead, and one more of them took the backward step of
+// 301^3 cells from 0.166 to 0.143 ms.
 // ---------------------------------------------------------------------------
 constexpr int kNumTiles = 10;
-constexpr int kTileTZ4[kNumTiles] = {16, 16, 32, 24, 25, 37, 19, 8, 32, 49};
-constexpr int kTileTX[kNumTiles] = {8, 16, 8, 8, 8, 8, 8, 16, 4, 4};
-constexpr int SHF = 8, SCF = 3;  // forward rings: halo slots, centre slots
-constexpr int SHB = 7, SCB = 3;  // backward rings
-
-// x rows per thread: two in the forward kernel, which shares the eight x
-// neighbour rows of a cell between both (10 instead of 14 shared-memory loads
-// per 4 cells); the backward kernel has no registers for it
-template <int I>
-using FwdTile = Tile<kTileTZ4[I], kTileTX[I], 2>;
-template <int I>
-using BwdTile = Tile<kTileTZ4[I], kTileTX[I], 1>;
+struct TileSpec {
+    int tz4, tx, sh, ctas;
+    double cost;
+};
+constexpr TileSpec kFwdTiles[kNumTiles] = {
+    {16, 8, 7, 4, 2.78},  {19, 20, 7, 2, 3.00}, {32, 24, 7, 1, 2.24}, {24, 16, 7, 2, 2.70}, {25, 24, 9, 1, 2.56},
+    {37, 24, 7, 1, 2.19}, {37, 18, 8, 1, 2.29}, {12, 8, 8, 4, 3.24},  {25, 32, 7, 1, 2.66}, {49, 16, 7, 1, 2.55}};
+constexpr TileSpec kBwdTiles[kNumTiles] = {
+    {16, 12, 7, 2, 5.40}, {19, 22, 7, 1, 5.30}, {16, 28, 7, 1, 4.90}, {25, 14, 8, 1, 5.20}, {25, 16, 7, 1, 5.20},
+    {19, 18, 8, 1, 5.40}, {8, 8, 7, 4, 6.00},   {37, 10, 7, 1, 4.72}, {12, 16, 7, 2, 5.60}, {37, 8, 8, 1, 4.75}};
 
 struct KInfo {
     const void *fn = nullptr;
@@ -51,35 +55,41 @@ struct KInfo {
     size_t smem = 0;
 };
 
+// The kernel of a tile: `fields` halo fields and `centres` centre fields per stage.
+template <class T, int fields>
+KInfo tile_info(int sh, int centres)
+{
+    KInfo k;
+    k.threads = Loop<T, fields>::THREADS;
+    k.tz = T::TZ;
+    k.tx = T::TX;
+    k.smem = sh * fields * T::HSLOT + (sh - 4) * centres * T::CSLOT + (2 * sh - 4) * 8;
+    return k;
+}
+
 template <int I>
 KInfo fwd_info(bool abc)
 {
-    using T = FwdTile<I>;
-    KInfo k;
-    k.threads = T::NT;
-    k.tz = T::TZ;
-    k.tx = T::TX;
-    k.smem = SHF * T::HSLOT + SCF * 2 * T::CSLOT + (SHF + SCF) * 8;
-    k.fn = abc ? (const void *)fd_forward_kernel<T, SHF, SCF, true>
-               : (const void *)fd_forward_kernel<T, SHF, SCF, false>;
+    constexpr TileSpec S = kFwdTiles[I];
+    using T = Tile<S.tz4, S.tx, 2>;
+    KInfo k = tile_info<T, 1>(S.sh, 2);
+    k.fn = abc ? (const void *)fd_forward_kernel<T, S.sh, true, S.ctas>
+               : (const void *)fd_forward_kernel<T, S.sh, false, S.ctas>;
     return k;
 }
 
 template <int I>
 KInfo bwd_info(bool grad, bool dy)
 {
-    using T = BwdTile<I>;
-    KInfo k;
-    k.threads = T::NT;
-    k.tz = T::TZ;
-    k.tx = T::TX;
-    k.smem = SHB * 2 * T::HSLOT + SCB * 5 * T::CSLOT + (SHB + SCB) * 8;
+    constexpr TileSpec S = kBwdTiles[I];
+    using T = Tile<S.tz4, S.tx, 2>;
+    KInfo k = tile_info<T, 2>(S.sh, 3);
     if (!grad)
-        k.fn = (const void *)fd_backward_kernel<T, SHB, SCB, false, false>;
+        k.fn = (const void *)fd_backward_kernel<T, S.sh, false, false, S.ctas>;
     else if (dy)
-        k.fn = (const void *)fd_backward_kernel<T, SHB, SCB, true, true>;
+        k.fn = (const void *)fd_backward_kernel<T, S.sh, true, true, S.ctas>;
     else
-        k.fn = (const void *)fd_backward_kernel<T, SHB, SCB, true, false>;
+        k.fn = (const void *)fd_backward_kernel<T, S.sh, true, false, S.ctas>;
     return k;
 }
 
@@ -198,21 +208,6 @@ double stability_velocity(double dh, double dt)
     return 2.0 / std::sqrt(3.0 * S) * dh / dt;
 }
 
-struct GraphKey {
-    int kind, n, tile, nchunk, flags, vslots;
-    bool operator<(const GraphKey &o) const
-    {
-        return std::tie(kind, n, tile, nchunk, flags, vslots) <
-               std::tie(o.kind, o.n, o.tile, o.nchunk, o.flags, o.vslots);
-    }
-};
-
-struct Graph {
-    cudaGraphExec_t exec = nullptr;
-    int nodes = 0;
-    int generation = -1;
-};
-
 struct BlobKey {
     uint64_t seed = 0;
     float xm = 0, ym = 0, zm = 0, ratio = 0, varVp = 0, fnb = 0;
@@ -304,9 +299,11 @@ struct fwi_ctx {
     DevBuf<float> Rf[2];      // adjoint pair [B][vol]
     DevBuf<float> acc_img, acc_ill;  // accumulators [B][vol]
     DevBuf<float> seis_tm, data_tm, raw;
-    DevBuf<long long> rec_cell, inj_cell;
+    DevBuf<long long> inj_cell;
     DevBuf<float> rec_damp;
-    DevBuf<int> inj_first, inj_rid;
+    DevBuf<int> inj_first, inj_rid, inj_y, col_first;
+    DevBuf<unsigned long long> ticket;
+    DevBuf<long long> progress;
     DevBuf<BatchInfo> binfo;
     DevBuf<double> partial, dsum;
     DevBuf<unsigned int> ubits;
@@ -321,7 +318,6 @@ struct fwi_ctx {
     bool shot_rbc = false;
     fwi_rbc shot_rbc_params{};
     uint64_t shot_rbc_seed = 0;
-    int generation = 0;  // bumped whenever a buffer a graph points at moves
     bool acc_dirty = false;
 
     // geometry (padded grid indices)
@@ -331,8 +327,7 @@ struct fwi_ctx {
     int nsrc = 0, nrec = 0;
 
     // tuning
-    int tile_fwd = -1, tile_bwd = -1, chunk_fwd = 0, chunk_bwd = 0;
-    std::map<GraphKey, Graph> graphs;
+    int tile_fwd = -1, tile_bwd = -1;
     std::vector<float> b1d_host;
 };
 
@@ -432,43 +427,37 @@ float host_cerjan(const fwi_ctx *c, int i, int j, int k)
 void ensure_fields(fwi_ctx *c, bool adjoint)
 {
     const size_t n = (size_t)c->B * c->vol;
-    bool moved = false;
-    for (int k = 0; k < 2; ++k) {
-        if (c->F[k].n < n) moved = true;
-        c->F[k].ensure(n);
-    }
+    for (auto &f : c->F) f.ensure(n);
     if (adjoint) {
-        for (int k = 0; k < 2; ++k) {
-            if (c->Rf[k].n < n) moved = true;
-            c->Rf[k].ensure(n);
-        }
+        for (auto &f : c->Rf) f.ensure(n);
         if (c->acc_img.n < n) {
-            moved = true;
             c->acc_img.ensure(n);
             c->acc_ill.ensure(n);
             CK(cudaMemsetAsync(c->acc_img.p, 0, n * sizeof(float), c->stream));
             CK(cudaMemsetAsync(c->acc_ill.p, 0, n * sizeof(float), c->stream));
         }
     }
-    if (moved) ++c->generation;
 }
 
-// Per-batch shot tables: sources, receivers (flat cells, damping) and the
-// distinct receiver cells with their receivers (injection lists).
+// Per-batch shot tables: sources, receiver damping and the distinct receiver
+// cells with their receivers, listed by the column of the tiling that owns
+// them and within a column by (y, x, z).
 struct BatchTables {
     BatchInfo info{};
-    std::vector<long long> cell;
     std::vector<float> damp;
     std::vector<long long> ucell;
-    std::vector<int> ufirst, urid;
+    std::vector<int> ufirst, urid, uy, col_first;
     std::vector<int> shot_nrec;
 };
 
-BatchTables build_batch(fwi_ctx *c, const int *shots, int n)
+// tz x tx: cells of a column of the kernel that uses the lists.
+BatchTables build_batch(fwi_ctx *c, const int *shots, int n, int tz, int tx)
 {
     BatchTables t;
     t.info.nshot = n;
     const bool abc = c->p.boundary == FWI_BOUNDARY_ABC;
+    const int ntz = (c->nzz - 8 + tz - 1) / tz, ntx = (c->nxx - 8 + tx - 1) / tx, ncol = ntz * ntx;
+    std::vector<long long> cell, key;  // key: (shot, column, cell), the order of the lists
     for (int s = 0; s < n; ++s) {
         const int id = shots[s];
         if (id < 0 || id >= c->nsrc) fail(FWI_ERR_ARG, "shot %d out of range [0,%d)", id, c->nsrc);
@@ -477,64 +466,64 @@ BatchTables build_batch(fwi_ctx *c, const int *shots, int n)
         t.shot_nrec.push_back(m);
         for (int r = f; r < f + m; ++r) {
             const int i = c->rijk[3 * r], j = c->rijk[3 * r + 1], k = c->rijk[3 * r + 2];
-            t.cell.push_back((long long)s * c->vol + i + (long long)j * c->ldz + (long long)k * c->ldz * c->nxx);
+            const long long in_shot = i + (long long)j * c->ldz + (long long)k * c->ldz * c->nxx;
+            const long long col = (long long)s * ncol + (i - 4) / tz + (j - 4) / tx * ntz;
+            cell.push_back((long long)s * c->vol + in_shot);
+            key.push_back(col * c->vol + in_shot);
             t.damp.push_back(abc ? host_cerjan(c, i, j, k) : 1.0f);
         }
     }
-    t.info.R = (int)t.cell.size();
+    t.info.R = (int)cell.size();
     std::vector<int> order(t.info.R);
     for (int r = 0; r < t.info.R; ++r) order[r] = r;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return t.cell[a] < t.cell[b]; });
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key[a] < key[b]; });
+    t.col_first.assign((size_t)n * ncol + 1, 0);
     for (int q = 0; q < t.info.R; ++q) {
         const int r = order[q];
-        if (t.ucell.empty() || t.ucell.back() != t.cell[r]) {
-            t.ucell.push_back(t.cell[r]);
+        if (t.ucell.empty() || t.ucell.back() != cell[r]) {
+            t.ucell.push_back(cell[r]);
             t.ufirst.push_back(q);
+            t.uy.push_back((int)(cell[r] % c->vol / ((long long)c->ldz * c->nxx)));
+            ++t.col_first[key[r] / c->vol + 1];
         }
         t.urid.push_back(r);
     }
+    for (size_t q = 1; q < t.col_first.size(); ++q) t.col_first[q] += t.col_first[q - 1];
     t.ufirst.push_back(t.info.R);
     t.info.ncell = (int)t.ucell.size();
     return t;
 }
 
+CellLists cell_lists(const fwi_ctx *c)
+{
+    return {c->col_first.p, c->inj_cell.p, c->inj_y.p, c->inj_first.p, c->inj_rid.p};
+}
+
 void upload_batch(fwi_ctx *c, const BatchTables &t)
 {
     const int R = std::max(t.info.R, 1);
-    if (c->rec_cell.n < (size_t)R || c->inj_first.n < (size_t)R + 1) {
-        c->rec_cell.ensure(R);
-        c->rec_damp.ensure(R);
-        c->inj_cell.ensure(R);
-        c->inj_first.ensure(R + 1);
-        c->inj_rid.ensure(R);
-        ++c->generation;
-    }
+    c->rec_damp.ensure(R);
+    c->inj_cell.ensure(R);
+    c->inj_y.ensure(R);
+    c->inj_first.ensure(R + 1);
+    c->inj_rid.ensure(R);
+    c->col_first.ensure(t.col_first.size());
     const size_t need = (size_t)c->p.nt * R;
-    if (c->seis_tm.n < need || c->data_tm.n < need || c->raw.n < need) {
-        c->seis_tm.ensure(need);
-        c->data_tm.ensure(need);
-        c->raw.ensure(need);
-        ++c->generation;
-    }
+    c->seis_tm.ensure(need);
+    c->data_tm.ensure(need);
+    c->raw.ensure(need);
     c->binfo.ensure(1);
     CK(cudaMemcpyAsync(c->binfo.p, &t.info, sizeof(BatchInfo), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->col_first.p, t.col_first.data(), t.col_first.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     if (t.info.R) {
-        CK(cudaMemcpyAsync(c->rec_cell.p, t.cell.data(), t.info.R * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemcpyAsync(c->rec_damp.p, t.damp.data(), t.info.R * sizeof(float), cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemcpyAsync(c->inj_cell.p, t.ucell.data(), t.ucell.size() * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
+        CK(cudaMemcpyAsync(c->inj_y.p, t.uy.data(), t.uy.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemcpyAsync(c->inj_first.p, t.ufirst.data(), t.ufirst.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemcpyAsync(c->inj_rid.p, t.urid.data(), t.urid.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     }
     // the host vectors die with t: make the copies complete before returning
     CK(cudaStreamSynchronize(c->stream));
-}
-
-// Number of z tiles, x tiles and the y chunk length for a tile / chunk count.
-void tiling(const fwi_ctx *c, const KInfo &k, int nchunk, int &ntz, int &ntx, int &ylen)
-{
-    ntz = (c->nzz - 8 + k.tz - 1) / k.tz;
-    ntx = (c->nxx - 8 + k.tx - 1) / k.tx;
-    ylen = (c->nyy - 8 + nchunk - 1) / nchunk;
 }
 
 void prepare_kernel(const KInfo &k)
@@ -546,38 +535,17 @@ void prepare_kernel(const KInfo &k)
                             (int)cudaSharedmemCarveoutMaxShared));
 }
 
-// Chunks along y so that the grid fills the GPU about twice per resident wave.
-int default_chunks(const fwi_ctx *c, const KInfo &k, int nshot)
-{
-    prepare_kernel(k);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.threads, k.smem);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    per_sm = std::max(per_sm, 1);
-    int ntz, ntx, ylen;
-    tiling(c, k, 1, ntz, ntx, ylen);
-    const long long cols = (long long)ntz * ntx * nshot;
-    const long long slots = (long long)per_sm * sms;
-    int nchunk = (int)std::max(1LL, (slots + cols - 1) / cols);
-    // keep at least ~24 planes per chunk so the 8-plane warm-up stays small
-    nchunk = std::min(nchunk, std::max(1, (c->nyy - 8) / 24));
-    return nchunk;
-}
-
-// Heuristic tile before tuning: least wasted z cells, then least x waste.
+// Tile before tuning: the one whose covered cells, updated or not, cost least.
+// Within 4 % of the best tile on 9 of 12 measured grids, at most 13 % off on
+// small ones, where the hand-over between steps counts more than the cells.
 int default_tile(const fwi_ctx *c, bool backward)
 {
     int best = 0;
     double best_cost = 1e30;
     for (int t = 0; t < kNumTiles; ++t) {
-        const int tz = 4 * kTileTZ4[t], tx = kTileTX[t];
-        const int nzi = c->nzz - 8, nxi = c->nxx - 8;
-        const double wz = (double)((nzi + tz - 1) / tz * tz) / nzi;
-        const double wx = (double)((nxi + tx - 1) / tx * tx) / nxi;
-        const double halo = (double)(tz + 8) * (tx + 8) / (tz * tx);
-        const double cost = wz * wx * (1.0 + (backward ? 0.30 : 0.15) * halo);
+        const TileSpec &s = (backward ? kBwdTiles : kFwdTiles)[t];
+        const int tz = 4 * s.tz4, ntz = (c->nzz - 8 + tz - 1) / tz, ntx = (c->nxx - 8 + s.tx - 1) / s.tx;
+        const double cost = s.cost * ntz * tz * ntx * s.tx;
         if (cost < best_cost) {
             best_cost = cost;
             best = t;
@@ -592,84 +560,107 @@ int default_tile(const fwi_ctx *c, bool backward)
 struct FwdLaunch {
     KInfo k;
     dim3 grid;
-    CUtensorMap mh[2], mq[2], mv;
+    FwdMaps m;
     FwdArgs a;
 };
 
-FwdLaunch make_fwd(fwi_ctx *c, int n, int tile, int nchunk, bool record)
+struct BwdLaunch {
+    KInfo k;
+    dim3 grid;
+    BwdMaps m;
+    BwdArgs a;
+};
+
+// Columns, progress counters and grid of a time loop over n shots: one wave of
+// resident CTAs at most.
+template <class L>
+void plan_loop(fwi_ctx *c, L &l, int n)
+{
+    prepare_kernel(l.k);
+    const int ntz = (c->nzz - 8 + l.k.tz - 1) / l.k.tz, ntx = (c->nxx - 8 + l.k.tx - 1) / l.k.tx;
+    l.a.ntz = ntz;
+    l.a.ncol = ntz * ntx;
+    int per_sm = 0, dev = 0, sms = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, l.k.fn, l.k.threads, l.k.smem));
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int ctas = std::max(per_sm, 1) * sms;
+    // steps of one column that can be in flight: a step follows the one
+    // before at four planes at least, and in practice at about twelve
+    const int steps = std::max(1, (c->nyy - 8) / 12);
+    LoopProgress &p = l.a.prog;
+    p.ring = c->nyy / 4 + 3;
+    // one shot after the other keeps its fields in L2 as far as they fit; as
+    // many side by side as it takes to occupy the GPU
+    p.shots = std::min(n, std::max(1, (ctas + l.a.ncol * steps - 1) / (l.a.ncol * steps)));
+    l.grid = dim3(std::min<long long>(ctas, (long long)p.shots * l.a.ncol * (c->nyy / 4 + 1)));
+    c->ticket.ensure(1);
+    c->progress.ensure((size_t)n * p.ring * l.a.ncol);
+    p.ticket = c->ticket.p;
+    p.done = c->progress.p;
+}
+
+// All steps of a batch of n shots in one launch.
+template <class L>
+void launch_loop(fwi_ctx *c, L &l, int n)
+{
+    CK(cudaMemsetAsync(l.a.prog.ticket, 0, sizeof(unsigned long long), c->stream));
+    CK(cudaMemsetAsync(l.a.prog.done, 0, (size_t)n * l.a.prog.ring * l.a.ncol * sizeof(long long), c->stream));
+    void *args[] = {&l.m, &l.a};
+    CK(cudaLaunchKernel(l.k.fn, l.grid, dim3(l.k.threads), args, l.k.smem, c->stream));
+    ++c->launches;
+}
+
+FwdLaunch make_fwd(fwi_ctx *c, int n, int tile, bool record)
 {
     FwdLaunch L;
     const bool abc = c->p.boundary == FWI_BOUNDARY_ABC;
     L.k = fwd_kernel(tile, abc);
-    prepare_kernel(L.k);
-    int ntz, ntx, ylen;
-    tiling(c, L.k, nchunk, ntz, ntx, ylen);
-    L.grid = dim3(ntz * ntx * nchunk, n, 1);
-    for (int b = 0; b < 2; ++b) {
-        L.mh[b] = make_map(c->F[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz + 8, L.k.tx + 8);
-        L.mq[b] = make_map(c->F[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz, L.k.tx);
-    }
-    L.mv = make_map(c->vc.p, c->nzz, c->nxx, c->nyy, c->ldz, c->vel_slots, L.k.tz, L.k.tx);
     FwdArgs &a = L.a;
     memset(&a, 0, sizeof a);
+    plan_loop(c, L, n);
+    for (int b = 0; b < 2; ++b) {
+        L.m.mh[b] = make_map(c->F[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz + 8, L.k.tx + 8);
+        L.m.mq[b] = make_map(c->F[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz, L.k.tx);
+        a.F[b] = c->F[b].p;
+    }
+    L.m.mv = make_map(c->vc.p, c->nzz, c->nxx, c->nyy, c->ldz, c->vel_slots, L.k.tz, L.k.tx);
     a.nzz = c->nzz;
     a.nxx = c->nxx;
     a.nyy = c->nyy;
     a.ldz = c->ldz;
     a.vol = c->vol;
-    a.ntz = ntz;
-    a.ntx = ntx;
-    a.ylen = ylen;
+    a.nsteps = c->nsteps;
     a.nt = c->p.nt;
     a.tlag = record ? c->tlag : (1 << 30);
-    a.cvel = c->p.dt * c->p.dt * c->idh2;
     a.idh3 = c->idh3;
     a.nb = c->g.nb;
     a.vel_slots = c->vel_slots;
     a.b1d = abc ? c->b1d.p : nullptr;
     a.wavelet = c->wavelet.p;
     a.binfo = c->binfo.p;
-    a.rec_cell = c->rec_cell.p;
+    a.rec = cell_lists(c);
     a.rec_damp = c->rec_damp.p;
     a.seis_tm = c->seis_tm.p;
     return L;
 }
 
-void launch_fwd(fwi_ctx *c, FwdLaunch &L, int t, int cur)
-{
-    FwdArgs a = L.a;
-    a.t = t;
-    a.A = c->F[cur].p;
-    a.Q = c->F[1 - cur].p;
-    void *args[] = {&L.mh[cur], &L.mq[1 - cur], &L.mv, &a};
-    CK(cudaLaunchKernel(L.k.fn, L.grid, dim3(L.k.threads), args, L.k.smem, c->stream));
-}
-
-struct BwdLaunch {
-    KInfo k;
-    dim3 grid;
-    CUtensorMap mhs[2], mhr[2], mcs[2], mcr[2], mv, mim, mil;
-    BwdArgs a;
-};
-
-BwdLaunch make_bwd(fwi_ctx *c, int n, int tile, int nchunk, bool grad)
+BwdLaunch make_bwd(fwi_ctx *c, int n, int tile, bool grad)
 {
     BwdLaunch L;
     L.k = bwd_kernel(tile, grad, (c->p.flags & FWI_FLAG_GRAD_DY) != 0);
-    prepare_kernel(L.k);
-    int ntz, ntx, ylen;
-    tiling(c, L.k, nchunk, ntz, ntx, ylen);
-    L.grid = dim3(ntz * ntx * nchunk, n, 1);
-    for (int b = 0; b < 2; ++b) {
-        L.mhs[b] = make_map(c->F[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz + 8, L.k.tx + 8);
-        L.mhr[b] = make_map(c->Rf[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz + 8, L.k.tx + 8);
-        L.mcs[b] = make_map(c->F[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz, L.k.tx);
-        L.mcr[b] = make_map(c->Rf[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz, L.k.tx);
-    }
-    // the gradient condition needs v^2 itself; the image condition only the coefficient
-    L.mv = make_map(grad ? c->vp.p : c->vc.p, c->nzz, c->nxx, c->nyy, c->ldz, c->vel_slots, L.k.tz, L.k.tx);
     BwdArgs &a = L.a;
     memset(&a, 0, sizeof a);
+    plan_loop(c, L, n);
+    for (int b = 0; b < 2; ++b) {
+        L.m.mhs[b] = make_map(c->F[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz + 8, L.k.tx + 8);
+        L.m.mhr[b] = make_map(c->Rf[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz + 8, L.k.tx + 8);
+        L.m.mcs[b] = make_map(c->F[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz, L.k.tx);
+        L.m.mcr[b] = make_map(c->Rf[b].p, c->nzz, c->nxx, c->nyy, c->ldz, n, L.k.tz, L.k.tx);
+        a.F[b] = c->F[b].p;
+        a.Rf[b] = c->Rf[b].p;
+    }
+    L.m.mv = make_map(c->vc.p, c->nzz, c->nxx, c->nyy, c->ldz, c->vel_slots, L.k.tz, L.k.tx);
     if (c->p.flags & FWI_FLAG_PAD_ACCUMULATE) {  // every updated cell
         a.acc_z0 = a.acc_x0 = a.acc_y0 = 4;
         a.acc_z1 = c->nzz - 4;
@@ -681,134 +672,52 @@ BwdLaunch make_bwd(fwi_ctx *c, int n, int tile, int nchunk, bool grad)
         a.acc_x1 = c->g.nb + c->g.nx;
         a.acc_y1 = c->g.nb + c->g.ny;
     }
-    // z extent of the accumulator tiles: the widest part of a z tile that
-    // reaches the box, from and to float4 boundaries (a multiple of 4 and at
-    // most tz, since every tile starts at a multiple of 4)
-    a.acc_zbox = 4;
-    for (int z0 = 4; z0 < c->nzz - 4; z0 += L.k.tz) {
-        const int lo = std::max(z0, a.acc_z0) & ~3, hi = (std::min(z0 + L.k.tz, a.acc_z1) + 3) & ~3;
-        if (lo < hi) a.acc_zbox = std::max(a.acc_zbox, hi - lo);
-    }
-    L.mim = make_map(c->acc_img.p, c->nzz, c->nxx, c->nyy, c->ldz, n, a.acc_zbox, L.k.tx);
-    L.mil = make_map(c->acc_ill.p, c->nzz, c->nxx, c->nyy, c->ldz, n, a.acc_zbox, L.k.tx);
     a.nzz = c->nzz;
     a.nxx = c->nxx;
     a.nyy = c->nyy;
     a.ldz = c->ldz;
     a.vol = c->vol;
-    a.ntz = ntz;
-    a.ntx = ntx;
-    a.ylen = ylen;
-    a.nt = c->p.nt;
     a.nsteps = c->nsteps;
-    a.cvel = c->p.dt * c->p.dt * c->idh2;
-    a.gscale = c->p.dt * c->idh2;
+    a.nt = c->p.nt;
+    a.gscale = 1.0f / c->p.dt;
     a.idh3 = c->idh3;
     a.subtract_src = (c->p.flags & FWI_FLAG_SUBTRACT_SOURCE) ? 1 : 0;
     a.vel_slots = c->vel_slots;
+    // the forward pass leaves u^N in F[N%2] and u^{N-1} in F[1-N%2]
+    a.s0 = 1 - (c->nsteps & 1);
     a.image = c->acc_img.p;
     a.illum = c->acc_ill.p;
     a.wavelet = c->wavelet.p;
     a.binfo = c->binfo.p;
+    a.inj = cell_lists(c);
+    a.data_tm = c->data_tm.p;
     return L;
-}
-
-void launch_bwd(fwi_ctx *c, BwdLaunch &L, int t, int scur, int rcur)
-{
-    BwdArgs a = L.a;
-    a.t = t;
-    a.Psold = c->F[scur].p;
-    a.Ps = c->F[1 - scur].p;
-    a.Pr = c->Rf[rcur].p;
-    a.Prold = c->Rf[1 - rcur].p;
-    void *args[] = {&L.mhs[scur], &L.mhr[rcur], &L.mcs[1 - scur], &L.mcr[1 - rcur],
-                    &L.mv,        &L.mim,       &L.mil,          &a};
-    CK(cudaLaunchKernel(L.k.fn, L.grid, dim3(L.k.threads), args, L.k.smem, c->stream));
-}
-
-void launch_inject(fwi_ctx *c, int t, int rcur)
-{
-    const int sample = c->p.nt - 1 - t;
-    inject_adjoint_kernel<<<64, 256, 0, c->stream>>>(c->Rf[rcur].p, c->binfo.p, c->inj_cell.p,
-                                                     c->inj_first.p, c->inj_rid.p, c->data_tm.p,
-                                                     sample, c->idh3);
-    CK(cudaGetLastError());
 }
 
 int tuned_fwd(fwi_ctx *c) { return c->tile_fwd >= 0 ? c->tile_fwd : default_tile(c, false); }
 int tuned_bwd(fwi_ctx *c) { return c->tile_bwd >= 0 ? c->tile_bwd : default_tile(c, true); }
 
-// ---------------------------------------------------------------------------
-// Time loops, captured once per (kind, batch size, tiles) as CUDA graphs.
-// kind 0: forward with receivers, 1: forward without, 2: backward image,
-// 3: backward gradient.  The fields start from the state the caller left.
-// ---------------------------------------------------------------------------
-Graph &time_loop_graph(fwi_ctx *c, int kind, int n)
+// The time loops, one launch each.  The fields start from the state the caller
+// left.
+void forward_loop(fwi_ctx *c, int n, bool record)
 {
-    const int tile = kind < 2 ? tuned_fwd(c) : tuned_bwd(c);
-    int nchunk = kind < 2 ? c->chunk_fwd : c->chunk_bwd;
-    if (nchunk <= 0)
-        nchunk = kind < 2 ? default_chunks(c, fwd_kernel(tile, c->p.boundary == FWI_BOUNDARY_ABC), n)
-                          : default_chunks(c, bwd_kernel(tile, kind == 3, false), n);
-    GraphKey key{kind, n, tile, nchunk, c->p.flags, c->vel_slots};
-    Graph &gr = c->graphs[key];
-    if (gr.exec && gr.generation == c->generation) return gr;
-    if (gr.exec) {
-        cudaGraphExecDestroy(gr.exec);
-        gr.exec = nullptr;
-    }
-    const int N = c->nsteps;
-    // descriptors, kernel attributes and occupancy queries before capture
-    FwdLaunch LF;
-    BwdLaunch LB;
-    if (kind < 2)
-        LF = make_fwd(c, n, tile, nchunk, kind == 0);
-    else
-        LB = make_bwd(c, n, tile, nchunk, kind == 3);
-    cudaGraph_t graph = nullptr;
-    CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    try {
-        int nodes = 0;
-        if (kind < 2) {
-            CK(cudaEventRecordWithFlags(c->ev[0], c->stream, cudaEventRecordExternal));
-            for (int t = 0; t < N; ++t) {
-                launch_fwd(c, LF, t, t & 1);
-                ++nodes;
-            }
-            CK(cudaEventRecordWithFlags(c->ev[1], c->stream, cudaEventRecordExternal));
-        } else {
-            // the forward pass leaves u^N in F[N%2] and u^{N-1} in F[1-N%2]
-            const int s0 = 1 - (N & 1);
-            CK(cudaEventRecordWithFlags(c->ev[2], c->stream, cudaEventRecordExternal));
-            for (int t = 0; t < N; ++t) {
-                const int scur = (s0 + t) & 1, rcur = t & 1;
-                if (t < c->p.nt) {
-                    launch_inject(c, t, rcur);
-                    ++nodes;
-                }
-                launch_bwd(c, LB, t, scur, rcur);
-                ++nodes;
-            }
-            CK(cudaEventRecordWithFlags(c->ev[3], c->stream, cudaEventRecordExternal));
-        }
-        gr.nodes = nodes;
-    } catch (...) {
-        cudaStreamEndCapture(c->stream, &graph);
-        if (graph) cudaGraphDestroy(graph);
-        throw;
-    }
-    CK(cudaStreamEndCapture(c->stream, &graph));
-    cudaError_t e = cudaGraphInstantiate(&gr.exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) fail(FWI_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
-    gr.generation = c->generation;
-    return gr;
+    FwdLaunch L = make_fwd(c, n, tuned_fwd(c), record);
+    CK(cudaEventRecord(c->ev[0], c->stream));
+    launch_loop(c, L, n);
+    CK(cudaEventRecord(c->ev[1], c->stream));
 }
 
-void run_graph(fwi_ctx *c, Graph &g)
+void backward_loop(fwi_ctx *c, int n, bool grad)
 {
-    CK(cudaGraphLaunch(g.exec, c->stream));
-    c->launches += g.nodes;
+    BwdLaunch L = make_bwd(c, n, tuned_bwd(c), grad);
+    CK(cudaEventRecord(c->ev[2], c->stream));
+    // adjoint source of step 0; the loop adds the others
+    inject_adjoint_kernel<<<64, 256, 0, c->stream>>>(c->Rf[0].p, c->binfo.p, c->inj_cell.p, c->inj_first.p,
+                                                     c->inj_rid.p, c->data_tm.p, c->p.nt - 1, c->idh3);
+    CK(cudaGetLastError());
+    ++c->launches;
+    launch_loop(c, L, n);
+    CK(cudaEventRecord(c->ev[3], c->stream));
 }
 
 // Zero both forward fields of the batch and add source sample 0.
@@ -852,13 +761,12 @@ void data_from_fortran(fwi_ctx *c, int R, const float *src, cudaStream_t st = nu
 void shot_pads(fwi_ctx *c, const int *ids, int n, const int *next, int n_next);
 
 // Stencil coefficients of the velocity slots in use, from their current
-// velocities (one grid-stride pass; a moved buffer invalidates the graphs).
+// velocities (one grid-stride pass).
 void update_coeff(fwi_ctx *c)
 {
     const size_t n = (size_t)c->vel_slots * c->vol;
     if (c->vc.n < n) {
         c->vc.ensure(n);
-        ++c->generation;
     }
     coeff_kernel<<<grid_blocks((long long)n), 256, 0, c->stream>>>(c->vp.p, c->vc.p, c->nzz, c->nxx, c->nyy, c->ldz,
                                                                    c->vel_slots, c->p.dt * c->p.dt * c->idh2);
@@ -875,7 +783,8 @@ void model_impl(fwi_ctx *c, const int *shots, int nshots, float *out, bool out_i
     size_t off = 0;
     for (int s0 = 0; s0 < nshots; s0 += c->B) {
         const int n = std::min(c->B, nshots - s0);
-        BatchTables t = build_batch(c, shots + s0, n);
+        const KInfo k = fwd_kernel(tuned_fwd(c), c->p.boundary == FWI_BOUNDARY_ABC);
+        BatchTables t = build_batch(c, shots + s0, n, k.tz, k.tx);
         upload_batch(c, t);
         if (c->shot_rbc)
             shot_pads(c, shots + s0, n, shots + s0 + n, std::min(c->B, nshots - s0 - n));
@@ -883,8 +792,7 @@ void model_impl(fwi_ctx *c, const int *shots, int nshots, float *out, bool out_i
         const int R = t.info.R;
         if (R) CK(cudaMemsetAsync(c->seis_tm.p, 0, (size_t)c->p.nt * R * sizeof(float), c->stream));
         start_forward(c, n);
-        Graph &g = time_loop_graph(c, 0, c->B);
-        run_graph(c, g);
+        forward_loop(c, n, true);
         const size_t cnt = (size_t)c->p.nt * R;
         if (R) {
             if (out_is_device) {
@@ -916,7 +824,8 @@ void migrate_impl(fwi_ctx *c, const int *shots, int nshots, const float *data, b
     size_t off = 0;
     for (int s0 = 0; s0 < nshots; s0 += c->B) {
         const int n = std::min(c->B, nshots - s0);
-        BatchTables t = build_batch(c, shots + s0, n);
+        const KInfo k = bwd_kernel(tuned_bwd(c), grad, false);
+        BatchTables t = build_batch(c, shots + s0, n, k.tz, k.tx);
         upload_batch(c, t);
         if (c->shot_rbc)
             shot_pads(c, shots + s0, n, shots + s0 + n, std::min(c->B, nshots - s0 - n));
@@ -941,14 +850,12 @@ void migrate_impl(fwi_ctx *c, const int *shots, int nshots, const float *data, b
             }
         }
         start_forward(c, n);
-        Graph &gf = time_loop_graph(c, 1, c->B);
-        run_graph(c, gf);
+        forward_loop(c, n, false);
         const size_t bytes = (size_t)n * c->vol * sizeof(float);
         CK(cudaMemsetAsync(c->Rf[0].p, 0, bytes, c->stream));
         CK(cudaMemsetAsync(c->Rf[1].p, 0, bytes, c->stream));
-        Graph &gb = time_loop_graph(c, grad ? 3 : 2, c->B);
         if (data_on_side) CK(cudaStreamWaitEvent(c->stream, c->ev_data, 0));
-        run_graph(c, gb);
+        backward_loop(c, n, grad);
         check_status(c);
         float ms = 0;
         CK(cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
@@ -1249,7 +1156,6 @@ void grow_velocity_slots(fwi_ctx *c, int n)
     }
     c->vp.release();
     c->vp = nv;
-    ++c->generation;
 }
 
 // Per-shot random pads of one batch (shots ids[0..n)).  The batch's blob sets
@@ -1318,8 +1224,8 @@ int fwi_num_tiles(int *n)
 int fwi_tile_shape(int tile, int *tz, int *tx)
 {
     if (tile < 0 || tile >= kNumTiles || !tz || !tx) return FWI_ERR_ARG;
-    *tz = 4 * kTileTZ4[tile];
-    *tx = kTileTX[tile];
+    *tz = 4 * kFwdTiles[tile].tz4;
+    *tx = kFwdTiles[tile].tx;
     return FWI_OK;
 }
 
@@ -1380,8 +1286,6 @@ int fwi_destroy(fwi_ctx *c)
 {
     if (!c) return FWI_ERR_ARG;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (auto &kv : c->graphs)
-        if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
     c->vp.release();
     c->vp_clean.release();
     c->vc.release();
@@ -1394,11 +1298,14 @@ int fwi_destroy(fwi_ctx *c)
     c->seis_tm.release();
     c->data_tm.release();
     c->raw.release();
-    c->rec_cell.release();
     c->rec_damp.release();
     c->inj_cell.release();
     c->inj_first.release();
     c->inj_rid.release();
+    c->inj_y.release();
+    c->col_first.release();
+    c->ticket.release();
+    c->progress.release();
     c->binfo.release();
     c->partial.release();
     c->dsum.release();
@@ -1859,8 +1766,8 @@ int fwi_set_tiles(fwi_ctx *c, int f, int b)
     return FWI_OK;
 }
 
-// Time every compiled tile (and two y-chunk counts) on a few steps of the
-// context's own fields and keep the fastest for each kernel.
+// Time every compiled tile on a few steps of the context's own fields and keep
+// the fastest for each kernel.
 int fwi_autotune(fwi_ctx *c)
 {
     if (!c) return FWI_ERR_ARG;
@@ -1869,7 +1776,7 @@ int fwi_autotune(fwi_ctx *c)
         const bool adj = c->p.boundary == FWI_BOUNDARY_RBC;
         ensure_fields(c, adj);
         std::vector<int> one(1, 0);
-        BatchTables t = build_batch(c, one.data(), 1);
+        BatchTables t = build_batch(c, one.data(), 1, 4, 4);
         t.info.nshot = c->B;  // every slot busy, like a full batch
         for (int s = 1; s < c->B; ++s)
             for (int a = 0; a < 3; ++a) t.info.src[s][a] = t.info.src[0][a];
@@ -1877,66 +1784,49 @@ int fwi_autotune(fwi_ctx *c)
         t.info.ncell = 0;
         upload_batch(c, t);
         update_coeff(c);
-        // Candidates: every compiled tile x three y-chunk counts.  Each is timed
-        // over kSteps launches after one warm launch, in two passes (the SM
-        // clock moves under the power cap during a sweep), and keeps its faster
-        // pass.  The heuristic default stays unless a candidate beats it by
-        // more than 1 %: a short window can favour whatever ran while the
-        // clock was high.
-        constexpr int kSteps = 12, kPasses = 2;
+        // Each tile is timed over kSteps steps after a warm launch, in two
+        // passes (the SM clock moves under the power cap during a sweep), and
+        // keeps its faster pass.  The heuristic default stays unless another
+        // beats it by more than 1 %: a short window can favour whatever ran
+        // while the clock was high.
+        constexpr int kSteps = 32, kPasses = 2;
         cudaEvent_t e0, e1;
         CK(cudaEventCreate(&e0));
         CK(cudaEventCreate(&e1));
-        struct Cand {
-            int tile, nchunk;
-            float ms;
-        };
-        auto tune = [&](bool backward, int &tile_out, int &chunk_out) {
-            std::vector<Cand> cands;
-            for (int tile = 0; tile < kNumTiles; ++tile) {
-                const KInfo k = backward ? bwd_kernel(tile, false, false) : fwd_kernel(tile, !adj);
-                const int base = default_chunks(c, k, c->B);
-                for (int nchunk : {base, std::max(1, base / 2), base * 2}) {
-                    bool dup = false;
-                    for (const Cand &q : cands) dup |= q.tile == tile && q.nchunk == nchunk;
-                    if (!dup) cands.push_back({tile, nchunk, 1e30f});
-                }
-            }
-            for (int pass = 0; pass < kPasses; ++pass) {
-                for (Cand &q : cands) {
+        auto tune = [&](bool backward) {
+            float ms[kNumTiles];
+            std::fill(ms, ms + kNumTiles, 1e30f);
+            auto timed = [&](auto &L) {
+                L.a.nsteps = std::min(kSteps, c->nsteps);
+                L.a.nt = 0;  // no sources, no adjoint data
+                launch_loop(c, L, c->B);
+                CK(cudaEventRecord(e0, c->stream));
+                launch_loop(c, L, c->B);
+                CK(cudaEventRecord(e1, c->stream));
+                CK(cudaEventSynchronize(e1));
+                float m = 0;
+                CK(cudaEventElapsedTime(&m, e0, e1));
+                return m;
+            };
+            for (int pass = 0; pass < kPasses; ++pass)
+                for (int tile = 0; tile < kNumTiles; ++tile) {
                     if (backward) {
-                        BwdLaunch L = make_bwd(c, c->B, q.tile, q.nchunk, false);
-                        launch_bwd(c, L, 0, 0, 0);
-                        CK(cudaEventRecord(e0, c->stream));
-                        for (int s = 0; s < kSteps; ++s) launch_bwd(c, L, 1, s & 1, s & 1);
+                        BwdLaunch L = make_bwd(c, c->B, tile, false);
+                        ms[tile] = std::min(ms[tile], timed(L));
                     } else {
-                        FwdLaunch L = make_fwd(c, c->B, q.tile, q.nchunk, false);
-                        launch_fwd(c, L, 0, 0);
-                        CK(cudaEventRecord(e0, c->stream));
-                        for (int s = 0; s < kSteps; ++s) launch_fwd(c, L, 1, s & 1);
+                        FwdLaunch L = make_fwd(c, c->B, tile, false);
+                        ms[tile] = std::min(ms[tile], timed(L));
                     }
-                    CK(cudaEventRecord(e1, c->stream));
-                    CK(cudaEventSynchronize(e1));
-                    float ms = 0;
-                    CK(cudaEventElapsedTime(&ms, e0, e1));
-                    q.ms = std::min(q.ms, ms);
-                    c->launches += kSteps + 1;
                 }
-            }
-            const Cand *best = &cands[0];
-            for (const Cand &q : cands)
-                if (q.ms < best->ms) best = &q;
+            int best = 0;
+            for (int tile = 1; tile < kNumTiles; ++tile)
+                if (ms[tile] < ms[best]) best = tile;
             const int dt = default_tile(c, backward);
-            const KInfo dk = backward ? bwd_kernel(dt, false, false) : fwd_kernel(dt, !adj);
-            const int dc = default_chunks(c, dk, c->B);
-            for (const Cand &q : cands)
-                if (q.tile == dt && q.nchunk == dc && q.ms <= best->ms * 1.01f) best = &q;
-            tile_out = best->tile;
-            chunk_out = best->nchunk;
+            return ms[dt] <= ms[best] * 1.01f ? dt : best;
         };
-        tune(false, c->tile_fwd, c->chunk_fwd);
+        c->tile_fwd = tune(false);
         if (adj) {
-            tune(true, c->tile_bwd, c->chunk_bwd);
+            c->tile_bwd = tune(true);
             // tuning ran the imaging condition on scratch data
             const size_t bytes = (size_t)c->B * c->vol * sizeof(float);
             CK(cudaMemsetAsync(c->acc_img.p, 0, bytes, c->stream));

@@ -1,11 +1,11 @@
 // stencil.cuh -- the two hot kernels of the wave-propagation path.
 //
-//   fd_forward_kernel   one leapfrog step of every shot of a batch:
+//   fd_forward_kernel   every leapfrog step of every shot of a batch:
 //                       Q <- d (dt^2 v^2 lap(A) + 2 A - d Q)   [+ source]
 //                       and the receiver samples of A
 //                       (reference: compute_pressure + compute_seismogram,
 //                        src/modeling/modeling.cu:324-393)
-//   fd_backward_kernel  the fused back-propagation step:
+//   fd_backward_kernel  every step of the fused back-propagation:
 //                       Ps    <- dt^2 v^2 lap(Psold) + 2 Psold - Ps  (source rebuilt)
 //                       Prold <- dt^2 v^2 lap(Pr) + 2 Pr - Prold      (adjoint)
 //                       illum += Ps^2 ; image += Ps Pr  or  the gradient term
@@ -18,24 +18,21 @@
 // on any axis are never written and stay 0 (the reference's stencil guard,
 // src/modeling/modeling.cu:350).
 //
-// Tiling: a CTA owns a TZ x TX (z, x) column of one shot and walks a chunk of
-// y planes.  Thread (lz, lx) owns 4 consecutive z cells of row lx.
-//   - The forward kernel works on packed pairs of z cells and two x rows per
-//     thread, and keeps the y derivative as eight partial sums instead of a
-//     queue of nine values (push_y).
+// Tiling: a CTA takes a TZ x TX (z, x) column of one step of one shot and walks
+// its y planes.  A thread owns 4 consecutive z cells of R neighbouring x rows.
+//   - Arithmetic is on packed pairs of z cells; the y derivative is kept as
+//     eight partial sums per cell (push_y).
 //   - Stencil fields arrive plane by plane as (TZ+8) x (TX+8) halo tiles,
-//     TMA-loaded into a ring of SH shared-memory slots (plane y needs slots
-//     y..y+4 resident; the rest is prefetch).  z and x neighbours come from the
-//     tile of plane y, y neighbours from a 9-deep register queue fed with the
-//     centre of plane y+4.
-//   - Centre-only fields (old time level, velocity, accumulators) arrive as
-//     TZ x TX tiles in a second ring of SC slots; the accumulators only
-//     where the tile meets the box of accumulated cells, and then only over
-//     the z range that meets it.
-//   - One elected thread issues every TMA copy; completion is tracked with
-//     mbarriers whose waits are bounded (kWaitLimitNs) and report through
-//     g_status instead of hanging.
+//     TMA-loaded into a ring of SH shared-memory slots (plane y needs the slots
+//     of planes y and y+4, and so those between; the rest is load-ahead).
+//   - Centre-only fields (old time level, coefficient) arrive as TZ x TX tiles
+//     in a second ring of SH - 4 slots.
+//   - One thread issues every TMA copy; completion is tracked with mbarriers
+//     whose waits are bounded (kWaitLimitNs) and report through g_status
+//     instead of hanging.
 #pragma once
+
+#include <type_traits>
 
 #include "device.cuh"
 
@@ -57,46 +54,6 @@ struct Tile {
     static_assert((HZ * 4) % 16 == 0, "TMA inner box must be a multiple of 16 bytes");
     static_assert(HZ <= 256 && HX <= 256, "TMA box dimension limit");
 };
-
-// Second derivative along one axis, without the 1/dh^2 factor, summed from the
-// outer taps inwards like the reference (src/modeling/modeling.cu:354-358).
-__device__ __forceinline__ float d2(float c, float m1, float p1, float m2, float p2, float m3,
-                                    float p3, float m4, float p4)
-{
-    float acc = -W4 * (m4 + p4);
-    acc = fmaf(W3, m3 + p3, acc);
-    acc = fmaf(-W2, m2 + p2, acc);
-    acc = fmaf(W1, m1 + p1, acc);
-    acc = fmaf(-W0, c, acc);
-    return acc;
-}
-
-// Per-axis second derivatives of 4 consecutive z cells of one thread.
-// H: halo tile of the plane (row stride HZ); q: register queue (q[4] = centre).
-template <class T>
-__device__ __forceinline__ void axis_d2(const float *H, int ro, int zo, const float4 (&q)[9],
-                                        float (&ax)[4], float (&ay)[4], float (&az)[4])
-{
-    const float4 zm = lds4(H + ro + zo - 4);
-    const float4 zp = lds4(H + ro + zo + 4);
-    const float4 c = q[4];
-    const float w[12] = {zm.x, zm.y, zm.z, zm.w, c.x, c.y, c.z, c.w, zp.x, zp.y, zp.z, zp.w};
-    float4 xm[4], xp[4];
-#pragma unroll
-    for (int m = 1; m <= 4; ++m) {
-        xm[m - 1] = lds4(H + ro - m * T::HZ + zo);
-        xp[m - 1] = lds4(H + ro + m * T::HZ + zo);
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const float c0 = w[4 + e];
-        ax[e] = d2(c0, comp(xm[0], e), comp(xp[0], e), comp(xm[1], e), comp(xp[1], e),
-                   comp(xm[2], e), comp(xp[2], e), comp(xm[3], e), comp(xp[3], e));
-        ay[e] = d2(c0, comp(q[3], e), comp(q[5], e), comp(q[2], e), comp(q[6], e), comp(q[1], e),
-                   comp(q[7], e), comp(q[0], e), comp(q[8], e));
-        az[e] = d2(c0, w[3 + e], w[5 + e], w[2 + e], w[6 + e], w[1 + e], w[7 + e], w[e], w[8 + e]);
-    }
-}
 
 __device__ __forceinline__ void raise_status(unsigned bits) { atomicOr(&g_status, bits); }
 
@@ -175,6 +132,7 @@ __device__ __forceinline__ q4 fma4(const q4 &w, const q4 &x, const q4 &c)
     return {fma2(w.a, x.a, c.a), fma2(w.b, x.b, c.b)};
 }
 __device__ __forceinline__ q4 mul4(f2 w, const q4 &x) { return {mul2(w, x.a), mul2(w, x.b)}; }
+__device__ __forceinline__ q4 mul4(const q4 &x, const q4 &y) { return {mul2(x.a, y.a), mul2(x.b, y.b)}; }
 __device__ __forceinline__ q4 add4(const q4 &x, const q4 &y) { return {add2(x.a, y.a), add2(x.b, y.b)}; }
 __device__ __forceinline__ float get(const q4 &x, int e)
 {
@@ -203,22 +161,25 @@ __device__ __forceinline__ q4 push_y(q4 (&s)[8], const q4 &v)
 
 // d += the z derivative of 4 cells c whose neighbours are m (4 below) and p (4
 // above).  Even distances are packed; odd distances straddle the pairs and
-// stay scalar, since building the straddling pairs would cost as many moves.
+// stay scalar, since building the straddling pairs would cost as many moves
+// (the packed ones first: one switch between pairs and scalars, 2 % fewer
+// instructions than outer to inner, and 7 % fewer than all scalar).
 __device__ __forceinline__ void add_dz(q4 &d, const q4 &m, const q4 &c, const q4 &p)
 {
-    q4 x = fma4(dup2(-W4), m, d);
-    x = fma4(dup2(-W4), p, x);
     const float w[12] = {lo(m.a), hi(m.a), lo(m.b), hi(m.b), lo(c.a), hi(c.a),
                          lo(c.b), hi(c.b), lo(p.a), hi(p.a), lo(p.b), hi(p.b)};
     float y[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) y[e] = fmaf(W3, w[e + 7], fmaf(W3, w[e + 1], get(x, e)));
-    x = mk4(y[0], y[1], y[2], y[3]);
+    q4 x = fma4(dup2(-W4), m, d);
+    x = fma4(dup2(-W4), p, x);
     x.a = fma2(dup2(-W2), c.b, fma2(dup2(-W2), m.b, x.a));
     x.b = fma2(dup2(-W2), p.a, fma2(dup2(-W2), c.a, x.b));
+    x = fma4(dup2(-W0), c, x);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) y[e] = fmaf(W1, w[e + 5], fmaf(W1, w[e + 3], get(x, e)));
-    d = fma4(dup2(-W0), c, mk4(y[0], y[1], y[2], y[3]));
+    for (int e = 0; e < 4; ++e) {
+        y[e] = fmaf(W3, w[e + 7], fmaf(W3, w[e + 1], get(x, e)));
+        y[e] = fmaf(W1, w[e + 5], fmaf(W1, w[e + 3], y[e]));
+    }
+    d = mk4(y[0], y[1], y[2], y[3]);
 }
 
 // x + z derivatives d of R neighbouring x rows (4 z cells each) of one plane,
@@ -227,486 +188,778 @@ template <class T>
 __device__ __forceinline__ void xz_d2(const float *H, q4 (&c)[T::R], q4 (&d)[T::R])
 {
     constexpr int R = T::R;
-    q4 row[R + 8];  // rows -4 .. R+3
+    // row by row, so that few of them are live at once
+    constexpr float w[9] = {-W4, W3, -W2, W1, -W0, W1, -W2, W3, -W4};
 #pragma unroll
-    for (int r = 0; r < R + 8; ++r) row[r] = ldq(H + (r - 4) * T::HZ);
+    for (int k = 0; k < R + 8; ++k) {  // row k - 4
+        const q4 v = ldq(H + (k - 4) * T::HZ);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        c[r] = row[r + 4];
-        q4 x = mul4(dup2(-W4), row[r]);
-        x = fma4(dup2(-W4), row[r + 8], x);
-        x = fma4(dup2(W3), row[r + 1], x);
-        x = fma4(dup2(W3), row[r + 7], x);
-        x = fma4(dup2(-W2), row[r + 2], x);
-        x = fma4(dup2(-W2), row[r + 6], x);
-        x = fma4(dup2(W1), row[r + 3], x);
-        x = fma4(dup2(W1), row[r + 5], x);
-        d[r] = fma4(dup2(-W0), c[r], x);
+        for (int r = 0; r < R; ++r) {
+            if (k < r || k > r + 8) continue;
+            d[r] = k == r ? mul4(dup2(w[0]), v) : fma4(dup2(w[k - r]), v, d[r]);
+            if (k == r + 4) c[r] = v;
+        }
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) add_dz(d[r], ldq(H + r * T::HZ - 4), c[r], ldq(H + r * T::HZ + 4));
 }
 
 // ---------------------------------------------------------------------------
-// Forward leapfrog step.
-// Bound by HBM: 4 shots of 301^3 padded cells take 0.282 ms a step, 6.19 TB/s
-// of 16 B per cell, 94 % of the 6.55 TB/s that a copy reaches (0.324 ms with
-// scalar arithmetic, one row per thread and a nine-deep y queue, which were
-// limited by instruction issue: 285 instead of about 110 instructions per 128
-// cells).  With damping, 201^3 cells take 36 us (73 us with the Cerjan factor
-// branched on per cell; here its z part sits in registers and the branch is on
-// the row).
-//   mh: halo-box map over A (the field read with the stencil)
-//   mq: centre-box map over Q (the field overwritten)
+// Time-loop kernels: roles and hand-over.
+//
+// One launch runs every step of every shot of a batch.  A work item is one
+// step of one column (a TZ x TX tile over all y planes); CTAs take items in
+// the order (shot, step, column) from a ticket counter, so every item that an
+// item waits for has been taken before it, by a CTA that is running: the waits
+// end whatever the number of resident CTAs.  Step t+1 of a column follows step
+// t a few planes behind: it may read plane p once its own column and the four
+// columns beside it have stored plane p of step t.  Several steps are thus in
+// flight at once, each a window of planes apart, and a plane that one step
+// stores is read by the next from L2.
+//
+// The same waits order the overwrites.  Step t overwrites plane y of u^(t-1)
+// after the plane y + 4 of u^t has arrived, so the neighbours have stored
+// plane y + 4 of step t-1 and therefore read all of plane y.  A halo box also
+// covers corner cells of diagonal neighbours, which the stencil never uses.
+//
+// Warps of a CTA: NW compute warps; one producer (tickets, waits for the other
+// columns, TMA); one publisher (tells the other columns which planes are in
+// memory, and samples receivers).  Stage g of a CTA carries halo plane p of
+// its current item and the centre tiles of plane y = p - 4; planes 0..3 hold
+// only zeros and are not loaded.
+// ---------------------------------------------------------------------------
+constexpr int kItemRing = 4;      // items described in shared memory at once
+constexpr int kNoMoreItems = 0x7fffffff;
+
+// FIELDS: fields that advance side by side, each with its own compute warps.
+template <class T, int FIELDS>
+struct Loop {
+    static constexpr int NWF = (T::NT + 31) / 32;  // compute warps of a field
+    static constexpr int NW = FIELDS * NWF;
+    static constexpr int THREADS = NW * 32 + 64;
+};
+
+// State of the CTA's roles in shared memory.
+template <int NW>
+struct LoopShared {
+    long long item[kItemRing];    // tickets of the items in flight, -1 ends
+    int staged[NW];               // stages finished by each compute warp
+    int items_read;               // items the publisher has looked up
+    int abort;
+};
+
+struct Item {
+    int shot, t, col;
+};
+
+// Ticket order: shots in groups of `group` whose steps interleave, then step,
+// shot of the group, column.
+__device__ __forceinline__ Item item_of(long long ticket, int nshot, int group, int nsteps, int ncol)
+{
+    const long long per_group = (long long)nsteps * ncol * group;
+    const int first = (int)(ticket / per_group) * group;
+    const long long r = ticket % per_group;
+    const int per_step = min(group, nshot - first) * ncol;
+    Item it;
+    it.t = (int)(r / per_step);
+    const int q = (int)(r - (long long)it.t * per_step);
+    it.shot = first + q / ncol;
+    it.col = q % ncol;
+    return it;
+}
+
+__device__ __forceinline__ bool aborted(const int *flag) { return *(const volatile int *)flag != 0; }
+
+__device__ __forceinline__ void loop_fail(int *flag)
+{
+    *(volatile int *)flag = 1;
+    raise_status(kErrTimeout);
+}
+
+// Bounded wait until *p >= v (shared memory).
+__device__ __forceinline__ bool wait_shared(const int *p, int v, const int *abort_flag)
+{
+    if (ld_acquire_cta(p) >= v) return true;
+    const uint64_t t0 = global_ns();
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 32; ++i) {
+            if (ld_acquire_cta(p) >= v) return true;
+            __nanosleep(64);
+        }
+        if (aborted(abort_flag) || global_ns() - t0 > kWaitLimitNs) return false;
+    }
+}
+
+// The columns whose progress an item waits for: lane 0 its own, lanes 1..4 the
+// neighbours along z and x that exist; the other lanes wait for nothing.
+__device__ __forceinline__ int dependency_column(int lane, int col, int ntz, int ncol)
+{
+    const int zt = col % ntz;
+    switch (lane) {
+    case 0: return col;
+    case 1: return zt > 0 ? col - 1 : -1;
+    case 2: return zt < ntz - 1 ? col + 1 : -1;
+    case 3: return col >= ntz ? col - ntz : -1;
+    case 4: return col + ntz < ncol ? col + ntz : -1;
+    default: return -1;
+    }
+}
+
+// Bounded wait of a warp until every lane's counter has reached `need`; `seen`
+// is the lane's last reading.
+__device__ __forceinline__ bool wait_columns(const long long *p, long long need, long long &seen,
+                                             const int *abort_flag)
+{
+    if (__all_sync(0xffffffffu, seen >= need)) return true;  // ordered by the fence below, earlier
+    const uint64_t t0 = global_ns();
+    for (int i = 0;; ++i) {
+        if (seen < need) seen = ld_acquire_gpu(p);
+        if (__all_sync(0xffffffffu, seen >= need)) break;
+        if ((i & 63) == 63) {
+            const bool late = aborted(abort_flag) || status_failed() || global_ns() - t0 > kWaitLimitNs;
+            if (__any_sync(0xffffffffu, late)) return false;
+        }
+    }
+    __syncwarp();
+    fence_proxy_async_global();  // what was acquired, before the copies that follow
+    return true;
+}
+
+// Smallest number of stages that the compute warps have finished.
+template <int NW>
+__device__ __forceinline__ int stages_done(const LoopShared<NW> &sh, int lane)
+{
+    int v = kNoMoreItems;
+    for (int w = lane; w < NW; w += 32) v = min(v, ld_acquire_cta(&sh.staged[w]));
+    return __reduce_min_sync(0xffffffffu, v);
+}
+
+// What the roles of a CTA need to know of the loop.
+struct LoopGeo {
+    int nshot, nsteps, ncol, ntz, nyy;
+};
+
+// Producer warp: takes tickets, waits until the planes an item reads are
+// stored, and issues the loads of each stage.  start(it) returns the state of
+// an item; issue(state, p, hs, cs, centre) runs in lane 0: it announces the
+// bytes on full[hs] and starts the copies of halo plane p and, if centre, of
+// centre plane p - 4.
+template <int SH, int NW, class Start, class Issue>
+__device__ __forceinline__ void loop_producer(LoopShared<NW> &sh, uint64_t *full, uint64_t *done, const LoopGeo &geo,
+                                              const LoopProgress &prog, int lane, Start start, Issue issue)
+{
+    constexpr int SC = SH - 4;
+    const long long total = (long long)geo.nshot * geo.nsteps * geo.ncol;
+    int hs = 0, cs = 0, cph = 1, g = 0;  // cph: parity of the previous use of done[cs]
+    bool ok = true;
+    for (int item = 0; ok; ++item) {
+        unsigned long long tk = 0;
+        if (lane == 0) tk = atomicAdd(prog.ticket, 1ull);
+        tk = __shfl_sync(0xffffffffu, tk, 0);
+        const bool end = (long long)tk >= total;
+        ok = wait_shared(&sh.items_read, item - (kItemRing - 1), &sh.abort) && (g < SC || mbar_wait(&done[cs], cph));
+        if (!__all_sync(0xffffffffu, ok)) {
+            ok = false;
+            break;
+        }
+        if (lane == 0) *(volatile long long *)&sh.item[item % kItemRing] = end ? -1 : (long long)tk;
+        if (end) {
+            if (lane == 0) mbar_arrive(&full[hs]);
+            break;
+        }
+        const Item it = item_of((long long)tk, geo.nshot, prog.shots, geo.nsteps, geo.ncol);
+        const int dep = it.t > 0 ? dependency_column(lane, it.col, geo.ntz, geo.ncol) : -1;
+        const long long *dp =
+            prog.done + ((long long)it.shot * prog.ring + (it.t + prog.ring - 1) % prog.ring) * geo.ncol + max(dep, 0);
+        long long seen = dep >= 0 ? 0 : 0x7fffffffffffffffll;
+        const long long base = (long long)(it.t - 1) * geo.nyy;
+        const auto state = start(it);
+        for (int p = 4; p < geo.nyy; ++p) {
+            if (p > 4 && g >= SC) ok = mbar_wait(&done[cs], cph);
+            // (the last four planes are never written)
+            if (p < geo.nyy - 4) ok = wait_columns(dp, base + p + 1, seen, &sh.abort) && ok;
+            if (!__all_sync(0xffffffffu, ok)) {
+                ok = false;
+                break;
+            }
+            if (lane == 0) issue(state, p, hs, cs, p >= 8);
+            ++g;
+            if (++hs == SH) hs = 0;
+            if (++cs == SC) {
+                cs = 0;
+                cph ^= 1;
+            }
+        }
+    }
+    if (!ok && lane == 0) {
+        loop_fail(&sh.abort);
+        mbar_arrive(&full[hs]);  // wakes the compute warps, which see the abort
+        // no copy may land after the CTA has gone: only the newest use of
+        // each slot can still be in flight
+        for (int k = 1; k <= min(g, SH); ++k) {
+            const int st = g - k;
+            mbar_wait(&full[st % SH], (st / SH) & 1);
+        }
+    }
+}
+
+// Publisher warp: follows the compute warps and tells the other columns which
+// planes of an item are stored.  start(it) returns the state of an item;
+// before(state, n) runs when the planes below n are stored and not yet
+// published, after(state, n) when they are published.
+template <int NW, class Start, class Before, class After>
+__device__ __forceinline__ void loop_publisher(LoopShared<NW> &sh, const LoopGeo &geo, const LoopProgress &prog,
+                                               int lane, Start start, Before before, After after)
+{
+    const int nstage = geo.nyy - 4;  // stages of an item: p = 4 .. nyy-1, y = p - 4
+    // stages finished by every compute warp, once there are more than s; -1
+    // when the wait gave up
+    auto more_than = [&](int s) {
+        int n = stages_done(sh, lane);
+        if (n > s) return n;
+        const uint64_t t0 = global_ns();
+        for (;;) {
+            for (int i = 0; i < 64; ++i) {
+                __nanosleep(20);
+                if ((n = stages_done(sh, lane)) > s) return n;
+            }
+            const bool late = aborted(&sh.abort) || global_ns() - t0 > 2 * kWaitLimitNs;
+            if (__any_sync(0xffffffffu, late)) return -1;
+        }
+    };
+    for (int item = 0;; ++item) {
+        const int s0 = item * nstage;
+        int n = more_than(s0);
+        if (n < 0 || n == kNoMoreItems) return;
+        const long long tk = *(volatile long long *)&sh.item[item % kItemRing];
+        __syncwarp();
+        if (lane == 0) st_release_cta(&sh.items_read, item + 1);
+        const Item it = item_of(tk, geo.nshot, prog.shots, geo.nsteps, geo.ncol);
+        long long *dp = prog.done + ((long long)it.shot * prog.ring + it.t % prog.ring) * geo.ncol + it.col;
+        const long long base = (long long)it.t * geo.nyy;
+        auto state = start(it);
+        int published = 4;  // the first four planes are never written
+        while (published < nstage) {
+            n = more_than(s0 + published);
+            if (n < 0) return;
+            published = min(n - s0, nstage);
+            before(state, published);
+            __syncwarp();
+            if (lane == 0) st_release_gpu(dp, base + published);
+            __syncwarp();
+            after(state, published);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Forward time loop.
+//   mh: halo-box maps over the field pair (read with the stencil)
+//   mq: centre-box maps over the field pair (the old level, overwritten)
 //   mv: centre-box map over the stencil coefficients dt^2 v^2 / dh^2 of the
 //       velocity slots (one slot shared by every shot, or one slot per shot
 //       when every shot has its own random pad).  They are 0 on the cells
 //       that are never updated, which keeps those cells at 0.
 // ---------------------------------------------------------------------------
-template <class T, int SH, int SC, bool ABC>
-__global__ void __launch_bounds__(T::NT)
-    fd_forward_kernel(const __grid_constant__ CUtensorMap mh, const __grid_constant__ CUtensorMap mq,
-                      const __grid_constant__ CUtensorMap mv, const FwdArgs a)
+struct FwdMaps {
+    CUtensorMap mh[2], mq[2], mv;
+};
+
+template <class T, int SH, bool ABC, int CTAS>
+__global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
+    fd_forward_kernel(const __grid_constant__ FwdMaps maps, const FwdArgs a)
 {
-    static_assert(SH >= 5, "plane y needs halo slots y..y+4");
-    constexpr int R = T::R;
+    static_assert(SH >= 6, "plane y needs halo slots y..y+4, and one more to load ahead");
+    constexpr int R = T::R, NW = Loop<T, 1>::NW;
+    constexpr int SC = SH - 4;  // centre slots: a stage's loads run SC stages ahead of its end
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char *hring = smem;
     unsigned char *cring = smem + SH * T::HSLOT;
-    uint64_t *hbar = reinterpret_cast<uint64_t *>(cring + SC * 2 * T::CSLOT);
-    uint64_t *cbar = hbar + SH;
-    __shared__ int abort_flag;
+    uint64_t *full = reinterpret_cast<uint64_t *>(cring + SC * 2 * T::CSLOT);  // [SH] stage loaded
+    uint64_t *done = full + SH;                                                // [SC] stage computed
+    __shared__ LoopShared<NW> sh;
+    __shared__ float b1s[ABC ? kMaxPad : 1];
 
-    const int tid = threadIdx.x;
-    const int shot = blockIdx.y;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (status_failed()) return;
-
-    // Receiver samples of A at this step (before the guard below, so that
-    // every launched thread takes part).  The reference records P after its
-    // in-place damping, i.e. d * A (src/modeling/modeling.cu:378, 391-392).
-    if (a.t > a.tlag) {
-        const int nrec = a.binfo->R;
-        const long long total = (long long)gridDim.x * gridDim.y * T::NT;
-        for (long long g = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * T::NT + tid; g < nrec;
-             g += total)
-            a.seis_tm[(long long)(a.t - a.tlag) * nrec + g] = a.rec_damp[g] * a.A[a.rec_cell[g]];
+    if constexpr (ABC) {
+        for (int i = tid; i < a.nb; i += Loop<T, 1>::THREADS) b1s[i] = a.b1d[i];
     }
-
-    int b = blockIdx.x;
-    const int zt = b % a.ntz;
-    b /= a.ntz;
-    const int xt = b % a.ntx;
-    const int ch = b / a.ntx;
-    const int z0 = 4 + zt * T::TZ, x0 = 4 + xt * T::TX;
-    const int ya = 4 + ch * a.ylen;
-    const int yb = min(ya + a.ylen, a.nyy - 4);
-    if (ya >= yb || shot >= a.binfo->nshot) return;  // uniform per CTA
-
-    const int lz = tid % T::TZ4, lx = tid / T::TZ4 * R;
-    const int zc = z0 + 4 * lz, xc = x0 + lx;
-    const int vshot = a.vel_slots > 1 ? shot : 0;
-
+    if (tid < NW) sh.staged[tid] = 0;
     if (tid == 0) {
-        abort_flag = 0;
-        prefetch_tmap(&mh);
-        prefetch_tmap(&mq);
-        prefetch_tmap(&mv);
-        for (int s = 0; s < SH; ++s) mbar_init(&hbar[s], 1);
-        for (int s = 0; s < SC; ++s) mbar_init(&cbar[s], 1);
+        sh.items_read = 0;
+        sh.abort = 0;
+        for (int s = 0; s < SH; ++s) mbar_init(&full[s], 1);
+        for (int s = 0; s < SC; ++s) mbar_init(&done[s], NW);
         fence_mbar_init();
     }
     __syncthreads();
 
-    const int pf = ya - 4, pl = yb + 3;  // halo planes loaded: [pf, pl]
-    int h_issued = pf - 1, c_issued = ya - 1;  // meaningful in thread 0 only
-    auto issue_h = [&](int p, int s) {
-        mbar_expect_tx(&hbar[s], T::HALO_BYTES);
-        tma_load_4d(hring + s * T::HSLOT, &mh, &hbar[s], z0 - 4, x0 - 4, p, shot);
-        h_issued = p;
-    };
-    auto issue_c = [&](int y, int s) {
-        mbar_expect_tx(&cbar[s], 2 * T::CTR_BYTES);
-        tma_load_4d(cring + (2 * s) * T::CSLOT, &mq, &cbar[s], z0, x0, y, shot);
-        tma_load_4d(cring + (2 * s + 1) * T::CSLOT, &mv, &cbar[s], z0, x0, y, vshot);
-        c_issued = y;
-    };
-    if (tid == 0) {
-        for (int p = pf; p < pf + SH && p <= pl; ++p) issue_h(p, p - pf);
-        for (int y = ya; y < ya + SC && y < yb; ++y) issue_c(y, y - ya);
-    }
-
-    // Cerjan factors of the thread's z cells, constant over the plane loop.
-    float bz[4] = {1.f, 1.f, 1.f, 1.f};
-    int zpad = 0;
-    if constexpr (ABC) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int d = zc + e < a.nzz ? pad_depth(zc + e, a.nzz, a.nb) : -1;
-            if (d >= 0) {
-                bz[e] = a.b1d[d];
-                zpad |= 1 << e;
-            }
-        }
-    }
-    float bx[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        bx[r] = -1.0f;  // outside the x pad
-        if constexpr (ABC) {
-            const int d = xc + r < a.nxx ? pad_depth(xc + r, a.nxx, a.nb) : -1;
-            if (d >= 0) bx[r] = a.b1d[d];
-        }
-    }
-
-    const int3 src = make_int3(a.binfo->src[shot][0], a.binfo->src[shot][1], a.binfo->src[shot][2]);
-    const int se = (src.x >= zc && src.x < zc + 4) ? src.x - zc : -1;  // source cell among this thread's
-    const int sr = (se >= 0 && src.y >= xc && src.y < xc + R) ? src.y - xc : -1;
-    const int ys = sr >= 0 && a.t + 1 < a.nt ? src.z : -1;
-    const int ho = (lx + 4) * T::HZ + 4 + 4 * lz, co = lx * T::TZ + 4 * lz;
-    const int nrow = zc < a.nzz - 4 ? min(R, a.nxx - 4 - xc) : 0;  // rows this thread writes
+    const LoopGeo geo{a.binfo->nshot, a.nsteps, a.ncol, a.ntz, a.nyy};
     const long long plane = (long long)a.ldz * a.nxx;
-    float *Qp = a.Q + (long long)shot * a.vol + (long long)ya * plane + (long long)xc * a.ldz + zc;
 
-    q4 s[R][8];
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int m = 0; m < 8; ++m) s[r][m] = mk4(0.f, 0.f, 0.f, 0.f);
-
-    // Ring positions: hs, hph = slot and phase parity of halo plane p; hy =
-    // slot of plane y = p - 4; cs, cph = slot and phase parity of centre plane y.
-    int hs = 0, hph = 0, hy = 0, cs = 0, cph = 0;
-    for (int p = pf; p <= pl; ++p) {
-        const int y = p - 4;
-        bool ok = mbar_wait(&hbar[hs], hph);
-        if (y >= ya) ok = mbar_wait(&cbar[cs], cph) && ok;
-        if (!ok) abort_flag = 1;
-
-        const float *Hp = reinterpret_cast<const float *>(hring + hs * T::HSLOT) + ho;
-        q4 dy[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) dy[r] = push_y(s[r], ldq(Hp + r * T::HZ));
-
-        if (y >= ya) {
-            const float *Hy = reinterpret_cast<const float *>(hring + hy * T::HSLOT) + ho;
-            const float *Cq = reinterpret_cast<const float *>(cring + (2 * cs) * T::CSLOT) + co;
-            const float *Cv = reinterpret_cast<const float *>(cring + (2 * cs + 1) * T::CSLOT) + co;
-            q4 c[R], d[R];
-            xz_d2<T>(Hy, c, d);
-            float by = -1.0f;
-            if constexpr (ABC) {
-                const int dep = pad_depth(y, a.nyy, a.nb);
-                if (dep >= 0) by = a.b1d[dep];
-            }
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const q4 lap = add4(d[r], dy[r]);
-                const q4 old = ldq(Cq + r * T::TZ), cv = ldq(Cv + r * T::TZ);
-                q4 out;
-                if constexpr (ABC) {
-                    // b2d / b3d of the reference (modeling.cu:101-127) from
-                    // the 1-D table; which axes are in the pad is the same
-                    // for the whole row except along z
-                    float f[4];
-                    const bool px = bx[r] >= 0.0f, py = by >= 0.0f;
-                    if (px && py) {
-                        const float bxy = __fadd_rn(bx[r], by), n2 = __fsub_rn(bxy, 1.0f);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            f[e] = (zpad >> e) & 1
-                                       ? __fsub_rn(__fadd_rn(__fadd_rn(__fadd_rn(bz[e], bx[r]), bxy),
-                                                             __fadd_rn(bz[e], by)), 5.0f)
-                                       : n2;
-                    } else if (px || py) {
-                        const float b1 = px ? bx[r] : by;
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            f[e] = (zpad >> e) & 1 ? __fsub_rn(__fadd_rn(bz[e], b1), 1.0f) : b1;
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) f[e] = bz[e];
+    if (warp == NW) {
+        if (lane == 0) {
+            prefetch_tmap(&maps.mh[0]);
+            prefetch_tmap(&maps.mh[1]);
+            prefetch_tmap(&maps.mq[0]);
+            prefetch_tmap(&maps.mq[1]);
+            prefetch_tmap(&maps.mv);
+        }
+        struct State {
+            const CUtensorMap *mh, *mq;
+            int z0, x0, shot, vshot;
+        };
+        loop_producer<SH>(
+            sh, full, done, geo, a.prog, lane,
+            [&](const Item &it) {
+                return State{&maps.mh[it.t & 1], &maps.mq[1 - (it.t & 1)], 4 + it.col % a.ntz * T::TZ,
+                             4 + it.col / a.ntz * T::TX, it.shot, a.vel_slots > 1 ? it.shot : 0};
+            },
+            [&](const State &st, int p, int hs, int cs, bool centre) {
+                uint64_t *bar = &full[hs];
+                mbar_expect_tx(bar, T::HALO_BYTES + (centre ? 2 * T::CTR_BYTES : 0));
+                tma_load_4d(hring + hs * T::HSLOT, st.mh, bar, st.z0 - 4, st.x0 - 4, p, st.shot);
+                if (centre) {
+                    unsigned char *c = cring + 2 * cs * T::CSLOT;
+                    tma_load_4d(c, st.mq, bar, st.z0, st.x0, p - 4, st.shot);
+                    tma_load_4d(c + T::CSLOT, &maps.mv, bar, st.z0, st.x0, p - 4, st.vshot);
+                }
+            });
+    } else if (warp == NW + 1) {
+        // after publishing: samples of the level the item stores, u^(t+1)
+        struct State {
+            int u, last, sample;
+            const float *F;
+        };
+        const int nrec = a.binfo->R;
+        loop_publisher(
+            sh, geo, a.prog, lane,
+            [&](const Item &it) {
+                State st{0, 0, it.t + 1 - a.tlag, a.F[1 - (it.t & 1)]};
+                if (st.sample > 0 && it.t + 1 < a.nsteps) {
+                    st.u = a.rec.col_first[it.shot * a.ncol + it.col];
+                    st.last = a.rec.col_first[it.shot * a.ncol + it.col + 1];
+                }
+                return st;
+            },
+            [](State &, int) {},
+            [&](State &st, int n) {
+                while (st.u < st.last) {
+                    const int e = st.u + lane;
+                    const bool mine = e < st.last && a.rec.y[min(e, st.last - 1)] < n;
+                    if (mine) {
+                        const float v = __ldcg(st.F + a.rec.cell[e]);
+                        for (int k = a.rec.first[e]; k < a.rec.first[e + 1]; ++k) {
+                            const int r = a.rec.rid[k];
+                            a.seis_tm[(long long)st.sample * nrec + r] = a.rec_damp[r] * v;
+                        }
                     }
-                    const q4 f4 = mk4(f[0], f[1], f[2], f[3]), n4 = mk4(-f[0], -f[1], -f[2], -f[3]);
-                    out = fma4(cv, lap, fma4(n4, old, add4(c[r], c[r])));
-                    out = {mul2(f4.a, out.a), mul2(f4.b, out.b)};
-                } else {
-                    out = fma4(cv, lap, fma4(dup2(-1.0f), old, add4(c[r], c[r])));
+                    const int got = __popc(__ballot_sync(0xffffffffu, mine));
+                    st.u += got;
+                    if (got < 32) break;
                 }
-                // Source sample t+1 goes into the new field, which is exactly where
-                // the reference adds it at the start of the next step
-                // (src/modeling/modeling.cu:347-348).
-                if (y == ys && r == sr) {
-                    const float add = a.idh3 * a.wavelet[a.t + 1];
-                    out = mk4(lo(out.a) + (se == 0 ? add : 0.f), hi(out.a) + (se == 1 ? add : 0.f),
-                              lo(out.b) + (se == 2 ? add : 0.f), hi(out.b) + (se == 3 ? add : 0.f));
-                }
-                if (r < nrow) stq(Qp + (long long)r * a.ldz, out);
+            });
+    } else {
+        // ---- compute ----
+        const int ct = min(tid, T::NT - 1);  // the last warp's spare lanes repeat its last thread
+        const int lz = ct % T::TZ4, lx = ct / T::TZ4 * R;
+        const int ho = (lx + 4) * T::HZ + 4 + 4 * lz, co = lx * T::TZ + 4 * lz;
+        int hs = 0, hph = 0, cs = 0, g = 0;
+        for (int item = 0;; ++item) {
+            bool ok = __all_sync(0xffffffffu, mbar_wait(&full[hs], hph) && !aborted(&sh.abort));
+            if (!ok) {
+                loop_fail(&sh.abort);
+                break;
             }
-            Qp += plane;
-        }
-        __syncthreads();
-        if (abort_flag) break;
-        if (tid == 0) {
-            fence_proxy_async();
-            if (p < ya) {
-                if (p + SH <= pl) issue_h(p + SH, hs);
-            } else if (y >= ya) {
-                if (y + SH <= pl) issue_h(y + SH, hy);
-                if (y + SC < yb) issue_c(y + SC, cs);
+            const long long tk = *(volatile long long *)&sh.item[item % kItemRing];
+            if (tk < 0) {
+                __syncwarp();
+                if (lane == 0) st_release_cta(&sh.staged[warp], kNoMoreItems);
+                break;
             }
-        }
-        if (++hs == SH) {
-            hs = 0;
-            hph ^= 1;
-        }
-        if (y >= ya) {
-            if (++hy == SH) hy = 0;
-            if (++cs == SC) {
-                cs = 0;
-                cph ^= 1;
-            }
-        } else if (y == ya - 1) {
-            hy = 4 % SH;
-        }
-    }
+            const Item it = item_of(tk, geo.nshot, a.prog.shots, a.nsteps, a.ncol);
+            const int zc = 4 + it.col % a.ntz * T::TZ + 4 * lz, xc = 4 + it.col / a.ntz * T::TX + lx;
 
-    if (abort_flag && tid == 0) {
-        raise_status(kErrTimeout);
-        // Drain copies still in flight into this CTA's shared memory.
-        // (only the newest use of each slot can still be in flight)
-        for (int p = max(pf, h_issued - SH + 1); p <= h_issued; ++p)
-            mbar_wait(&hbar[(p - pf) % SH], ((p - pf) / SH) & 1);
-        for (int y = max(ya, c_issued - SC + 1); y <= c_issued; ++y)
-            mbar_wait(&cbar[(y - ya) % SC], ((y - ya) / SC) & 1);
+            // Cerjan factors of the thread's z cells and x rows, constant over the plane loop
+            float bz[4] = {1.f, 1.f, 1.f, 1.f};
+            float bx[R];
+            int zpad = 0;
+#pragma unroll
+            for (int r = 0; r < R; ++r) bx[r] = -1.0f;  // outside the x pad
+            if constexpr (ABC) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int d = zc + e < a.nzz ? pad_depth(zc + e, a.nzz, a.nb) : -1;
+                    if (d >= 0) {
+                        bz[e] = b1s[d];
+                        zpad |= 1 << e;
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int d = xc + r < a.nxx ? pad_depth(xc + r, a.nxx, a.nb) : -1;
+                    if (d >= 0) bx[r] = b1s[d];
+                }
+            }
+            // source cell among this thread's cells: element se of row sr on plane ys
+            const int sz = a.binfo->src[it.shot][0], sx = a.binfo->src[it.shot][1];
+            const int se = (sz >= zc && sz < zc + 4) ? sz - zc : -1;
+            const int sr = (se >= 0 && sx >= xc && sx < xc + R) ? sx - xc : -1;
+            const int ys = sr >= 0 && it.t + 1 < a.nt ? a.binfo->src[it.shot][2] : -1;
+            // rows this thread writes
+            const int nrow = zc < a.nzz - 4 && tid < T::NT ? min(R, a.nxx - 4 - xc) : 0;
+            float *Qp = a.F[1 - (it.t & 1)] + (long long)it.shot * a.vol + 4 * plane + (long long)xc * a.ldz + zc;
+
+            q4 s[R][8];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int m = 0; m < 8; ++m) s[r][m] = mk4(0.f, 0.f, 0.f, 0.f);
+
+            for (int p = 4; p < a.nyy; ++p) {
+                const int y = p - 4;
+                if (p > 4) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(&full[hs], hph) && !aborted(&sh.abort));
+                    if (!ok) break;
+                }
+                const float *Hp = reinterpret_cast<const float *>(hring + hs * T::HSLOT) + ho;
+                q4 dy[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    dy[r] = push_y(s[r], ldq(Hp + r * T::HZ));
+                }
+                if (y >= 4) {
+                    const int hy = hs >= 4 ? hs - 4 : hs + SH - 4;
+                    const float *Hy = reinterpret_cast<const float *>(hring + hy * T::HSLOT) + ho;
+                    const float *Cq = reinterpret_cast<const float *>(cring + (2 * cs) * T::CSLOT) + co;
+                    const float *Cv = reinterpret_cast<const float *>(cring + (2 * cs + 1) * T::CSLOT) + co;
+                    q4 c[R], d[R];
+                    xz_d2<T>(Hy, c, d);
+                    float by = -1.0f;
+                    if constexpr (ABC) {
+                        const int dep = pad_depth(y, a.nyy, a.nb);
+                        if (dep >= 0) by = b1s[dep];
+                    }
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const q4 lap = add4(d[r], dy[r]);
+                        const q4 old = ldq(Cq + r * T::TZ), cv = ldq(Cv + r * T::TZ);
+                        q4 out;
+                        if constexpr (ABC) {
+                            // b2d / b3d of the reference (modeling.cu:101-127) from
+                            // the 1-D table; which axes are in the pad is the same
+                            // for the whole row except along z
+                            float f[4];
+                            const bool px = bx[r] >= 0.0f, py = by >= 0.0f;
+                            if (px && py) {
+                                const float bxy = __fadd_rn(bx[r], by), n2 = __fsub_rn(bxy, 1.0f);
+#pragma unroll
+                                for (int e = 0; e < 4; ++e)
+                                    f[e] = (zpad >> e) & 1
+                                               ? __fsub_rn(__fadd_rn(__fadd_rn(__fadd_rn(bz[e], bx[r]), bxy),
+                                                                     __fadd_rn(bz[e], by)), 5.0f)
+                                               : n2;
+                            } else if (px || py) {
+                                const float b1 = px ? bx[r] : by;
+#pragma unroll
+                                for (int e = 0; e < 4; ++e)
+                                    f[e] = (zpad >> e) & 1 ? __fsub_rn(__fadd_rn(bz[e], b1), 1.0f) : b1;
+                            } else {
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) f[e] = bz[e];
+                            }
+                            const q4 f4 = mk4(f[0], f[1], f[2], f[3]), n4 = mk4(-f[0], -f[1], -f[2], -f[3]);
+                            out = fma4(cv, lap, fma4(n4, old, add4(c[r], c[r])));
+                            out = {mul2(f4.a, out.a), mul2(f4.b, out.b)};
+                        } else {
+                            out = fma4(cv, lap, fma4(dup2(-1.0f), old, add4(c[r], c[r])));
+                        }
+                        // Source sample t+1 goes into the new field, which is exactly where
+                        // the reference adds it at the start of the next step
+                        // (src/modeling/modeling.cu:347-348).
+                        if (y == ys && r == sr) {
+                            const float add = a.idh3 * a.wavelet[it.t + 1];
+                            out = mk4(lo(out.a) + (se == 0 ? add : 0.f), hi(out.a) + (se == 1 ? add : 0.f),
+                                      lo(out.b) + (se == 2 ? add : 0.f), hi(out.b) + (se == 3 ? add : 0.f));
+                        }
+                        if (r < nrow) stq(Qp + (long long)r * a.ldz, out);
+                    }
+                    Qp += plane;
+                }
+                ++g;
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&done[cs]);
+                    st_release_cta(&sh.staged[warp], g);
+                }
+                if (++hs == SH) {
+                    hs = 0;
+                    hph ^= 1;
+                }
+                if (++cs == SC) cs = 0;
+            }
+            if (!ok) {
+                loop_fail(&sh.abort);
+                break;
+            }
+        }
     }
 }
 
 // ---------------------------------------------------------------------------
-// Fused backward step.
-//   mhs, mhr: halo maps over Psold and Pr
-//   mcs, mcr: centre maps over Ps and Prold (old time levels, overwritten)
-//   mv:       centre map over the velocity slots (shared, or one per shot);
-//             with the image condition over their stencil coefficient
-//             dt^2 v^2 / dh^2 instead (the gradient condition also needs v^2)
-//   mim, mil: maps over the image/gradient and illumination slots, with a box
-//             of acc_zbox x TX cells (the widest z range of a tile that meets
-//             the accumulated box)
-// GRAD: gradient imaging condition (with GRAD_DY the d2y term is kept).
+// Backward time loop: the source field is rebuilt backwards, the adjoint field
+// propagates, and the image (or gradient) and the illumination accumulate.
+//   mhs, mhr: halo maps over the source and adjoint field pairs
+//   mcs, mcr: centre maps over the same (old time levels, overwritten)
+//   mv:       centre map over the stencil coefficients (0 on the cells that
+//             are never updated)
+// GRAD: gradient imaging condition (with GRAD_DY the d2y term is kept).  Its
+// factor dt v^2 / dh^2 is the coefficient times 1/dt.
+// The accumulators are updated by vector reductions in L2: they take no shared
+// memory, so the rings run a stage deeper, and nothing waits for them.  The
+// steps of a column follow one another, so every cell adds its steps in order.
 // ---------------------------------------------------------------------------
-template <class T, int SH, int SC, bool GRAD, bool GRAD_DY>
-__global__ void __launch_bounds__(T::NT)
-    fd_backward_kernel(const __grid_constant__ CUtensorMap mhs, const __grid_constant__ CUtensorMap mhr,
-                       const __grid_constant__ CUtensorMap mcs, const __grid_constant__ CUtensorMap mcr,
-                       const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mim,
-                       const __grid_constant__ CUtensorMap mil, const BwdArgs a)
+struct BwdMaps {
+    CUtensorMap mhs[2], mhr[2], mcs[2], mcr[2], mv;
+};
+
+template <class T, int SH, bool GRAD, bool GRAD_DY, int CTAS>
+__global__ void __launch_bounds__(Loop<T, 2>::THREADS, CTAS)
+    fd_backward_kernel(const __grid_constant__ BwdMaps maps, const BwdArgs a)
 {
-    static_assert(SH >= 5, "plane y needs halo slots y..y+4");
-    constexpr int NCF = 5;  // centre fields: Ps, Prold, v, image, illum
+    static_assert(SH >= 6, "plane y needs halo slots y..y+4, and one more to load ahead");
+    constexpr int R = T::R, NW = Loop<T, 2>::NW;
+    constexpr int SC = SH - 4, NCF = 3;  // centre fields: Ps, Prold, coefficient
     extern __shared__ __align__(128) unsigned char smem[];
-    unsigned char *hring = smem;                            // SH x {Psold, Pr}
-    unsigned char *cring = smem + SH * 2 * T::HSLOT;        // SC x {Ps, Prold, v, img, ill}
-    uint64_t *hbar = reinterpret_cast<uint64_t *>(cring + SC * NCF * T::CSLOT);
-    uint64_t *cbar = hbar + SH;
-    __shared__ int abort_flag;
+    unsigned char *hring = smem;                      // SH x {Psold, Pr}
+    unsigned char *cring = smem + SH * 2 * T::HSLOT;  // SC x {Ps, Prold, coefficient}
+    uint64_t *full = reinterpret_cast<uint64_t *>(cring + SC * NCF * T::CSLOT);
+    uint64_t *done = full + SH;
+    __shared__ LoopShared<NW> sh;
 
-    const int tid = threadIdx.x;
-    const int shot = blockIdx.y;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (status_failed()) return;
-    int b = blockIdx.x;
-    const int zt = b % a.ntz;
-    b /= a.ntz;
-    const int xt = b % a.ntx;
-    const int ch = b / a.ntx;
-    const int z0 = 4 + zt * T::TZ, x0 = 4 + xt * T::TX;
-    const int ya = 4 + ch * a.ylen;
-    const int yb = min(ya + a.ylen, a.nyy - 4);
-    if (ya >= yb || shot >= a.binfo->nshot) return;
-
-    const int lz = tid % T::TZ4, lx = tid / T::TZ4;
-    const int zc = z0 + 4 * lz, xc = x0 + lx;
-    const int vshot = a.vel_slots > 1 ? shot : 0;
-    // Accumulator box: a CTA whose tile misses it in z or x, and every plane
-    // outside it in y, moves no accumulator bytes at all.
-    const bool acc_tile = z0 < a.acc_z1 && z0 + T::TZ > a.acc_z0 && x0 < a.acc_x1 && x0 + T::TX > a.acc_x0;
-    const bool acc_row = xc >= a.acc_x0 && xc < a.acc_x1 && zc < a.acc_z1 && zc + 4 > a.acc_z0;
-    auto acc_plane = [&](int y) { return acc_tile && y >= a.acc_y0 && y < a.acc_y1; };
-    // Accumulator tiles cover z in [za, za + acc_zbox) only: the part of the
-    // tile's z range that reaches the box, widened to float4 boundaries (the
-    // TMA start stays 16-byte aligned).
-    const int za = max(z0, a.acc_z0) & ~3;
-    const int acc_bytes = a.acc_zbox * T::TX * 4;
-
+    if (tid < NW) sh.staged[tid] = 0;
     if (tid == 0) {
-        abort_flag = 0;
-        prefetch_tmap(&mhs);
-        prefetch_tmap(&mhr);
-        for (int s = 0; s < SH; ++s) mbar_init(&hbar[s], 1);
-        for (int s = 0; s < SC; ++s) mbar_init(&cbar[s], 1);
+        sh.items_read = 0;
+        sh.abort = 0;
+        for (int s = 0; s < SH; ++s) mbar_init(&full[s], 1);
+        for (int s = 0; s < SC; ++s) mbar_init(&done[s], NW);
         fence_mbar_init();
     }
     __syncthreads();
 
-    const int pf = ya - 4, pl = yb + 3;
-    int h_issued = pf - 1, c_issued = ya - 1;
-    auto issue_h = [&](int p, int s) {
-        mbar_expect_tx(&hbar[s], 2 * T::HALO_BYTES);
-        tma_load_4d(hring + (2 * s) * T::HSLOT, &mhs, &hbar[s], z0 - 4, x0 - 4, p, shot);
-        tma_load_4d(hring + (2 * s + 1) * T::HSLOT, &mhr, &hbar[s], z0 - 4, x0 - 4, p, shot);
-        h_issued = p;
-    };
-    auto issue_c = [&](int y, int s) {
-        unsigned char *base = cring + s * NCF * T::CSLOT;
-        const bool acc = acc_plane(y);
-        mbar_expect_tx(&cbar[s], (NCF - 2) * T::CTR_BYTES + (acc ? 2 * acc_bytes : 0));
-        tma_load_4d(base + 0 * T::CSLOT, &mcs, &cbar[s], z0, x0, y, shot);
-        tma_load_4d(base + 1 * T::CSLOT, &mcr, &cbar[s], z0, x0, y, shot);
-        tma_load_4d(base + 2 * T::CSLOT, &mv, &cbar[s], z0, x0, y, vshot);
-        if (acc) {
-            tma_load_4d(base + 3 * T::CSLOT, &mim, &cbar[s], za, x0, y, shot);
-            tma_load_4d(base + 4 * T::CSLOT, &mil, &cbar[s], za, x0, y, shot);
-        }
-        c_issued = y;
-    };
-    if (tid == 0) {
-        for (int p = pf; p < pf + SH && p <= pl; ++p) issue_h(p, p - pf);
-        for (int y = ya; y < ya + SC && y < yb; ++y) issue_c(y, y - ya);
-    }
-
-    const int3 src = make_int3(a.binfo->src[shot][0], a.binfo->src[shot][1], a.binfo->src[shot][2]);
-    // Stored field A_{N-t} carried source sample N-t; the exact rebuild adds it back.
-    const float scorr = (a.subtract_src && a.nsteps - a.t < a.nt)
-                            ? a.idh3 * a.wavelet[a.nsteps - a.t] : 0.0f;
-    const int ro = (lx + 4) * T::HZ, zo = 4 + 4 * lz;
-    const bool row_ok = xc < a.nxx - 4 && zc < a.nzz - 4;
+    const LoopGeo geo{a.binfo->nshot, a.nsteps, a.ncol, a.ntz, a.nyy};
     const long long plane = (long long)a.ldz * a.nxx;
-    const long long sh_off = (long long)shot * a.vol;
-
-    float4 qs[9], qr[9];
-#pragma unroll
-    for (int m = 0; m < 9; ++m) {
-        qs[m] = make_float4(0.f, 0.f, 0.f, 0.f);
-        qr[m] = qs[m];
-    }
-
-    // Ring positions as counters (no division by the ring depths per plane):
-    // hs, hph = slot and phase parity of halo plane p; hy = slot of plane
-    // y = p - 4; cs, cph = slot and phase parity of centre plane y.
-    int hs = 0, hph = 0, cs = 0, cph = 0;
-    for (int p = pf; p <= pl; ++p) {
-        const int y = p - 4;
-        const int hy = hs >= 4 ? hs - 4 : hs + SH - 4;
-        bool ok = mbar_wait(&hbar[hs], hph);
-        if (y >= ya) ok = mbar_wait(&cbar[cs], cph) && ok;
-        if (!ok) abort_flag = 1;
-
-        const float *Hs = reinterpret_cast<const float *>(hring + (2 * hs) * T::HSLOT);
-        const float *Hr = reinterpret_cast<const float *>(hring + (2 * hs + 1) * T::HSLOT);
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            qs[m] = qs[m + 1];
-            qr[m] = qr[m + 1];
+    if (warp == NW) {
+        if (lane == 0) {
+            for (int b = 0; b < 2; ++b) {
+                prefetch_tmap(&maps.mhs[b]);
+                prefetch_tmap(&maps.mhr[b]);
+                prefetch_tmap(&maps.mcs[b]);
+                prefetch_tmap(&maps.mcr[b]);
+            }
+            prefetch_tmap(&maps.mv);
         }
-        qs[8] = lds4(Hs + ro + zo);
-        qr[8] = lds4(Hr + ro + zo);
-
-        if (y >= ya) {
-            const float *Hys = reinterpret_cast<const float *>(hring + (2 * hy) * T::HSLOT);
-            const float *Hyr = reinterpret_cast<const float *>(hring + (2 * hy + 1) * T::HSLOT);
-            const float *C = reinterpret_cast<const float *>(cring + cs * NCF * T::CSLOT);
+        struct State {
+            const CUtensorMap *mhs, *mhr, *mcs, *mcr;
+            int z0, x0, shot, vshot;
+        };
+        loop_producer<SH>(
+            sh, full, done, geo, a.prog, lane,
+            [&](const Item &it) {
+                const int sc = (a.s0 + it.t) & 1, rc = it.t & 1;
+                return State{&maps.mhs[sc], &maps.mhr[rc], &maps.mcs[1 - sc], &maps.mcr[1 - rc],
+                             4 + it.col % a.ntz * T::TZ, 4 + it.col / a.ntz * T::TX, it.shot,
+                             a.vel_slots > 1 ? it.shot : 0};
+            },
+            [&](const State &st, int p, int hs, int cs, bool centre) {
+                uint64_t *bar = &full[hs];
+                mbar_expect_tx(bar, 2 * T::HALO_BYTES + (centre ? NCF * T::CTR_BYTES : 0));
+                unsigned char *h = hring + 2 * hs * T::HSLOT;
+                tma_load_4d(h, st.mhs, bar, st.z0 - 4, st.x0 - 4, p, st.shot);
+                tma_load_4d(h + T::HSLOT, st.mhr, bar, st.z0 - 4, st.x0 - 4, p, st.shot);
+                if (centre) {
+                    unsigned char *c = cring + cs * NCF * T::CSLOT;
+                    tma_load_4d(c + 0 * T::CSLOT, st.mcs, bar, st.z0, st.x0, p - 4, st.shot);
+                    tma_load_4d(c + 1 * T::CSLOT, st.mcr, bar, st.z0, st.x0, p - 4, st.shot);
+                    tma_load_4d(c + 2 * T::CSLOT, &maps.mv, bar, st.z0, st.x0, p - 4, st.vshot);
+                }
+            });
+    } else if (warp == NW + 1) {
+        // Before publishing: the adjoint source of step t+1 (inject_seismogram
+        // / inject_residuo, src/migration/migration.cu:119-132,
+        // src/inversion/inversion.cu:385-398) is added to the level the item
+        // stores.  Lane l holds entry u + l of the column's list, with the sum
+        // of its receivers in receiver order, loaded ahead of its plane.
+        struct State {
+            int u, last, y;
+            long long cell;
+            float f;
+            const float *d;
+            float *Pr;
+        };
+        const int nrec = a.binfo->R;
+        auto load = [&](State &st) {
+            const int e = st.u + lane;
+            st.y = 0x7fffffff;
+            if (e < st.last) {
+                st.y = a.inj.y[e];
+                st.cell = a.inj.cell[e];
+                float f = 0.0f;
+                for (int k = a.inj.first[e]; k < a.inj.first[e + 1]; ++k) f += a.idh3 * st.d[a.inj.rid[k]];
+                st.f = f;
+            }
+        };
+        loop_publisher(
+            sh, geo, a.prog, lane,
+            [&](const Item &it) {
+                State st{0, 0, 0, 0, 0.0f, nullptr, a.Rf[1 - (it.t & 1)]};
+                if (it.t + 1 < a.nt) {
+                    st.u = a.inj.col_first[it.shot * a.ncol + it.col];
+                    st.last = a.inj.col_first[it.shot * a.ncol + it.col + 1];
+                    st.d = a.data_tm + (long long)(a.nt - 2 - it.t) * nrec;
+                }
+                load(st);
+                return st;
+            },
+            [&](State &st, int n) {
+                for (;;) {
+                    const bool mine = st.y < n;
+                    const int got = __popc(__ballot_sync(0xffffffffu, mine));
+                    if (got == 0) break;
+                    if (mine) red_add(st.Pr + st.cell, st.f);
+                    st.u += got;
+                    load(st);
+                    if (got < 32) break;
+                }
+            },
+            [](State &, int) {});
+    } else {
+        // ---- compute: the first NWF warps advance the source field and
+        // accumulate, the others advance the adjoint field ----
+        auto compute = [&](auto source_field) {
+            constexpr bool SRC = decltype(source_field)::value;
             constexpr int CF = T::CSLOT / 4;  // floats per centre slot
-            const int co = lx * T::TZ + 4 * lz;
-            const float4 ps_old = lds4(C + 0 * CF + co);
-            const float4 pr_old = lds4(C + 1 * CF + co);
-            const float4 vv = lds4(C + 2 * CF + co);
-            const bool acc = acc_plane(y);
-            float4 img = make_float4(0.f, 0.f, 0.f, 0.f), ill = img;
-            if (acc && acc_row) {  // then za <= zc and zc + 4 <= za + acc_zbox
-                const int ao = lx * a.acc_zbox + (zc - za);
-                img = lds4(C + 3 * CF + ao);
-                ill = lds4(C + 4 * CF + ao);
-            }
-
-            float sx[4], sy[4], sz[4];
-            axis_d2<T>(Hys, ro, zo, qs, sx, sy, sz);
-            float4 ps_new, pr_new;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float v = comp(vv, e);
-                const float cv = GRAD ? v * v * a.cvel : v;
-                float s = fmaf(cv, sx[e] + sy[e] + sz[e], 2.0f * comp(qs[4], e) - comp(ps_old, e));
-                set_comp(ps_new, e, s);
-            }
-            if (y == src.z && xc == src.y) {
-                const int e = src.x - zc;
-                if (e >= 0 && e < 4) set_comp(ps_new, e, comp(ps_new, e) + scorr);
-            }
-            float rx[4], ry[4], rz[4];
-            axis_d2<T>(Hyr, ro, zo, qr, rx, ry, rz);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float v = comp(vv, e);
-                const float v2 = v * v;  // used by the gradient condition only
-                const float cv = GRAD ? v2 * a.cvel : v;
-                const float prc = comp(qr[4], e);
-                set_comp(pr_new, e, fmaf(cv, rx[e] + ry[e] + rz[e], 2.0f * prc - comp(pr_old, e)));
-                const float psn = comp(ps_new, e);
-                const int ze = zc + e;
-                if (ze >= a.nzz - 4) {
-                    set_comp(ps_new, e, comp(ps_old, e));
-                    set_comp(pr_new, e, comp(pr_old, e));
+            const int ft = SRC ? tid : tid - Loop<T, 2>::NWF * 32;
+            const int ct = min(ft, T::NT - 1);  // the last warp's spare lanes repeat its last thread
+            const int lz = ct % T::TZ4, lx = ct / T::TZ4 * R;
+            const int ho = (lx + 4) * T::HZ + 4 + 4 * lz, co = lx * T::TZ + 4 * lz;
+            int hs = 0, hph = 0, cs = 0, g = 0;
+            for (int item = 0;; ++item) {
+                bool ok = __all_sync(0xffffffffu, mbar_wait(&full[hs], hph) && !aborted(&sh.abort));
+                if (!ok) {
+                    loop_fail(&sh.abort);
+                    break;
                 }
-                // (the box lies inside the updated cells: acc_z1 <= nzz - 4)
-                if (acc && acc_row && ze >= a.acc_z0 && ze < a.acc_z1) {
-                    float im = comp(img, e), il = comp(ill, e);
-                    il = fmaf(psn, psn, il);
-                    if constexpr (GRAD) {
-                        const float lz2 = GRAD_DY ? (sx[e] + sz[e] + sy[e]) : (sx[e] + sz[e]);
-                        im += a.gscale * prc * lz2 * v2;
-                    } else {
-                        im = fmaf(psn, prc, im);
+                const long long tk = *(volatile long long *)&sh.item[item % kItemRing];
+                if (tk < 0) {
+                    __syncwarp();
+                    if (lane == 0) st_release_cta(&sh.staged[warp], kNoMoreItems);
+                    break;
+                }
+                const Item it = item_of(tk, geo.nshot, a.prog.shots, a.nsteps, a.ncol);
+                const int zc = 4 + it.col % a.ntz * T::TZ + 4 * lz, xc = 4 + it.col / a.ntz * T::TX + lx;
+                const int nrow = zc < a.nzz - 4 && ft < T::NT ? min(R, a.nxx - 4 - xc) : 0;  // rows this thread writes
+                long long off = (long long)it.shot * a.vol + 4 * plane + (long long)xc * a.ldz + zc;
+                float *out = SRC ? a.F[1 - ((a.s0 + it.t) & 1)] : a.Rf[1 - (it.t & 1)];
+                // source cell among this thread's cells: element se of row sr on
+                // plane ys.  Stored field A_{N-t} carried source sample N-t; the
+                // exact rebuild adds it back.
+                int se = -1, sr = -1, ys = -1;
+                int zmask = 0;  // cells of the thread's quad that accumulate
+                if constexpr (SRC) {
+                    const int sz = a.binfo->src[it.shot][0], sx = a.binfo->src[it.shot][1];
+                    if (sz >= zc && sz < zc + 4) se = sz - zc;
+                    if (se >= 0 && sx >= xc && sx < xc + R) sr = sx - xc;
+                    if (sr >= 0 && a.subtract_src && a.nsteps - it.t < a.nt) ys = a.binfo->src[it.shot][2];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) zmask |= (zc + e >= a.acc_z0 && zc + e < a.acc_z1) ? 1 << e : 0;
+                }
+
+                q4 s[R][8];  // y derivatives in the making
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) s[r][m] = mk4(0.f, 0.f, 0.f, 0.f);
+
+                for (int p = 4; p < a.nyy; ++p) {
+                    const int y = p - 4;
+                    if (p > 4) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(&full[hs], hph) && !aborted(&sh.abort));
+                        if (!ok) break;
                     }
-                    set_comp(img, e, im);
-                    set_comp(ill, e, il);
+                    const float *Hp =
+                        reinterpret_cast<const float *>(hring + (2 * hs + (SRC ? 0 : 1)) * T::HSLOT) + ho;
+                        q4 dy[R];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        dy[r] = push_y(s[r], ldq(Hp + r * T::HZ));
+                    }
+                    if (y >= 4) {
+                        const int hy = hs >= 4 ? hs - 4 : hs + SH - 4;
+                        const float *Hy =
+                            reinterpret_cast<const float *>(hring + (2 * hy + (SRC ? 0 : 1)) * T::HSLOT) + ho;
+                        const float *C = reinterpret_cast<const float *>(cring + cs * NCF * T::CSLOT);
+                        const bool acc = SRC && zmask && y >= a.acc_y0 && y < a.acc_y1;
+                        q4 c[R], d[R];
+                        xz_d2<T>(Hy, c, d);
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            const q4 cv = ldq(C + 2 * CF + co + r * T::TZ);
+                            const q4 old = ldq(C + (SRC ? 0 : CF) + co + r * T::TZ);
+                            const q4 lap = add4(d[r], dy[r]);
+                            q4 nv = fma4(cv, lap, fma4(dup2(-1.0f), old, add4(c[r], c[r])));
+                            if (SRC && y == ys && r == sr) {
+                                const float add = a.idh3 * a.wavelet[a.nsteps - it.t];
+                                nv = mk4(lo(nv.a) + (se == 0 ? add : 0.f), hi(nv.a) + (se == 1 ? add : 0.f),
+                                         lo(nv.b) + (se == 2 ? add : 0.f), hi(nv.b) + (se == 3 ? add : 0.f));
+                            }
+                            if (r >= nrow) continue;
+                            const long long o = off + (long long)r * a.ldz;
+                            stq(out + o, nv);
+                            // (the box lies inside the updated cells)
+                            if (acc && xc + r >= a.acc_x0 && xc + r < a.acc_x1) {
+                                const q4 pr = ldq(Hy + T::HSLOT / 4 + r * T::HZ);  // the adjoint field's own value
+                                const q4 il = mul4(nv, nv);
+                                const q4 im = GRAD ? mul4(mul4(mul4(dup2(a.gscale), cv), pr), GRAD_DY ? lap : d[r])
+                                                   : mul4(nv, pr);
+                                float vi[4], vl[4];
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    vi[e] = (zmask >> e) & 1 ? get(im, e) : 0.0f;
+                                    vl[e] = (zmask >> e) & 1 ? get(il, e) : 0.0f;
+                                }
+                                red_add4(a.image + o, vi[0], vi[1], vi[2], vi[3]);
+                                red_add4(a.illum + o, vl[0], vl[1], vl[2], vl[3]);
+                            }
+                        }
+                        off += plane;
+                    }
+                    ++g;
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&done[cs]);
+                        st_release_cta(&sh.staged[warp], g);
+                    }
+                    if (++hs == SH) {
+                        hs = 0;
+                        hph ^= 1;
+                    }
+                    if (++cs == SC) cs = 0;
+                }
+                if (!ok) {
+                    loop_fail(&sh.abort);
+                    break;
                 }
             }
-            if (row_ok) {
-                const long long off = sh_off + y * plane + (long long)xc * a.ldz + zc;
-                *reinterpret_cast<float4 *>(a.Ps + off) = ps_new;
-                *reinterpret_cast<float4 *>(a.Prold + off) = pr_new;
-                if (acc && acc_row) {
-                    *reinterpret_cast<float4 *>(a.image + off) = img;
-                    *reinterpret_cast<float4 *>(a.illum + off) = ill;
-                }
-            }
-        }
-        __syncthreads();
-        if (abort_flag) break;
-        if (tid == 0) {
-            fence_proxy_async();
-            if (p < ya) {
-                if (p + SH <= pl) issue_h(p + SH, hs);
-            } else if (y >= ya) {
-                if (y + SH <= pl) issue_h(y + SH, hy);
-                if (y + SC < yb) issue_c(y + SC, cs);
-            }
-        }
-        if (++hs == SH) {
-            hs = 0;
-            hph ^= 1;
-        }
-        if (y >= ya && ++cs == SC) {
-            cs = 0;
-            cph ^= 1;
-        }
-    }
-
-    if (abort_flag && tid == 0) {
-        raise_status(kErrTimeout);
-        // (only the newest use of each slot can still be in flight)
-        for (int p = max(pf, h_issued - SH + 1); p <= h_issued; ++p)
-            mbar_wait(&hbar[(p - pf) % SH], ((p - pf) / SH) & 1);
-        for (int y = max(ya, c_issued - SC + 1); y <= c_issued; ++y)
-            mbar_wait(&cbar[(y - ya) % SC], ((y - ya) / SC) & 1);
+        };
+        if (warp < Loop<T, 2>::NWF)
+            compute(std::true_type{});
+        else
+            compute(std::false_type{});
     }
 }
 

@@ -21,7 +21,7 @@
  *     the ABI.  fwi_last_error() returns the message of the last failure.
  *   - One context per host thread; calls on one context are not re-entrant.
  *     Each context owns one CUDA stream (or uses the one set with
- *     fwi_set_stream) and its captured time-loop graphs.
+ *     fwi_set_stream).
  *   - The library keeps per-device state for the life of the process (kernel
  *     attributes, grid sizes, the no-alloc scratch address); cudaDeviceReset
  *     while it is loaded is not supported.
@@ -267,8 +267,8 @@ int fwi_write_binary(const char *file, const float *buf, int64_t n);
 int fwi_selftest_bounded_wait(fwi_ctx *ctx, int limit_ms);
 /* Device time [ms] of the last call's forward and backward time loops. */
 int fwi_last_timing(fwi_ctx *ctx, float *fwd_ms, float *bwd_ms);
-/* Kernel launches issued by the library since creation (graph nodes count
- * once per replay). */
+/* Kernel launches issued by the library since creation (the time loop of a
+ * batch is one launch). */
 int fwi_launch_count(fwi_ctx *ctx, int64_t *count);
 /* Stencil tile chosen by the autotuner for the forward and backward kernels
  * (index into the compiled tile table; -1 = not tuned yet). */
@@ -276,6 +276,7 @@ int fwi_get_tiles(fwi_ctx *ctx, int *fwd_tile, int *bwd_tile);
 int fwi_set_tiles(fwi_ctx *ctx, int fwd_tile, int bwd_tile);
 int fwi_autotune(fwi_ctx *ctx);
 int fwi_num_tiles(int *n);
+/* Cells of a forward tile (the backward kernel has shapes of its own). */
 int fwi_tile_shape(int tile, int *tz, int *tx);
 
 #ifdef __cplusplus
