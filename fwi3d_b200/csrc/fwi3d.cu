@@ -305,8 +305,9 @@ struct fwi_ctx {
     DevBuf<unsigned long long> ticket;
     DevBuf<long long> progress;
     DevBuf<BatchInfo> binfo;
-    DevBuf<double> partial, dsum;
-    DevBuf<unsigned int> ubits;
+    DevBuf<double> partial;
+    double *hsum = nullptr;  // mapped host memory
+    DevBuf<unsigned int> ubits, arrived;
     DevBuf<float> post;  // [nz*nx*ny] post-processing output
     DevBuf<float> stage;  // host-model uploads and padded downloads
     BlobCache blob_cache;
@@ -883,21 +884,43 @@ void fold_accumulators(fwi_ctx *c)
 }
 
 // FP64 sum of squares of obs-cal (and the residual) with fixed-order partials.
-constexpr int kRedThreads = 256, kRedBlocks = 296;
+constexpr int kRedThreads = 256, kRedBlocks = 148 * 6;
+
+// Blocks of a reduction of n elements: no more than there is work for.
+int reduction_blocks(long long n)
+{
+    return (int)std::max(1LL, std::min<long long>(kRedBlocks, (n / 4 + kQuads * kRedThreads - 1) / (kQuads * kRedThreads)));
+}
+
+// Whether every pointer (null ones included) allows 16-byte accesses.
+bool aligned16(const void *a, const void *b, const void *c = nullptr)
+{
+    return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15u) == 0;
+}
+
+// Scratch of the reductions: partials, block counter (0 between calls) and the
+// total in host memory that the GPU writes.
+void ensure_reduction(fwi_ctx *c)
+{
+    c->partial.ensure(kRedBlocks);
+    if (!c->arrived.p) {
+        c->arrived.ensure(1);
+        CK(cudaMemsetAsync(c->arrived.p, 0, sizeof(unsigned), c->stream));
+    }
+    if (!c->hsum) CK(cudaHostAlloc((void **)&c->hsum, sizeof(double), cudaHostAllocMapped));
+}
 
 double residual_impl(fwi_ctx *c, const float *d_obs, const float *d_cal, long long n, float *d_res)
 {
-    c->partial.ensure(kRedBlocks);
-    c->dsum.ensure(1);
-    residual_partial_kernel<kRedThreads><<<kRedBlocks, kRedThreads, 0, c->stream>>>(d_obs, d_cal, n, d_res,
-                                                                                   c->partial.p);
-    finish_sum_kernel<kRedThreads><<<1, kRedThreads, 0, c->stream>>>(c->partial.p, kRedBlocks, c->dsum.p);
+    ensure_reduction(c);
+    auto *kernel = aligned16(d_obs, d_cal, d_res) ? residual_partial_kernel<kRedThreads, true>
+                                                  : residual_partial_kernel<kRedThreads, false>;
+    kernel<<<reduction_blocks(n), kRedThreads, 0, c->stream>>>(d_obs, d_cal, n, d_res, c->partial.p, c->arrived.p,
+                                                               c->hsum);
     CK(cudaGetLastError());
-    c->launches += 2;
-    double s = 0;
-    CK(cudaMemcpyAsync(&s, c->dsum.p, sizeof s, cudaMemcpyDeviceToHost, c->stream));
+    ++c->launches;
     CK(cudaStreamSynchronize(c->stream));
-    return s;
+    return *c->hsum;
 }
 
 // Host Poisson-disk sampling (Bridson's method, as poissonDiskSampling of
@@ -1308,7 +1331,8 @@ int fwi_destroy(fwi_ctx *c)
     c->progress.release();
     c->binfo.release();
     c->partial.release();
-    c->dsum.release();
+    if (c->hsum) cudaFreeHost(c->hsum);
+    c->arrived.release();
     c->ubits.release();
     c->post.release();
     c->stage.release();
@@ -1713,14 +1737,13 @@ int fwi_dot_dev(fwi_ctx *c, const float *a, const float *b, int64_t n, double *o
 {
     if (!c || !a || !b || n < 0 || !out) return FWI_ERR_ARG;
     return guarded(c, [&] {
-        c->partial.ensure(kRedBlocks);
-        c->dsum.ensure(1);
-        dot_partial_kernel<kRedThreads><<<kRedBlocks, kRedThreads, 0, c->stream>>>(a, b, n, c->partial.p);
-        finish_sum_kernel<kRedThreads><<<1, kRedThreads, 0, c->stream>>>(c->partial.p, kRedBlocks, c->dsum.p);
+        ensure_reduction(c);
+        auto *kernel = aligned16(a, b) ? dot_partial_kernel<kRedThreads, true> : dot_partial_kernel<kRedThreads, false>;
+        kernel<<<reduction_blocks(n), kRedThreads, 0, c->stream>>>(a, b, n, c->partial.p, c->arrived.p, c->hsum);
         CK(cudaGetLastError());
-        c->launches += 2;
-        CK(cudaMemcpyAsync(out, c->dsum.p, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        ++c->launches;
         CK(cudaStreamSynchronize(c->stream));
+        *out = *c->hsum;
     });
 }
 
