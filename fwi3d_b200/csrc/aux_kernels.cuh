@@ -425,45 +425,97 @@ __global__ void rbc_background_kernel(float *__restrict__ vp, int nzz, int nxx, 
 }
 
 // Gaussian blobs (random_boundary_gp, src/modeling/modeling.cu:594-615): every
-// cell outside the strict inner box visits, in order, the blobs binned near it
-// and applies v += s A exp(-|x-c|^2 / (2 r^2)) followed by the clamp.  Blobs
+// cell outside the strict inner box visits, in order, the blobs near it and
+// applies v += s A exp(-|x-c|^2 / (2 r^2)) followed by the clamp.  Blobs
 // are truncated at 5 r (the omitted tail is below 4e-6 A).
 struct Blob {
     float x, y, z, r, amp;  // centre [m], radius [m], signed amplitude [m/s]
 };
 
-__global__ void rbc_blobs_kernel(float *__restrict__ vp, int nzz, int nxx, int nyy, int ldz, int nb,
-                                 float dh, const Blob *__restrict__ blobs,
-                                 const int *__restrict__ bin_first, const int *__restrict__ bin_list,
-                                 int nbz, int nbx, int nby, float bin_size, float vlo, float vhi)
+// A block owns a brick of 32 x bx x by cells.  It keeps the blobs whose 5 r ball reaches the
+// brick, in blob order, in shared memory; a warp then goes through its rows of
+// 32 z cells and drops, 32 blobs at a time, those that do not reach the row.
+// Bound by instruction issue: about 60 blobs act on a cell.  301^3 cells, 8000
+// blobs: 2.32 ms (4.45 ms with a thread per cell going through host-built bins).
+constexpr int kBrickZ = 32, kBrickThreads = 256, kBrickBlobs = 1024;
+
+// Whether the 5 r ball of a blob reaches a box, with a margin for rounding.
+__device__ __forceinline__ bool blob_reaches(const Blob &b, float z0, float z1, float x0, float x1, float y0, float y1)
 {
-    const long long n = (long long)ldz * nxx * nyy;
+    const float dz = fmaxf(fmaxf(z0 - b.z, b.z - z1), 0.0f), dx = fmaxf(fmaxf(x0 - b.x, b.x - x1), 0.0f),
+                dy = fmaxf(fmaxf(y0 - b.y, b.y - y1), 0.0f), e = 5.001f * b.r;
+    return dz * dz + dx * dx + dy * dy <= e * e;
+}
+
+__global__ void __launch_bounds__(kBrickThreads)
+    rbc_blobs_kernel(float *__restrict__ vp, int nzz, int nxx, int nyy, int ldz, int nb, float dh,
+                     const Blob *__restrict__ blobs, int nblob, float vlo, float vhi, int bx, int by)
+{
+    __shared__ Blob list[kBrickBlobs];
+    __shared__ float inv_r[kBrickBlobs];
+    __shared__ int warp_count[kBrickThreads / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int i0 = blockIdx.x * kBrickZ, j0 = blockIdx.y * bx, k0 = blockIdx.z * by;
+    const int i1 = min(i0 + kBrickZ, nzz) - 1, j1 = min(j0 + bx, nxx) - 1, k1 = min(k0 + by, nyy) - 1;
     const float fnb = nb * dh;
     const float xmax = (nxx - 1) * dh, ymax = (nyy - 1) * dh, zmax = (nzz - 1) * dh;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % ldz);
-        const long long r = c / ldz;
-        const int j = (int)(r % nxx), k = (int)(r / nxx);
-        if (i >= nzz) continue;
-        const float X = j * dh, Y = k * dh, Z = i * dh;
-        if (X > fnb && X < xmax - fnb && Y > fnb && Y < ymax - fnb && Z > fnb && Z < zmax - fnb)
-            continue;
-        const int bz = min((int)(Z / bin_size), nbz - 1);
-        const int bx = min((int)(X / bin_size), nbx - 1);
-        const int by = min((int)(Y / bin_size), nby - 1);
-        const int b = bz + nbz * (bx + nbx * by);
-        float v = vp[c];
-        for (int q = bin_first[b]; q < bin_first[b + 1]; ++q) {
-            const Blob bl = blobs[bin_list[q]];
-            const float ir = 1.0f / bl.r;
-            const float ex = (X - bl.x) * ir, ey = (Y - bl.y) * ir, ez = (Z - bl.z) * ir;
-            const float e2 = ex * ex + ey * ey + ez * ez;
-            if (e2 > 25.0f) continue;
-            v += bl.amp * expf(-0.5f * e2);
-            v = fminf(fmaxf(v, vlo), vhi);
+    if (i0 * dh > fnb && i1 * dh < zmax - fnb && j0 * dh > fnb && j1 * dh < xmax - fnb && k0 * dh > fnb &&
+        k1 * dh < ymax - fnb)
+        return;  // no cell outside the strict inner box
+
+    const int i = i0 + lane;
+    const float Z = i * dh;
+    int n = 0;  // blobs in the list
+    for (int b0 = 0; b0 < nblob; b0 += kBrickThreads) {
+        // append the blobs of this round that reach the brick
+        Blob b;
+        bool in = false;
+        if (b0 + tid < nblob) {
+            b = blobs[b0 + tid];
+            in = blob_reaches(b, i0 * dh, i1 * dh, j0 * dh, j1 * dh, k0 * dh, k1 * dh);
         }
-        vp[c] = v;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (lane == 0) warp_count[warp] = __popc(m);
+        __syncthreads();
+        int at = n;
+        for (int w = 0; w < kBrickThreads / 32; ++w) {
+            if (w < warp) at += warp_count[w];
+            n += warp_count[w];
+        }
+        if (in) {
+            at += __popc(m & ((1u << lane) - 1u));
+            list[at] = b;
+            inv_r[at] = 1.0f / b.r;
+        }
+        __syncthreads();
+        if (n <= kBrickBlobs - kBrickThreads && b0 + kBrickThreads < nblob) continue;
+        // apply the list
+        for (int row = warp; row < bx * by; row += kBrickThreads / 32) {
+            const int j = j0 + row % bx, k = k0 + row / bx;
+            if (j > j1 || k > k1) continue;
+            const float X = j * dh, Y = k * dh;
+            const bool mine = i <= i1 && !(X > fnb && X < xmax - fnb && Y > fnb && Y < ymax - fnb && Z > fnb &&
+                                           Z < zmax - fnb);
+            if (!__any_sync(0xffffffffu, mine)) continue;
+            const long long c = i + (long long)j * ldz + (long long)k * ldz * nxx;
+            float v = mine ? vp[c] : 0.0f;
+            for (int q0 = 0; q0 < n; q0 += 32) {
+                const bool near = q0 + lane < n && blob_reaches(list[q0 + lane], i0 * dh, i1 * dh, X, X, Y, Y);
+                for (unsigned todo = __ballot_sync(0xffffffffu, near); todo; todo &= todo - 1) {
+                    const int q = q0 + __ffs(todo) - 1;
+                    const Blob bl = list[q];
+                    const float ir = inv_r[q];
+                    const float ex = (X - bl.x) * ir, ey = (Y - bl.y) * ir, ez = (Z - bl.z) * ir;
+                    const float e2 = ex * ex + ey * ey + ez * ez;
+                    if (e2 > 25.0f) continue;
+                    v += bl.amp * expf(-0.5f * e2);
+                    v = fminf(fmaxf(v, vlo), vhi);
+                }
+            }
+            if (mine) vp[c] = v;
+        }
+        n = 0;
+        __syncthreads();
     }
 }
 
