@@ -14,6 +14,7 @@
 #include <cstring>
 #include <future>
 #include <map>
+#include <memory>
 #include <random>
 #include <string>
 #include <tuple>
@@ -906,6 +907,14 @@ double residual_impl(fwi_ctx *c, const float *d_obs, const float *d_cal, long lo
     return *c->hsum;
 }
 
+float host_uniform01(std::mt19937_64 &rng)
+{
+    // what std::uniform_real_distribution<float>(0, 1) gives, without its
+    // run-time logarithms
+    const float u = (float)rng() * 0x1p-64f;
+    return u < 1.0f ? u : 0x1.fffffep-1f;
+}
+
 // Host Poisson-disk sampling (Bridson's method, as poissonDiskSampling of
 // src/admin/admin.cpp:105-207: up to 30 candidates in the shell [r, 2r] around
 // a random active point), seeded and deterministic.  Only points outside the
@@ -919,35 +928,42 @@ std::vector<float> poisson_points(float xm, float ym, float zm, float r, const f
     const float cell = r / std::sqrt(3.0f);
     const int gx = std::max(1, (int)std::ceil(xm / cell)), gy = std::max(1, (int)std::ceil(ym / cell)),
               gz = std::max(1, (int)std::ceil(zm / cell));
-    std::vector<int> grid((size_t)gx * gy * gz, -1);
+    // background grid with two empty cells around it, so that no neighbour
+    // needs a bounds check; a free cell holds a point far away
+    struct Point {
+        float x, y, z;
+    };
+    const size_t sz = (size_t)gz + 4, sx = (size_t)gx + 4;
+    std::vector<Point> grid(sz * sx * ((size_t)gy + 4), Point{-1e30f, -1e30f, -1e30f});
     std::vector<float> pts;  // x, y, z triples
     std::vector<int> active;
-    std::uniform_real_distribution<float> U(0.0f, 1.0f);
-    // neighbour offsets whose nearest point can be closer than r
-    std::vector<int> offs;
+    // neighbour offsets whose nearest point can be closer than r, nearest
+    // first: most candidates fail, and then at one of the first
+    struct Off {
+        int d2;
+        std::ptrdiff_t at;
+    };
+    std::vector<Off> offs;
     for (int k = -2; k <= 2; ++k)
         for (int j = -2; j <= 2; ++j)
             for (int i = -2; i <= 2; ++i) {
                 auto g = [](int d) { return std::max(std::abs(d) - 1, 0); };
-                if (g(i) * g(i) + g(j) * g(j) + g(k) * g(k) < 3) {
-                    offs.push_back(i);
-                    offs.push_back(j);
-                    offs.push_back(k);
-                }
+                if (g(i) * g(i) + g(j) * g(j) + g(k) * g(k) < 3)
+                    offs.push_back({i * i + j * j + k * k,
+                                    i + (std::ptrdiff_t)sz * (j + (std::ptrdiff_t)sx * k)});
             }
-    auto cell_of = [&](float x, float y, float z, int &a, int &b, int &d) {
-        a = std::min(gx - 1, (int)(x / cell));
-        b = std::min(gy - 1, (int)(y / cell));
-        d = std::min(gz - 1, (int)(z / cell));
+    std::stable_sort(offs.begin(), offs.end(), [](const Off &a, const Off &b) { return a.d2 < b.d2; });
+    auto cell_of = [&](float x, float y, float z) {
+        const size_t a = std::min(gx - 1, (int)(x / cell)), b = std::min(gy - 1, (int)(y / cell)),
+                     d = std::min(gz - 1, (int)(z / cell));
+        return d + 2 + sz * (a + 2 + sx * (b + 2));
     };
     auto inside_keep_out = [&](float x, float y, float z) {
         return x > keep_out[0] && x < keep_out[1] && y > keep_out[2] && y < keep_out[3] && z > keep_out[4] &&
                z < keep_out[5];
     };
     auto insert = [&](float x, float y, float z) {
-        int a, b, d;
-        cell_of(x, y, z, a, b, d);
-        grid[d + (size_t)gz * (a + (size_t)gx * b)] = (int)(pts.size() / 3);
+        grid[cell_of(x, y, z)] = {x, y, z};
         pts.push_back(x);
         pts.push_back(y);
         pts.push_back(z);
@@ -956,41 +972,72 @@ std::vector<float> poisson_points(float xm, float ym, float zm, float r, const f
     auto valid = [&](float x, float y, float z) {
         if (x < 0 || y < 0 || z < 0 || x >= xm || y >= ym || z >= zm) return false;
         if (inside_keep_out(x, y, z)) return false;
-        int a, b, d;
-        cell_of(x, y, z, a, b, d);
-        for (size_t o = 0; o < offs.size(); o += 3) {
-            const int A = a + offs[o + 1], Bq = b + offs[o + 2], D = d + offs[o];
-            if (A < 0 || Bq < 0 || D < 0 || A >= gx || Bq >= gy || D >= gz) continue;
-            const int q = grid[D + (size_t)gz * (A + (size_t)gx * Bq)];
-            if (q < 0) continue;
-            const float dx = pts[3 * q] - x, dy = pts[3 * q + 1] - y, dz = pts[3 * q + 2] - z;
+        const Point *g = grid.data() + cell_of(x, y, z);
+        for (const Off &o : offs) {
+            const Point &q = g[o.at];
+            const float dx = q.x - x, dy = q.y - y, dz = q.z - z;
             if (dx * dx + dy * dy + dz * dz < r * r) return false;
         }
         return true;
     };
     for (int tries = 0; tries < 1000 && pts.empty(); ++tries) {
-        const float x = U(rng) * xm, y = U(rng) * ym, z = U(rng) * zm;
+        const float x = host_uniform01(rng) * xm, y = host_uniform01(rng) * ym, z = host_uniform01(rng) * zm;
         if (!inside_keep_out(x, y, z)) insert(x, y, z);
     }
-    const float pi = (float)M_PI;
+    // The draws do not depend on the points: one for the active point and
+    // three for each of its 30 candidates.  A second thread turns them into
+    // offsets, one chunk ahead of the conflict checks.
+    constexpr int kPicks = 256, kTries = 30;
+    struct Chunk {
+        std::mt19937_64 before;  // generator at the chunk's start
+        float pick[kPicks];
+        float off[kPicks][kTries][3];
+    };
+    auto fill = [r](Chunk *c, std::mt19937_64 *g) {
+        const float pi = (float)M_PI;
+        c->before = *g;
+        for (int p = 0; p < kPicks; ++p) {
+            c->pick[p] = host_uniform01(*g);
+            for (auto &o : c->off[p]) {
+                const float th = 2.0f * pi * host_uniform01(*g), ph = pi * host_uniform01(*g), rr = r * (1.0f + host_uniform01(*g));
+                o[0] = rr * sinf(ph) * cosf(th);
+                o[1] = rr * sinf(ph) * sinf(th);
+                o[2] = rr * cosf(ph);
+            }
+        }
+    };
+    std::mt19937_64 ahead = rng;
+    auto cur = std::make_unique<Chunk>(), next = std::make_unique<Chunk>();
+    std::future<void> filling = std::async(std::launch::async, fill, next.get(), &ahead);
+    int used = kPicks;
     while (!active.empty()) {
-        const int ai = (int)(U(rng) * active.size()) % (int)active.size();
+        if (used == kPicks) {
+            filling.get();
+            cur.swap(next);
+            filling = std::async(std::launch::async, fill, next.get(), &ahead);
+            used = 0;
+        }
+        const int ai = (int)(cur->pick[used] * active.size()) % (int)active.size();
         const int q = active[ai];
+        const float px = pts[3 * q], py = pts[3 * q + 1], pz = pts[3 * q + 2];
         bool found = false;
-        for (int tries = 0; tries < 30; ++tries) {
-            const float th = 2.0f * pi * U(rng), ph = pi * U(rng), rr = r * (1.0f + U(rng));
-            const float x = pts[3 * q] + rr * sinf(ph) * cosf(th);
-            const float y = pts[3 * q + 1] + rr * sinf(ph) * sinf(th);
-            const float z = pts[3 * q + 2] + rr * cosf(ph);
+        for (const auto &o : cur->off[used]) {
+            const float x = px + o[0], y = py + o[1], z = pz + o[2];
             if (valid(x, y, z)) {
                 insert(x, y, z);
                 found = true;
             }
         }
+        ++used;
         if (!found) {
             active[ai] = active.back();
             active.pop_back();
         }
+    }
+    filling.get();
+    if (!pts.empty()) {  // the generator as if every draw had been made here
+        rng = cur->before;
+        rng.discard((unsigned long long)used * (1 + 3 * kTries));
     }
     return pts;
 }
