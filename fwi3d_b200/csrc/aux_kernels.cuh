@@ -536,6 +536,36 @@ __global__ void coeff_kernel(const float *__restrict__ vp, float *__restrict__ o
     }
 }
 
+// Range of a velocity model and its first value that is not a positive number.
+// Positive floats order like their bits.
+struct VelocityRange {
+    unsigned long long bad;  // index, ~0 when there is none
+    unsigned lo, hi;         // bits
+};
+
+__global__ void velocity_range_kernel(const float *__restrict__ v, long long n, VelocityRange *__restrict__ out)
+{
+    unsigned lo = 0x7f800000u, hi = 0u;
+    unsigned long long bad = ~0ull;
+    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
+         c += (long long)gridDim.x * blockDim.x) {
+        const float x = v[c];
+        if (!isfinite(x) || x <= 0.0f) {
+            bad = min(bad, (unsigned long long)c);
+        } else {
+            lo = min(lo, __float_as_uint(x));
+            hi = max(hi, __float_as_uint(x));
+        }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(&out->lo, lo);
+        atomicMax(&out->hi, hi);
+    }
+    if (bad != ~0ull) atomicMin(&out->bad, bad);
+}
+
 // Largest |v| in a pitched field restricted to the real cells (CFL check).
 __global__ void max_abs_kernel(const float *__restrict__ v, long long n, int ldz, int nzz,
                                unsigned int *__restrict__ out_bits)

@@ -292,6 +292,7 @@ struct fwi_ctx {
     DevBuf<double> partial;
     double *hsum = nullptr;  // mapped host memory
     DevBuf<unsigned int> ubits, arrived;
+    DevBuf<VelocityRange> vrange;
     DevBuf<float> post;  // [nz*nx*ny] post-processing output
     DevBuf<float> stage;  // host-model uploads and padded downloads
     BlobCache blob_cache;
@@ -1070,6 +1071,26 @@ BlobSet make_blobs(BlobKey k)
     return out;
 }
 
+// Uploads a velocity model into `stage` and checks it there: every value a
+// positive number; the range goes to vmin, vmax.  The context's model does not
+// change before the check has passed.
+void stage_velocity(fwi_ctx *c, const float *vp, size_t n)
+{
+    c->stage.ensure(n);
+    c->vrange.ensure(1);
+    VelocityRange r{~0ull, 0x7f800000u, 0u};
+    CK(cudaMemcpyAsync(c->stage.p, vp, n * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->vrange.p, &r, sizeof r, cudaMemcpyHostToDevice, c->stream));
+    velocity_range_kernel<<<grid_blocks((long long)n), 256, 0, c->stream>>>(c->stage.p, (long long)n, c->vrange.p);
+    CK(cudaGetLastError());
+    ++c->launches;
+    CK(cudaMemcpyAsync(&r, c->vrange.p, sizeof r, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    if (r.bad < n) fail(FWI_ERR_NUMERIC, "velocity[%llu] = %g is not a positive number", r.bad, vp[r.bad]);
+    memcpy(&c->vmin, &r.lo, sizeof(float));
+    memcpy(&c->vmax, &r.hi, sizeof(float));
+}
+
 float device_max_abs(fwi_ctx *c, const float *v, long long n)
 {
     c->ubits.ensure(1);
@@ -1335,6 +1356,7 @@ int fwi_destroy(fwi_ctx *c)
     c->partial.release();
     if (c->hsum) cudaFreeHost(c->hsum);
     c->arrived.release();
+    c->vrange.release();
     c->ubits.release();
     c->post.release();
     c->stage.release();
@@ -1376,17 +1398,7 @@ int fwi_set_velocity(fwi_ctx *c, const float *vp)
 {
     if (!c || !vp) return FWI_ERR_ARG;
     return guarded(c, [&] {
-        const size_t n = (size_t)c->g.nz * c->g.nx * c->g.ny;
-        float lo = 1e30f, hi = -1e30f;
-        for (size_t i = 0; i < n; ++i) {
-            if (!std::isfinite(vp[i]) || vp[i] <= 0) fail(FWI_ERR_NUMERIC, "velocity[%zu] = %g is not a positive number", i, vp[i]);
-            lo = std::min(lo, vp[i]);
-            hi = std::max(hi, vp[i]);
-        }
-        c->vmin = lo;
-        c->vmax = hi;
-        c->stage.ensure(n);
-        CK(cudaMemcpyAsync(c->stage.p, vp, n * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+        stage_velocity(c, vp, (size_t)c->g.nz * c->g.nx * c->g.ny);
         pad_edges_kernel<<<grid_blocks(c->vol), 256, 0, c->stream>>>(c->stage.p, c->g.nz, c->g.nx, c->g.ny, c->g.nb,
                                                                      c->nzz, c->nxx, c->nyy, c->ldz, c->vp.p);
         CK(cudaGetLastError());
@@ -1402,17 +1414,7 @@ int fwi_set_padded_velocity(fwi_ctx *c, const float *vpp)
 {
     if (!c || !vpp) return FWI_ERR_ARG;
     return guarded(c, [&] {
-        const size_t n = (size_t)c->nzz * c->nxx * c->nyy;
-        float lo = 1e30f, hi = -1e30f;
-        for (size_t i = 0; i < n; ++i) {
-            if (!std::isfinite(vpp[i]) || vpp[i] <= 0) fail(FWI_ERR_NUMERIC, "velocity[%zu] = %g is not a positive number", i, vpp[i]);
-            lo = std::min(lo, vpp[i]);
-            hi = std::max(hi, vpp[i]);
-        }
-        c->vmin = lo;
-        c->vmax = hi;
-        c->stage.ensure(n);
-        CK(cudaMemcpyAsync(c->stage.p, vpp, n * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+        stage_velocity(c, vpp, (size_t)c->nzz * c->nxx * c->nyy);
         dense_to_pitched_kernel<<<grid_blocks(c->vol), 256, 0, c->stream>>>(c->stage.p, c->nzz, c->nxx, c->nyy,
                                                                             c->ldz, c->vp.p);
         CK(cudaGetLastError());
