@@ -47,9 +47,15 @@ struct CellLists {
 
 // Progress of the items of a time-loop kernel: an item is one step of one
 // column of one shot; it publishes the y planes it has stored.
+// Every counter has a 128-byte line to itself: up to five columns poll it, and
+// the line of several counters was what the hand-over between steps waited for
+// (146 x 123 x 101 cells, forward: 10.4 us a step with counters side by side,
+// 7.3 with one per 32-byte sector, 7.0 with one per line).
+constexpr int kCounterStride = 16;
+
 struct LoopProgress {
     unsigned long long *ticket;   // next item
-    long long *done;              // [shot][step % ring][column]: step * nyy + planes stored
+    long long *done;              // [shot][step % ring][column] (kCounterStride apart): step * nyy + planes stored
     int ring;
     int shots;                    // shots whose steps interleave in the ticket order
 };

@@ -44,11 +44,11 @@ struct TileSpec {
     double cost;
 };
 constexpr TileSpec kFwdTiles[kNumTiles] = {
-    {16, 8, 7, 4, 2.78},  {19, 20, 7, 2, 3.00}, {32, 24, 7, 1, 2.24}, {24, 16, 7, 2, 2.70}, {25, 24, 9, 1, 2.56},
-    {37, 24, 7, 1, 2.19}, {37, 18, 8, 1, 2.29}, {12, 8, 8, 4, 3.24},  {25, 32, 7, 1, 2.66}, {49, 16, 7, 1, 2.55}};
+    {16, 8, 7, 4, 2.55},  {19, 20, 7, 2, 2.47}, {32, 24, 7, 1, 2.20}, {24, 16, 7, 2, 2.35}, {25, 24, 9, 1, 2.25},
+    {37, 24, 7, 1, 2.35}, {37, 18, 8, 1, 2.22}, {12, 8, 8, 4, 3.05},  {25, 32, 7, 1, 2.30}, {49, 16, 7, 1, 2.20}};
 constexpr TileSpec kBwdTiles[kNumTiles] = {
     {16, 12, 7, 2, 5.40}, {19, 22, 7, 1, 5.30}, {16, 28, 7, 1, 4.90}, {25, 14, 8, 1, 5.20}, {25, 16, 7, 1, 5.20},
-    {19, 18, 8, 1, 5.40}, {8, 8, 7, 4, 6.00},   {37, 10, 7, 1, 4.72}, {12, 16, 7, 2, 5.60}, {37, 8, 8, 1, 4.75}};
+    {19, 18, 8, 1, 5.40}, {8, 8, 7, 4, 6.00},   {37, 10, 7, 1, 4.72}, {12, 16, 7, 2, 5.20}, {37, 8, 8, 1, 4.75}};
 
 struct KInfo {
     const void *fn = nullptr;
@@ -522,7 +522,7 @@ void prepare_kernel(const KInfo &k)
 }
 
 // Tile before tuning: the one whose covered cells, updated or not, cost least.
-// Within 4 % of the best tile on 9 of 12 measured grids, at most 13 % off on
+// Within 4 % of the best tile on 10 of 13 measured grids, at most 12 % off on
 // small ones, where the hand-over between steps counts more than the cells.
 int default_tile(const fwi_ctx *c, bool backward)
 {
@@ -581,7 +581,7 @@ void plan_loop(fwi_ctx *c, L &l, int n)
     p.shots = std::min(n, std::max(1, (ctas + l.a.ncol * steps - 1) / (l.a.ncol * steps)));
     l.grid = dim3(std::min<long long>(ctas, (long long)p.shots * l.a.ncol * (c->nyy / 4 + 1)));
     c->ticket.ensure(1);
-    c->progress.ensure((size_t)n * p.ring * l.a.ncol);
+    c->progress.ensure((size_t)n * p.ring * l.a.ncol * kCounterStride);
     p.ticket = c->ticket.p;
     p.done = c->progress.p;
 }
@@ -591,7 +591,8 @@ template <class L>
 void launch_loop(fwi_ctx *c, L &l, int n)
 {
     CK(cudaMemsetAsync(l.a.prog.ticket, 0, sizeof(unsigned long long), c->stream));
-    CK(cudaMemsetAsync(l.a.prog.done, 0, (size_t)n * l.a.prog.ring * l.a.ncol * sizeof(long long), c->stream));
+    CK(cudaMemsetAsync(l.a.prog.done, 0, (size_t)n * l.a.prog.ring * l.a.ncol * kCounterStride * sizeof(long long),
+                       c->stream));
     void *args[] = {&l.m, &l.a};
     CK(cudaLaunchKernel(l.k.fn, l.grid, dim3(l.k.threads), args, l.k.smem, c->stream));
     ++c->launches;

@@ -306,6 +306,11 @@ __device__ __forceinline__ int dependency_column(int lane, int col, int ntz, int
     }
 }
 
+__device__ __forceinline__ long long *counter(const LoopProgress &prog, int ncol, int shot, int t, int col)
+{
+    return prog.done + (((long long)shot * prog.ring + t % prog.ring) * ncol + col) * kCounterStride;
+}
+
 // Bounded wait of a warp until every lane's counter has reached `need`; `seen`
 // is the lane's last reading.
 __device__ __forceinline__ bool wait_columns(const long long *p, long long need, long long &seen,
@@ -370,8 +375,7 @@ __device__ __forceinline__ void loop_producer(LoopShared<NW> &sh, uint64_t *full
         }
         const Item it = item_of((long long)tk, geo.nshot, prog.shots, geo.nsteps, geo.ncol);
         const int dep = it.t > 0 ? dependency_column(lane, it.col, geo.ntz, geo.ncol) : -1;
-        const long long *dp =
-            prog.done + ((long long)it.shot * prog.ring + (it.t + prog.ring - 1) % prog.ring) * geo.ncol + max(dep, 0);
+        const long long *dp = counter(prog, geo.ncol, it.shot, it.t + prog.ring - 1, max(dep, 0));
         long long seen = dep >= 0 ? 0 : 0x7fffffffffffffffll;
         const long long base = (long long)(it.t - 1) * geo.nyy;
         const auto state = start(it);
@@ -436,7 +440,7 @@ __device__ __forceinline__ void loop_publisher(LoopShared<NW> &sh, const LoopGeo
         __syncwarp();
         if (lane == 0) st_release_cta(&sh.items_read, item + 1);
         const Item it = item_of(tk, geo.nshot, prog.shots, geo.nsteps, geo.ncol);
-        long long *dp = prog.done + ((long long)it.shot * prog.ring + it.t % prog.ring) * geo.ncol + it.col;
+        long long *dp = counter(prog, geo.ncol, it.shot, it.t, it.col);
         const long long base = (long long)it.t * geo.nyy;
         auto state = start(it);
         int published = 4;  // the first four planes are never written
@@ -528,36 +532,51 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
                 }
             });
     } else if (warp == NW + 1) {
-        // after publishing: samples of the level the item stores, u^(t+1)
+        // After publishing: samples of the level the item stores, u^(t+1).
+        // Lane l holds entry u + l of the column's list, looked up ahead of
+        // its plane.
         struct State {
-            int u, last, sample;
+            int u, last, sample, y, first, end;
+            long long cell;
             const float *F;
         };
         const int nrec = a.binfo->R;
+        auto load = [&](State &st) {
+            const int e = st.u + lane;
+            st.y = 0x7fffffff;
+            if (e < st.last) {
+                st.y = a.rec.y[e];
+                st.cell = a.rec.cell[e];
+                st.first = a.rec.first[e];
+                st.end = a.rec.first[e + 1];
+            }
+        };
         loop_publisher(
             sh, geo, a.prog, lane,
             [&](const Item &it) {
-                State st{0, 0, it.t + 1 - a.tlag, a.F[1 - (it.t & 1)]};
+                State st{0, 0, it.t + 1 - a.tlag, 0, 0, 0, 0, a.F[1 - (it.t & 1)]};
                 if (st.sample > 0 && it.t + 1 < a.nsteps) {
                     st.u = a.rec.col_first[it.shot * a.ncol + it.col];
                     st.last = a.rec.col_first[it.shot * a.ncol + it.col + 1];
                 }
+                load(st);
                 return st;
             },
             [](State &, int) {},
             [&](State &st, int n) {
-                while (st.u < st.last) {
-                    const int e = st.u + lane;
-                    const bool mine = e < st.last && a.rec.y[min(e, st.last - 1)] < n;
+                for (;;) {
+                    const bool mine = st.y < n;
+                    const int got = __popc(__ballot_sync(0xffffffffu, mine));
+                    if (got == 0) break;
                     if (mine) {
-                        const float v = __ldcg(st.F + a.rec.cell[e]);
-                        for (int k = a.rec.first[e]; k < a.rec.first[e + 1]; ++k) {
+                        const float v = __ldcg(st.F + st.cell);
+                        for (int k = st.first; k < st.end; ++k) {
                             const int r = a.rec.rid[k];
                             a.seis_tm[(long long)st.sample * nrec + r] = a.rec_damp[r] * v;
                         }
                     }
-                    const int got = __popc(__ballot_sync(0xffffffffu, mine));
                     st.u += got;
+                    load(st);
                     if (got < 32) break;
                 }
             });
