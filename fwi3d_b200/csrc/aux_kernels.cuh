@@ -433,10 +433,12 @@ struct Blob {
 };
 
 // A block owns a brick of 32 x bx x by cells.  It keeps the blobs whose 5 r ball reaches the
-// brick, in blob order, in shared memory; a warp then goes through its rows of
-// 32 z cells and drops, 32 blobs at a time, those that do not reach the row.
+// brick, in blob order, in shared memory; a warp then goes through its patches
+// of 8 x 4 (z, x) cells and drops, 32 blobs at a time, those that do not reach
+// the patch.
 // Bound by instruction issue: about 60 blobs act on a cell.  301^3 cells, 8000
-// blobs: 2.32 ms (4.45 ms with a thread per cell going through host-built bins).
+// blobs: 1.83 ms (2.32 ms with rows of 32 z cells as patches, 4.45 ms with a
+// thread per cell going through host-built bins).
 constexpr int kBrickZ = 32, kBrickThreads = 256, kBrickBlobs = 1024;
 
 // Whether the 5 r ball of a blob reaches a box, with a margin for rounding.
@@ -463,8 +465,6 @@ __global__ void __launch_bounds__(kBrickThreads)
         k1 * dh < ymax - fnb)
         return;  // no cell outside the strict inner box
 
-    const int i = i0 + lane;
-    const float Z = i * dh;
     int n = 0;  // blobs in the list
     for (int b0 = 0; b0 < nblob; b0 += kBrickThreads) {
         // append the blobs of this round that reach the brick
@@ -489,18 +489,21 @@ __global__ void __launch_bounds__(kBrickThreads)
         }
         __syncthreads();
         if (n <= kBrickBlobs - kBrickThreads && b0 + kBrickThreads < nblob) continue;
-        // apply the list
-        for (int row = warp; row < bx * by; row += kBrickThreads / 32) {
-            const int j = j0 + row % bx, k = k0 + row / bx;
-            if (j > j1 || k > k1) continue;
-            const float X = j * dh, Y = k * dh;
-            const bool mine = i <= i1 && !(X > fnb && X < xmax - fnb && Y > fnb && Y < ymax - fnb && Z > fnb &&
-                                           Z < zmax - fnb);
+        // apply the list, patch by patch
+        const int px = bx / 4;
+        for (int patch = warp; patch < kBrickZ / 8 * px * by; patch += kBrickThreads / 32) {
+            const int pi = i0 + patch % (kBrickZ / 8) * 8, pj = j0 + patch / (kBrickZ / 8) % px * 4,
+                      k = k0 + patch / (kBrickZ / 8 * px);
+            const int i = pi + (lane & 7), j = pj + (lane >> 3);
+            const float X = j * dh, Y = k * dh, Z = i * dh;
+            const bool mine = i <= i1 && j <= j1 && k <= k1 &&
+                              !(X > fnb && X < xmax - fnb && Y > fnb && Y < ymax - fnb && Z > fnb && Z < zmax - fnb);
             if (!__any_sync(0xffffffffu, mine)) continue;
             const long long c = i + (long long)j * ldz + (long long)k * ldz * nxx;
             float v = mine ? vp[c] : 0.0f;
             for (int q0 = 0; q0 < n; q0 += 32) {
-                const bool near = q0 + lane < n && blob_reaches(list[q0 + lane], i0 * dh, i1 * dh, X, X, Y, Y);
+                const bool near = q0 + lane < n && blob_reaches(list[q0 + lane], pi * dh, (pi + 7) * dh, pj * dh,
+                                                                (pj + 3) * dh, Y, Y);
                 for (unsigned todo = __ballot_sync(0xffffffffu, near); todo; todo &= todo - 1) {
                     const int q = q0 + __ffs(todo) - 1;
                     const Blob bl = list[q];
