@@ -650,17 +650,24 @@ __global__ void __launch_bounds__(wg::THREADS, wg::CTAS_PER_SM)
     }
 }
 
-// Fixed-order sum of per-CTA partials: out[i] = sum_b part[b][i].  A block
-// is 32 entries x 8 slices of b; slice y sums b = y, y+8, ... in order, then
-// the eight slice sums are added in order.
+// Fixed-order sums of the per-CTA partials of a layer's weight and bias
+// gradients, times `scale`: out[i] = scale * sum_b part[b][i].  A block is 32
+// entries x 8 slices of b; slice y sums b = y, y+8, ... in order, then the
+// eight slice sums are added in order.  The last block has the biases.
 constexpr int RED_X = 32, RED_Y = 8;
+constexpr int RED_WBLOCKS = (WSZ + RED_X - 1) / RED_X;
 
 __global__ void __launch_bounds__(RED_X * RED_Y)
-    reduce_partials_kernel(const float *__restrict__ part, int nb, int n, float *__restrict__ out)
+    reduce_partials_kernel(const float *__restrict__ wpart, const float *__restrict__ bpart, int nb, float scale,
+                           float *__restrict__ gw, float *__restrict__ gb)
 {
     __shared__ float red[RED_Y][RED_X];
+    const bool weights = blockIdx.x < RED_WBLOCKS;
+    const float *part = weights ? wpart : bpart;
+    float *out = weights ? gw : gb;
+    const int n = weights ? WSZ : CH;
     const int x = threadIdx.x % RED_X, y = threadIdx.x / RED_X;
-    const int i = blockIdx.x * RED_X + x;
+    const int i = (weights ? blockIdx.x * RED_X : 0) + x;
     float s = 0.0f;
     if (i < n)
         for (int b = y; b < nb; b += RED_Y) s += part[(long long)b * n + i];
@@ -669,7 +676,7 @@ __global__ void __launch_bounds__(RED_X * RED_Y)
     if (y == 0 && i < n) {
         float t = red[0][x];
         for (int k = 1; k < RED_Y; ++k) t += red[k][x];
-        out[i] = t;
+        out[i] = t * scale;
     }
 }
 
@@ -729,38 +736,43 @@ __global__ void sum_f64_kernel(const double *__restrict__ p, int n, double *__re
 
 // Adam on the FP32 master weights (Kingma & Ba, 2015), then the BF16 copies:
 // forward layout [t][co][ci] and the data-gradient layout [t][ci][co].  The
-// mask keeps the padding channels of the first and last layer at zero.
-__global__ void adam_kernel(int n, float *__restrict__ w, const float *__restrict__ gw, float *__restrict__ m,
-                            float *__restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2,
-                            const float *__restrict__ mask, __nv_bfloat16 *__restrict__ wb,
-                            __nv_bfloat16 *__restrict__ wt)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float g = gw[i] * mask[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * g;
-        const float vi = b2 * v[i] + (1.0f - b2) * g * g;
-        m[i] = mi;
-        v[i] = vi;
-        const float wi = (w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps)) * mask[i];
-        w[i] = wi;
-        if (wb) {
-            wb[i] = __float2bfloat16_rn(wi);
-            const int t = i / (CH * CH), co = (i / CH) % CH, ci = i % CH;
-            wt[t * CH * CH + ci * CH + co] = __float2bfloat16_rn(wi);
-        }
-    }
-}
+// mask keeps the padding channels of the first and last layer at zero.  One
+// launch updates every layer (blockIdx.y); it changes nothing once a kernel of
+// the step has given up a wait.
+struct AdamLayer {
+    float *w, *gw, *mw, *vw, *mask, *b, *gb, *mb, *vb;
+    __nv_bfloat16 *wb, *wt;
+    int nreal;  // biases in use
+};
+struct AdamArgs {
+    AdamLayer layer[NL];
+    float lr, b1, b2, eps, c1, c2;
+};
 
-__global__ void bias_adam_kernel(int n, float *__restrict__ b, const float *__restrict__ gb, float *__restrict__ m,
-                                 float *__restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2,
-                                 int nreal)
+__global__ void adam_kernel(const __grid_constant__ AdamArgs a)
 {
-    const int i = threadIdx.x;
-    if (i < n) {
-        const float g = i < nreal ? gb[i] : 0.0f;
-        m[i] = b1 * m[i] + (1.0f - b1) * g;
-        v[i] = b2 * v[i] + (1.0f - b2) * g * g;
-        b[i] = i < nreal ? b[i] - lr * (m[i] / c1) / (sqrtf(v[i] / c2) + eps) : 0.0f;
+    if (*(volatile unsigned int *)&g_cnn_status) return;
+    const AdamLayer &l = a.layer[blockIdx.y];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < WSZ) {
+        const float g = l.gw[i] * l.mask[i];
+        const float mi = a.b1 * l.mw[i] + (1.0f - a.b1) * g;
+        const float vi = a.b2 * l.vw[i] + (1.0f - a.b2) * g * g;
+        l.mw[i] = mi;
+        l.vw[i] = vi;
+        const float wi = (l.w[i] - a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps)) * l.mask[i];
+        l.w[i] = wi;
+        l.wb[i] = __float2bfloat16_rn(wi);
+        const int t = i / (CH * CH), co = (i / CH) % CH, ci = i % CH;
+        l.wt[t * CH * CH + ci * CH + co] = __float2bfloat16_rn(wi);
+    }
+    if (i < CH) {
+        const float g = i < l.nreal ? l.gb[i] : 0.0f;
+        const float mi = a.b1 * l.mb[i] + (1.0f - a.b1) * g;
+        const float vi = a.b2 * l.vb[i] + (1.0f - a.b2) * g * g;
+        l.mb[i] = mi;
+        l.vb[i] = vi;
+        l.b[i] = i < l.nreal ? l.b[i] - a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps) : 0.0f;
     }
 }
 
@@ -791,8 +803,9 @@ struct Buf {
 struct fwi_cnn {
     Geo g{};
     cudaStream_t stream = nullptr;
-    Buf<float> w32[NL], gw[NL], mw[NL], vw[NL], mask[NL];
-    Buf<float> b32[NL], gb[NL], mb[NL], vb[NL];
+    Buf<float> w32[NL], mw[NL], vw[NL], mask[NL];
+    Buf<float> b32[NL], mb[NL], vb[NL];
+    Buf<float> gw, gb;  // gradients of all layers, [NL][WSZ] and [NL][CH]
     Buf<__nv_bfloat16> wb[NL], wt[NL];
     Buf<__nv_bfloat16> act[NL];  // act[0] input, act[l] = output of layer l-1 (l = 1..3)
     Buf<__nv_bfloat16> dg[2];    // data gradients, ping-pong
@@ -951,9 +964,9 @@ int forward_impl(fwi_cnn *n)
     return FWI_OK;
 }
 
-// Weight and bias gradients of one layer into gw / gb: x = the layer's input
+// Weight and bias gradients of one layer, times scale, into gw / gb: x = the layer's input
 // rows, dy = the gradient rows of its output.
-int launch_wgrad(fwi_cnn *n, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, float *gw, float *gb)
+int launch_wgrad(fwi_cnn *n, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, float scale, float *gw, float *gb)
 {
     static int ctas_of[kMaxDevices] = {};  // per device, under a lock, as in launch_conv
     static std::mutex lock_of[kMaxDevices];
@@ -987,8 +1000,8 @@ int launch_wgrad(fwi_cnn *n, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, fl
     const int grid = (a.ntiles + a.tiles_per_cta - 1) / a.tiles_per_cta;
     wgrad_tc_kernel<<<grid, wg::THREADS, wg::SMEM, n->stream>>>(mx, mdy, a);
     CNN_CK(cudaGetLastError());
-    reduce_partials_kernel<<<(WSZ + RED_X - 1) / RED_X, RED_X * RED_Y, 0, n->stream>>>(n->partial.p, grid, WSZ, gw);
-    reduce_partials_kernel<<<1, RED_X * RED_Y, 0, n->stream>>>(n->bpartial.p, grid, CH, gb);
+    reduce_partials_kernel<<<RED_WBLOCKS + 1, RED_X * RED_Y, 0, n->stream>>>(n->partial.p, n->bpartial.p, grid, scale,
+                                                                            gw, gb);
     CNN_CK(cudaGetLastError());
     return FWI_OK;
 }
@@ -1025,6 +1038,8 @@ int ensure_volume(fwi_cnn *n, int nz, int nx, int ny)
     CNN_CK(n->pred.ensure(g.V));
     CNN_CK(n->partial.ensure((size_t)kMaxPartials * WSZ));
     CNN_CK(n->bpartial.ensure((size_t)kMaxPartials * CH));
+    CNN_CK(n->gw.ensure((size_t)NL * WSZ));
+    CNN_CK(n->gb.ensure((size_t)NL * CH));
     CNN_CK(n->lpart.ensure(1024));
     CNN_CK(n->lsum.ensure(1));
     return FWI_OK;
@@ -1072,9 +1087,9 @@ int fwi_cnn_create(uint64_t seed, fwi_cnn **out)
                     w[i] = N(rng) * (l == NL - 1 ? 0.1f : 1.0f);
                     mk[i] = 1.0f;
                 }
-        for (auto *b : {&n->w32[l], &n->gw[l], &n->mw[l], &n->vw[l], &n->mask[l]})
+        for (auto *b : {&n->w32[l], &n->mw[l], &n->vw[l], &n->mask[l]})
             if (b->ensure(WSZ) != cudaSuccess) st = FWI_ERR_ALLOC;
-        for (auto *b : {&n->b32[l], &n->gb[l], &n->mb[l], &n->vb[l]})
+        for (auto *b : {&n->b32[l], &n->mb[l], &n->vb[l]})
             if (b->ensure(CH) != cudaSuccess) st = FWI_ERR_ALLOC;
         for (auto *b : {&n->wb[l], &n->wt[l]})
             if (b->ensure(WSZ) != cudaSuccess) st = FWI_ERR_ALLOC;
@@ -1100,13 +1115,14 @@ int fwi_cnn_destroy(fwi_cnn *n)
 {
     if (!n) return FWI_ERR_ARG;
     for (int l = 0; l < NL; ++l) {
-        for (auto *b : {&n->w32[l], &n->gw[l], &n->mw[l], &n->vw[l], &n->mask[l], &n->b32[l], &n->gb[l], &n->mb[l],
-                        &n->vb[l]})
+        for (auto *b : {&n->w32[l], &n->mw[l], &n->vw[l], &n->mask[l], &n->b32[l], &n->mb[l], &n->vb[l]})
             b->release();
         n->wb[l].release();
         n->wt[l].release();
         n->act[l].release();
     }
+    n->gw.release();
+    n->gb.release();
     n->dg[0].release();
     n->dg[1].release();
     n->pred.release();
@@ -1197,10 +1213,12 @@ int fwi_cnn_train_step(fwi_cnn *n, int nz, int nx, int ny, const float *d_in, co
     const int lblk = 1024;
     mse_kernel<<<lblk, 256, 0, n->stream>>>(g, n->pred.p, d_target, 1.0f, n->dg[0].p, n->lpart.p);
     sum_f64_kernel<<<1, 32, 0, n->stream>>>(n->lpart.p, lblk, n->lsum.p);
+    // (d, not d/V: the parameter gradients are scaled by 1/V as they are summed)
+    const float inv = 1.0f / (float)V;
     int cur = 0;
     for (int l = NL - 1; l >= 0; --l) {
         // weight and bias gradients of layer l: input act[l], output gradient dg[cur]
-        st = launch_wgrad(n, n->act[l].p, n->dg[cur].p, n->gw[l].p, n->gb[l].p);
+        st = launch_wgrad(n, n->act[l].p, n->dg[cur].p, inv, n->gw.p + (size_t)l * WSZ, n->gb.p + (size_t)l * CH);
         if (st != FWI_OK) return st;
         if (l > 0) {
             // data gradient through layer l, masked by the ReLU of act[l]
@@ -1209,44 +1227,32 @@ int fwi_cnn_train_step(fwi_cnn *n, int nz, int nx, int ny, const float *d_in, co
             cur = 1 - cur;
         }
     }
+    if (lr > 0) {
+        const int step = n->adam_step + 1;
+        AdamArgs a;
+        a.lr = lr;
+        a.b1 = 0.9f;
+        a.b2 = 0.999f;
+        a.eps = 1e-8f;
+        a.c1 = 1.0f - powf(a.b1, (float)step);
+        a.c2 = 1.0f - powf(a.b2, (float)step);
+        for (int l = 0; l < NL; ++l)
+            a.layer[l] = {n->w32[l].p, n->gw.p + (size_t)l * WSZ, n->mw[l].p, n->vw[l].p, n->mask[l].p, n->b32[l].p,
+                          n->gb.p + (size_t)l * CH, n->mb[l].p, n->vb[l].p, n->wb[l].p, n->wt[l].p, COUT[l]};
+        adam_kernel<<<dim3((WSZ + 255) / 256, NL), 256, 0, n->stream>>>(a);
+    }
     CNN_CK(cudaGetLastError());
     double lsum = 0.0;
     CNN_CK(cudaMemcpyAsync(&lsum, n->lsum.p, sizeof(double), cudaMemcpyDeviceToHost, n->stream));
+    if (grad_w)
+        CNN_CK(cudaMemcpyAsync(grad_w, n->gw.p, (size_t)NL * WSZ * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
+    if (grad_b)
+        CNN_CK(cudaMemcpyAsync(grad_b, n->gb.p, (size_t)NL * CH * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
     CNN_CK(cudaStreamSynchronize(n->stream));
     st = check_cnn_status(n);
     if (st != FWI_OK) return st;
+    if (lr > 0) ++n->adam_step;
     if (loss) *loss = 0.5 * lsum / (double)V;
-    // the loss gradient was d (not d/V): scale the parameter gradients by 1/V
-    const float inv = 1.0f / (float)V;
-    std::vector<float> tmp(WSZ), tb(CH);
-    for (int l = 0; l < NL; ++l) {
-        if (grad_w || lr > 0) {
-            CNN_CK(cudaMemcpy(tmp.data(), n->gw[l].p, WSZ * sizeof(float), cudaMemcpyDeviceToHost));
-            for (auto &x : tmp) x *= inv;
-            if (grad_w) memcpy(grad_w + (size_t)l * WSZ, tmp.data(), WSZ * sizeof(float));
-            CNN_CK(cudaMemcpy(n->gw[l].p, tmp.data(), WSZ * sizeof(float), cudaMemcpyHostToDevice));
-        }
-        if (grad_b || lr > 0) {
-            CNN_CK(cudaMemcpy(tb.data(), n->gb[l].p, CH * sizeof(float), cudaMemcpyDeviceToHost));
-            for (auto &x : tb) x *= inv;
-            if (grad_b) memcpy(grad_b + (size_t)l * CH, tb.data(), CH * sizeof(float));
-            CNN_CK(cudaMemcpy(n->gb[l].p, tb.data(), CH * sizeof(float), cudaMemcpyHostToDevice));
-        }
-    }
-    if (lr > 0) {
-        ++n->adam_step;
-        const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-        const float c1 = 1.0f - powf(b1, (float)n->adam_step), c2 = 1.0f - powf(b2, (float)n->adam_step);
-        for (int l = 0; l < NL; ++l) {
-            adam_kernel<<<(WSZ + 255) / 256, 256, 0, n->stream>>>(WSZ, n->w32[l].p, n->gw[l].p, n->mw[l].p,
-                                                                  n->vw[l].p, lr, b1, b2, eps, c1, c2, n->mask[l].p,
-                                                                  n->wb[l].p, n->wt[l].p);
-            bias_adam_kernel<<<1, CH, 0, n->stream>>>(CH, n->b32[l].p, n->gb[l].p, n->mb[l].p, n->vb[l].p, lr, b1,
-                                                      b2, eps, c1, c2, COUT[l]);
-        }
-        CNN_CK(cudaGetLastError());
-        CNN_CK(cudaStreamSynchronize(n->stream));
-    }
     return FWI_OK;
 }
 
