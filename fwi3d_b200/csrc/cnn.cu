@@ -680,39 +680,61 @@ __global__ void __launch_bounds__(RED_X * RED_Y)
     }
 }
 
+// The two kernels below write 32-byte rows and are bound by HBM: a thread
+// writes one 16-byte half of a row, so that a warp's stores are contiguous, and
+// has kHalves rows in flight.  301 x 301 x 151 voxels: packing
+// 0.121 ms, 5.1 TB/s (0.196 ms with a thread per row), loss gradient 0.125 ms
+// (0.138 ms).
+constexpr int kHalves = 4;
+
 // Pack three FP32 channel volumes into the BF16 input rows (zero halo).
-__global__ void pack_input_kernel(Geo g, const float *__restrict__ c0, const float *__restrict__ c1,
-                                  const float *__restrict__ c2, __nv_bfloat16 *__restrict__ out)
+__global__ void __launch_bounds__(256)
+    pack_input_kernel(Geo g, const float *__restrict__ c0, const float *__restrict__ c1, const float *__restrict__ c2,
+                      __nv_bfloat16 *__restrict__ out)
 {
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.R; r += (long long)gridDim.x * blockDim.x) {
-        const long long v = interior_of(g, r);
-        uint4 r0 = make_uint4(0u, 0u, 0u, 0u);
-        if (v >= 0) {
-            r0.x = pack_bf16(c0[v], c1[v]);
-            r0.y = pack_bf16(c2[v], 0.0f);
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (long long h0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; h0 < 2 * g.R; h0 += kHalves * step) {
+        float x[kHalves][3];
+#pragma unroll
+        for (int k = 0; k < kHalves; ++k) {
+            const long long h = h0 + k * step, v = h < 2 * g.R && !(h & 1) ? interior_of(g, h >> 1) : -1;
+            x[k][0] = v >= 0 ? __ldcs(c0 + v) : 0.0f;
+            x[k][1] = v >= 0 ? __ldcs(c1 + v) : 0.0f;
+            x[k][2] = v >= 0 ? __ldcs(c2 + v) : 0.0f;
         }
-        reinterpret_cast<uint4 *>(out + r * CH)[0] = r0;
-        reinterpret_cast<uint4 *>(out + r * CH)[1] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int k = 0; k < kHalves; ++k) {
+            const long long h = h0 + k * step;
+            if (h < 2 * g.R)
+                reinterpret_cast<uint4 *>(out)[h] =
+                    make_uint4(pack_bf16(x[k][0], x[k][1]), pack_bf16(x[k][2], 0.0f), 0u, 0u);
+        }
     }
 }
 
 // Loss 0.5 * mean (pred - target)^2 (FP64 partials) and its gradient, scaled
 // by `gscale`, into channel 0 of BF16 rows (zero halo).
-__global__ void mse_kernel(Geo g, const float *__restrict__ pred, const float *__restrict__ target,
-                           float gscale, __nv_bfloat16 *__restrict__ grad, double *__restrict__ partial)
+__global__ void __launch_bounds__(256)
+    mse_kernel(Geo g, const float *__restrict__ pred, const float *__restrict__ target, float gscale,
+               __nv_bfloat16 *__restrict__ grad, double *__restrict__ partial)
 {
     __shared__ double red[8];
     double acc = 0.0;
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.R; r += (long long)gridDim.x * blockDim.x) {
-        const long long v = interior_of(g, r);
-        uint4 r0 = make_uint4(0u, 0u, 0u, 0u);
-        if (v >= 0) {
-            const float d = pred[v] - target[v];
-            acc += (double)d * d;
-            r0.x = pack_bf16(d * gscale, 0.0f);
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (long long h0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; h0 < 2 * g.R; h0 += kHalves * step) {
+        float d[kHalves];
+#pragma unroll
+        for (int k = 0; k < kHalves; ++k) {
+            const long long h = h0 + k * step, v = h < 2 * g.R && !(h & 1) ? interior_of(g, h >> 1) : -1;
+            d[k] = v >= 0 ? __ldcs(pred + v) - __ldcs(target + v) : 0.0f;
         }
-        reinterpret_cast<uint4 *>(grad + r * CH)[0] = r0;
-        reinterpret_cast<uint4 *>(grad + r * CH)[1] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int k = 0; k < kHalves; ++k) {
+            const long long h = h0 + k * step;
+            acc += (double)d[k] * d[k];
+            if (h < 2 * g.R)
+                reinterpret_cast<uint4 *>(grad)[h] = make_uint4(pack_bf16(d[k] * gscale, 0.0f), 0u, 0u, 0u);
+        }
     }
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -951,14 +973,14 @@ int launch_conv(fwi_cnn *n, const __nv_bfloat16 *in, const __nv_bfloat16 *w, con
     return FWI_OK;
 }
 
-int forward_impl(fwi_cnn *n)
+// All layers, from act[0] to the FP32 volume `out`.
+int forward_impl(fwi_cnn *n, float *out)
 {
     for (int l = 0; l < NL; ++l) {
         const int st = l < NL - 1
                            ? launch_conv<1, 0>(n, n->act[l].p, n->wb[l].p, n->b32[l].p, nullptr, n->act[l + 1].p,
                                                nullptr)
-                           : launch_conv<1, 2>(n, n->act[l].p, n->wb[l].p, n->b32[l].p, nullptr, nullptr,
-                                               n->pred.p);
+                           : launch_conv<1, 2>(n, n->act[l].p, n->wb[l].p, n->b32[l].p, nullptr, nullptr, out);
         if (st != FWI_OK) return st;
     }
     return FWI_OK;
@@ -1187,9 +1209,8 @@ int fwi_cnn_forward(fwi_cnn *n, int nz, int nx, int ny, const float *d_in, float
     if (st != FWI_OK) return st;
     const long long V = n->g.V;
     pack_input_kernel<<<1184, 256, 0, n->stream>>>(n->g, d_in, d_in + V, d_in + 2 * V, n->act[0].p);
-    st = forward_impl(n);
+    st = forward_impl(n, d_out);
     if (st != FWI_OK) return st;
-    CNN_CK(cudaMemcpyAsync(d_out, n->pred.p, V * sizeof(float), cudaMemcpyDeviceToDevice, n->stream));
     CNN_CK(cudaStreamSynchronize(n->stream));
     return check_cnn_status(n);
 }
@@ -1206,7 +1227,7 @@ int fwi_cnn_train_step(fwi_cnn *n, int nz, int nx, int ny, const float *d_in, co
     const Geo &g = n->g;
     const long long V = g.V;
     pack_input_kernel<<<1184, 256, 0, n->stream>>>(g, d_in, d_in + V, d_in + 2 * V, n->act[0].p);
-    st = forward_impl(n);
+    st = forward_impl(n, n->pred.p);
     if (st != FWI_OK) return st;
     // loss gradient d(0.5 mean d^2)/dpred = d / V, carried in BF16 scaled up
     // by V (loss scaling) and scaled back in the weight gradients
