@@ -31,24 +31,30 @@ namespace {
 // ---------------------------------------------------------------------------
 // Tile tables: z quads (cells = 4*TZ4), x rows, halo slots of the ring, CTAs per
 // SM, and the picoseconds a step takes per cell that the tiles cover on a busy
-// GPU (measured on 201^3 .. 483 x 483 x 283 cells).  A thread owns two x rows,
+// GPU (measured on 60^3 .. 483 x 483 x 283 cells).  A thread owns two x rows,
 // which share their eight x neighbours: 10 instead of 14 shared-memory loads
 // per 4 cells.  16 warps of 128 registers fill an SM, so the large tiles take
 // 14 compute warps or less and all the shared memory: halo slots beyond the
 // five in use are load-ahead, and one more of them took the backward step of
-// 301^3 cells from 0.166 to 0.143 ms.
+// 301^3 cells from 0.166 to 0.143 ms.  Several small CTAs per SM hide each
+// other's waits while the fields stay in the L2, but cover HBM latency with
+// fewer bytes in flight per column: the backward step of 130 x 150 x 140
+// cells takes 24.8 us with 64 x 12 tiles, 28.8 us with 148 x 8; of
+// 401 x 401 x 251 cells 600 and 461 us.
 // ---------------------------------------------------------------------------
 constexpr int kNumTiles = 10;
 struct TileSpec {
     int tz4, tx, sh, ctas;
-    double cost;
+    double in_l2, in_hbm;  // where one shot's fields fit the L2, and where not
 };
 constexpr TileSpec kFwdTiles[kNumTiles] = {
-    {16, 8, 7, 4, 2.55},  {19, 20, 7, 2, 2.47}, {32, 24, 7, 1, 2.20}, {24, 16, 7, 2, 2.35}, {25, 24, 9, 1, 2.25},
-    {37, 24, 7, 1, 2.35}, {37, 18, 8, 1, 2.22}, {12, 8, 8, 4, 3.05},  {25, 32, 7, 1, 2.30}, {49, 16, 7, 1, 2.20}};
+    {16, 8, 7, 4, 2.55, 2.55},  {19, 20, 7, 2, 2.47, 2.47}, {32, 24, 7, 1, 2.20, 2.20}, {24, 16, 7, 2, 2.35, 2.35},
+    {25, 24, 9, 1, 2.25, 2.25}, {37, 24, 7, 1, 2.35, 2.35}, {37, 18, 8, 1, 2.22, 2.22}, {12, 8, 8, 4, 3.05, 3.05},
+    {25, 32, 7, 1, 2.30, 2.30}, {49, 16, 7, 1, 2.20, 2.20}};
 constexpr TileSpec kBwdTiles[kNumTiles] = {
-    {16, 12, 7, 2, 5.40}, {19, 22, 7, 1, 5.30}, {16, 28, 7, 1, 4.90}, {25, 14, 8, 1, 5.20}, {25, 16, 7, 1, 5.20},
-    {19, 18, 8, 1, 5.40}, {8, 8, 7, 4, 6.00},   {37, 10, 7, 1, 4.72}, {12, 16, 7, 2, 5.20}, {37, 8, 8, 1, 4.75}};
+    {16, 12, 7, 2, 5.40, 6.40}, {19, 22, 7, 1, 5.30, 5.30}, {16, 28, 7, 1, 5.60, 5.60}, {25, 14, 8, 1, 5.20, 5.20},
+    {25, 16, 7, 1, 5.40, 5.20}, {19, 18, 8, 1, 5.40, 5.35}, {8, 8, 7, 4, 6.00, 6.00},   {37, 10, 7, 1, 4.72, 4.70},
+    {12, 16, 7, 2, 5.50, 6.00}, {37, 8, 8, 1, 4.75, 4.70}};
 
 struct KInfo {
     const void *fn = nullptr;
@@ -522,16 +528,18 @@ void prepare_kernel(const KInfo &k)
 }
 
 // Tile before tuning: the one whose covered cells, updated or not, cost least.
-// Within 4 % of the best tile on 10 of 13 measured grids, at most 12 % off on
+// Within 4 % of the best tile on 11 of 14 measured grids, at most 12 % off on
 // small ones, where the hand-over between steps counts more than the cells.
 int default_tile(const fwi_ctx *c, bool backward)
 {
     int best = 0;
     double best_cost = 1e30;
+    // fields of one shot: two or four levels and the coefficient
+    const bool in_hbm = (double)c->vol * sizeof(float) * (backward ? 5 : 3) > 100e6;
     for (int t = 0; t < kNumTiles; ++t) {
         const TileSpec &s = (backward ? kBwdTiles : kFwdTiles)[t];
         const int tz = 4 * s.tz4, ntz = (c->nzz - 8 + tz - 1) / tz, ntx = (c->nxx - 8 + s.tx - 1) / s.tx;
-        const double cost = s.cost * ntz * tz * ntx * s.tx;
+        const double cost = (in_hbm ? s.in_hbm : s.in_l2) * ntz * tz * ntx * s.tx;
         if (cost < best_cost) {
             best_cost = cost;
             best = t;

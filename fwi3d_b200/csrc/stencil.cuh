@@ -397,8 +397,7 @@ __device__ __forceinline__ void loop_producer(LoopShared<NW> &sh, uint64_t *full
         }
     }
     if (!ok && lane == 0) {
-        loop_fail(&sh.abort);
-        mbar_arrive(&full[hs]);  // wakes the compute warps, which see the abort
+        loop_fail(&sh.abort);  // (the compute warps wait for the same stage and give up as well)
         // no copy may land after the CTA has gone: only the newest use of
         // each slot can still be in flight
         for (int k = 1; k <= min(g, SH); ++k) {
@@ -465,6 +464,15 @@ __device__ __forceinline__ void loop_publisher(LoopShared<NW> &sh, const LoopGeo
 //       velocity slots (one slot shared by every shot, or one slot per shot
 //       when every shot has its own random pad).  They are 0 on the cells
 //       that are never updated, which keeps those cells at 0.
+// Bound: shared-memory wavefronts (74 % of the L1 pipe: 10 halo rows read for
+// 8 cells) together with HBM.  301^3 cells, random pad, one shot, per step:
+// 86.5 us as one launch per step with a register queue per cell, 60.1 us now;
+// 11.3 bytes per cell from HBM instead of 14.9, since a plane that one step
+// stores is still in L2 when the next reads it; 16 bytes per cell at the
+// 6.55 TB/s of a copy take 67 us.  Small grids were bound by the launches and
+// by few planes per CTA: 56 x 60 x 58 cells with the Cerjan pad 29 us, now 6.2 us.
+// The Cerjan factors per row instead of a branch per cell: 201^3 cells 73 us,
+// now 20 us.
 // ---------------------------------------------------------------------------
 struct FwdMaps {
     CUtensorMap mh[2], mq[2], mv;
@@ -640,7 +648,7 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
             for (int p = 4; p < a.nyy; ++p) {
                 const int y = p - 4;
                 if (p > 4) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(&full[hs], hph) && !aborted(&sh.abort));
+                    ok = __all_sync(0xffffffffu, mbar_wait(&full[hs], hph));
                     if (!ok) break;
                 }
                 const float *Hp = reinterpret_cast<const float *>(hring + hs * T::HSLOT) + ho;
@@ -703,7 +711,7 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
                             out = mk4(lo(out.a) + (se == 0 ? add : 0.f), hi(out.a) + (se == 1 ? add : 0.f),
                                       lo(out.b) + (se == 2 ? add : 0.f), hi(out.b) + (se == 3 ? add : 0.f));
                         }
-                        if (r < nrow) stq(Qp + (long long)r * a.ldz, out);
+                        if (r < nrow) stq(Qp + r * a.ldz, out);
                     }
                     Qp += plane;
                 }
@@ -739,6 +747,16 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
 // The accumulators are updated by vector reductions in L2: they take no shared
 // memory, so the rings run a stage deeper, and nothing waits for them.  The
 // steps of a column follow one another, so every cell adds its steps in order.
+// Each field has its own compute warps, since one thread with the sums of both
+// for two rows would need more than 200 registers, and with one row each
+// 14 loads per 4 cells (301^3 cells, 4 shots: 0.694 ms per step, by field
+// 0.665, with the accumulators out of shared memory 0.573 and the ring that
+// this makes room for 0.543).
+// Bound: HBM.  301^3 cells, random pad, one shot: 32.4 bytes per cell and step
+// at 6.5 TB/s, the rate of a copy (the old levels and the coefficients arrive
+// in 148 x 8 boxes, the halos of the two fields are read 2.1 times, from L2).
+// 185 us per step as one launch per step, 136 us now; 88^3 cells,
+// 4 shots: 35 and 11.7 us.
 // ---------------------------------------------------------------------------
 struct BwdMaps {
     CUtensorMap mhs[2], mhr[2], mcs[2], mcr[2], mv;
@@ -882,8 +900,10 @@ __global__ void __launch_bounds__(Loop<T, 2>::THREADS, CTAS)
                 const Item it = item_of(tk, geo.nshot, a.prog.shots, a.nsteps, a.ncol);
                 const int zc = 4 + it.col % a.ntz * T::TZ + 4 * lz, xc = 4 + it.col / a.ntz * T::TX + lx;
                 const int nrow = zc < a.nzz - 4 && ft < T::NT ? min(R, a.nxx - 4 - xc) : 0;  // rows this thread writes
-                long long off = (long long)it.shot * a.vol + 4 * plane + (long long)xc * a.ldz + zc;
-                float *out = SRC ? a.F[1 - ((a.s0 + it.t) & 1)] : a.Rf[1 - (it.t & 1)];
+                const long long off = (long long)it.shot * a.vol + 4 * plane + (long long)xc * a.ldz + zc;
+                float *out = (SRC ? a.F[1 - ((a.s0 + it.t) & 1)] : a.Rf[1 - (it.t & 1)]) + off;
+                float *image = a.image + off;
+                const long long to_illum = a.illum - a.image;
                 // source cell among this thread's cells: element se of row sr on
                 // plane ys.  Stored field A_{N-t} carried source sample N-t; the
                 // exact rebuild adds it back.
@@ -907,7 +927,7 @@ __global__ void __launch_bounds__(Loop<T, 2>::THREADS, CTAS)
                 for (int p = 4; p < a.nyy; ++p) {
                     const int y = p - 4;
                     if (p > 4) {
-                        ok = __all_sync(0xffffffffu, mbar_wait(&full[hs], hph) && !aborted(&sh.abort));
+                        ok = __all_sync(0xffffffffu, mbar_wait(&full[hs], hph));
                         if (!ok) break;
                     }
                     const float *Hp =
@@ -937,8 +957,7 @@ __global__ void __launch_bounds__(Loop<T, 2>::THREADS, CTAS)
                                          lo(nv.b) + (se == 2 ? add : 0.f), hi(nv.b) + (se == 3 ? add : 0.f));
                             }
                             if (r >= nrow) continue;
-                            const long long o = off + (long long)r * a.ldz;
-                            stq(out + o, nv);
+                            stq(out + r * a.ldz, nv);
                             // (the box lies inside the updated cells)
                             if (acc && xc + r >= a.acc_x0 && xc + r < a.acc_x1) {
                                 const q4 pr = ldq(Hy + T::HSLOT / 4 + r * T::HZ);  // the adjoint field's own value
@@ -951,11 +970,12 @@ __global__ void __launch_bounds__(Loop<T, 2>::THREADS, CTAS)
                                     vi[e] = (zmask >> e) & 1 ? get(im, e) : 0.0f;
                                     vl[e] = (zmask >> e) & 1 ? get(il, e) : 0.0f;
                                 }
-                                red_add4(a.image + o, vi[0], vi[1], vi[2], vi[3]);
-                                red_add4(a.illum + o, vl[0], vl[1], vl[2], vl[3]);
+                                red_add4(image + r * a.ldz, vi[0], vi[1], vi[2], vi[3]);
+                                red_add4(image + to_illum + r * a.ldz, vl[0], vl[1], vl[2], vl[3]);
                             }
                         }
-                        off += plane;
+                        out += plane;
+                        if (SRC) image += plane;
                     }
                     ++g;
                     __syncwarp();
