@@ -40,7 +40,10 @@ namespace {
 // other's waits while the fields stay in the L2, but cover HBM latency with
 // fewer bytes in flight per column: the backward step of 130 x 150 x 140
 // cells takes 24.8 us with 64 x 12 tiles, 28.8 us with 148 x 8; of
-// 401 x 401 x 251 cells 600 and 461 us.
+// 251 x 401 x 401 cells, 2 shots, 600 and 461 us.  The z sizes of the large
+// tiles (100, 112, 124, 148) leave few cells of any z extent beyond the grid:
+// 228^3 cells, 9 shots, take 496 us backward with 112 x 12 tiles (2 cover the
+// 220 updated cells), at least 519 us with any other of these.
 // ---------------------------------------------------------------------------
 constexpr int kNumTiles = 10;
 struct TileSpec {
@@ -52,7 +55,7 @@ constexpr TileSpec kFwdTiles[kNumTiles] = {
     {25, 24, 9, 1, 2.25, 2.25}, {37, 24, 7, 1, 2.35, 2.35}, {37, 18, 8, 1, 2.22, 2.22}, {12, 8, 8, 4, 3.05, 3.05},
     {25, 32, 7, 1, 2.30, 2.30}, {49, 16, 7, 1, 2.20, 2.20}};
 constexpr TileSpec kBwdTiles[kNumTiles] = {
-    {16, 12, 7, 2, 5.40, 6.40}, {19, 22, 7, 1, 5.30, 5.30}, {16, 28, 7, 1, 5.60, 5.60}, {25, 14, 8, 1, 5.20, 5.20},
+    {16, 12, 7, 2, 5.40, 6.40}, {28, 12, 8, 1, 4.90, 4.90}, {31, 10, 8, 1, 5.00, 5.60}, {25, 14, 8, 1, 5.20, 5.20},
     {25, 16, 7, 1, 5.40, 5.20}, {19, 18, 8, 1, 5.40, 5.35}, {8, 8, 7, 4, 6.00, 6.00},   {37, 10, 7, 1, 4.72, 4.70},
     {12, 16, 7, 2, 5.50, 6.00}, {37, 8, 8, 1, 4.75, 4.70}};
 
