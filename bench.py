@@ -5,8 +5,8 @@ Workload (default, the batched-RTM configuration): 201^3 model at 10 m, five
 layers plus -8 %/+12 % Gaussian anomalies, smoothed migration model, 50-cell
 random boundary (301^3 padded cells), nt = 2001 at 1 ms, Ricker 10 Hz peak
 (N = 2120 time steps), 64 shots on an 8 x 8 grid with clipped 121 x 121
-receiver patches.  One step = one batch of B shots (--batch, default 4) in
-one launch per time step, each shot through its own new random boundary:
+receiver patches.  One step = one batch of B shots (--batch, default 4), all
+its time steps in one launch, each shot through its own new random boundary:
 forward propagation, then the fused pass (source rebuilt backwards + adjoint
 propagation + imaging), 3 x B padded cells x N steps of cell-updates.
 
@@ -259,7 +259,7 @@ def run_ours(args, ws, rank, local):
     # box, the only cells that accumulate), the forward step (16 B per
     # cell-update) for modeling
     peak, peak_kind = hbm_peak()
-    # per launch: B shots of the padded grid; frac_updated charges the field
+    # per time step: B shots of the padded grid; frac_updated charges the field
     # bytes only to the cells a launch writes (the outer 4-cell shell is read,
     # never written)
     box = w.nz * w.nx * w.ny
@@ -351,7 +351,7 @@ def run_ours(args, ws, rank, local):
         "data": "synthetic: seeded layered model with Gaussian anomalies, seeded random observed data",
         "config": {
             "workload": (f"{w.name}: padded {ctx.nzz}x{ctx.nxx}x{ctx.nyy}, nt={w.nt}, N={N} steps; "
-                         + (f"one batch of {B} shots per step, in one launch per time step, each shot through its "
+                         + (f"one batch of {B} shots per step, in one launch per time loop, each shot through its "
                             "own new random boundary: forward + fused backward (3 cell-updates per padded cell, "
                             "time step and shot)" if rtm else "one shot per step: forward modeling")),
             "shots": nsrc, "shots_per_step": B, "shots_per_launch": B, "l2": l2_note,
