@@ -7,6 +7,25 @@
 
 namespace fwi {
 
+// f(i, j, k, row) for every cell of nz x nx x ny, a warp to a z row.  The kernels
+// built on it are copies that HBM bounds; with a thread to a cell, two 64-bit
+// divisions per cell took longer than the copy.  Now a lane divides once per
+// row.  301^3 cells: coefficients 135 -> 39 us (33 us at the rate of a copy),
+// largest velocity 63 -> 31 us (18 us to read), edge padding 94 -> 32 us;
+// image of 201^3 cells from dense accumulators, with 32 MB to the host, 806 ->
+// 732 us.  Rows shorter than a warp leave lanes idle, which costs less than
+// the divisions (88^3 cells: no difference).
+template <class F>
+__device__ __forceinline__ void for_cells(int nz, int nx, int ny, F f)
+{
+    const long long rows = (long long)nx * ny, step = (long long)gridDim.x * (blockDim.x / 32);
+    for (long long r = blockIdx.x * (long long)(blockDim.x / 32) + threadIdx.x / 32; r < rows; r += step) {
+        const int k = (int)(r / nx), j = (int)(r - (long long)k * nx);
+#pragma unroll 4
+        for (int i = threadIdx.x % 32; i < nz; i += 32) f(i, j, k, r);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Edge-replication padding of an unpadded [nz,nx,ny] model into a pitched
 // padded field: every padded cell copies the nearest model cell
@@ -15,61 +34,26 @@ namespace fwi {
 __global__ void pad_edges_kernel(const float *__restrict__ in, int nz, int nx, int ny, int nb,
                                  int nzz, int nxx, int nyy, int ldz, float *__restrict__ out)
 {
-    const long long n = (long long)ldz * nxx * nyy;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % ldz);
-        const long long r = c / ldz;
-        const int j = (int)(r % nxx), k = (int)(r / nxx);
-        if (i >= nzz) {
-            out[c] = 0.0f;
-            continue;
-        }
+    for_cells(ldz, nxx, nyy, [&](int i, int j, int k, long long r) {
         const int is = min(max(i - nb, 0), nz - 1);
         const int js = min(max(j - nb, 0), nx - 1);
         const int ks = min(max(k - nb, 0), ny - 1);
-        out[c] = in[is + (long long)js * nz + (long long)ks * nx * nz];
-    }
+        out[r * ldz + i] = i < nzz ? in[is + (long long)js * nz + (long long)ks * nx * nz] : 0.0f;
+    });
 }
 
 // Dense padded [nzz,nxx,nyy] <-> pitched [nyy][nxx][ldz].
 __global__ void dense_to_pitched_kernel(const float *__restrict__ in, int nzz, int nxx, int nyy,
                                         int ldz, float *__restrict__ out)
 {
-    const long long n = (long long)ldz * nxx * nyy;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % ldz);
-        const long long r = c / ldz;
-        out[c] = i < nzz ? in[i + r * nzz] : 0.0f;
-    }
+    for_cells(ldz, nxx, nyy,
+              [&](int i, int, int, long long r) { out[r * ldz + i] = i < nzz ? in[r * nzz + i] : 0.0f; });
 }
 
 __global__ void pitched_to_dense_kernel(const float *__restrict__ in, int nzz, int nxx, int nyy,
                                         int ldz, float *__restrict__ out)
 {
-    const long long n = (long long)nzz * nxx * nyy;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % nzz);
-        const long long r = c / nzz;
-        out[c] = in[i + r * ldz];
-    }
-}
-
-// Crop the pad of a pitched field into [nz,nx,ny] (reduce_boundary,
-// src/modeling/modeling.cu:230-241).
-__global__ void crop_kernel(const float *__restrict__ in, int nz, int nx, int ny, int nb, int nxx,
-                            int ldz, float *__restrict__ out)
-{
-    const long long n = (long long)nz * nx * ny;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % nz);
-        const long long r = c / nz;
-        const int j = (int)(r % nx), k = (int)(r / nx);
-        out[c] = in[(i + nb) + (long long)(j + nb) * ldz + (long long)(k + nb) * ldz * nxx];
-    }
+    for_cells(nzz, nxx, nyy, [&](int i, int, int, long long r) { out[r * nzz + i] = in[r * ldz + i]; });
 }
 
 // Sum the accumulator slots of a batch into slot 0.
@@ -153,12 +137,7 @@ __global__ void rtm_image_kernel(const float *__restrict__ img, const float *__r
                                  int nz, int nx, int ny, int nb, int nxx, int ldz, float idh2,
                                  float *__restrict__ out)
 {
-    const long long n = (long long)nz * nx * ny;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % nz);
-        const long long r = c / nz;
-        const int j = (int)(r % nx), k = (int)(r / nx);
+    for_cells(nz, nx, ny, [&](int i, int j, int k, long long r) {
         float v = 0.0f;
         if (i > 0 && i < nz - 1) {
             const long long p = (i + nb) + (long long)(j + nb) * ldz + (long long)(k + nb) * ldz * nxx;
@@ -167,8 +146,8 @@ __global__ void rtm_image_kernel(const float *__restrict__ img, const float *__r
             const float sp = ratio(img[p + 1], ill[p + 1]);
             v = -1.0f * (sm - 2.0f * s0 + sp) * idh2;
         }
-        out[c] = v;
-    }
+        out[r * nz + i] = v;
+    });
 }
 
 // Gradient post-processing, first pass: crop, divide, -d2/dz2 below the mask
@@ -179,13 +158,8 @@ __global__ void grad_post_kernel(const float *__restrict__ g, const float *__res
                                  int nx, int ny, int nb, int nxx, int ldz, float idh2, int imask,
                                  float *__restrict__ out, unsigned int *__restrict__ gmax_bits)
 {
-    const long long n = (long long)nz * nx * ny;
     float lmax = 0.0f;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % nz);
-        const long long r = c / nz;
-        const int j = (int)(r % nx), k = (int)(r / nx);
+    for_cells(nz, nx, ny, [&](int i, int j, int k, long long r) {
         float v = 0.0f;
         if (i > imask && i < nz - 1) {
             const long long p = (i + nb) + (long long)(j + nb) * ldz + (long long)(k + nb) * ldz * nxx;
@@ -194,9 +168,9 @@ __global__ void grad_post_kernel(const float *__restrict__ g, const float *__res
             const float sp = ratio(g[p + 1], ill[p + 1]);
             v = -1.0f * (sm - 2.0f * s0 + sp) * idh2;
         }
-        out[c] = v;
+        out[r * nz + i] = v;
         lmax = fmaxf(lmax, fabsf(v));
-    }
+    });
     for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
     if ((threadIdx.x & 31) == 0) atomicMax(gmax_bits, __float_as_uint(lmax));
 }
@@ -527,16 +501,12 @@ __global__ void __launch_bounds__(kBrickThreads)
 __global__ void coeff_kernel(const float *__restrict__ vp, float *__restrict__ out, int nzz, int nxx, int nyy,
                              int ldz, int nslot, float cvel)
 {
-    const long long n = (long long)ldz * nxx * nyy * nslot;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % ldz);
-        const long long r = c / ldz;
-        const int j = (int)(r % nxx), k = (int)(r / nxx % nyy);
+    for_cells(ldz, nxx, nyy * nslot, [&](int i, int j, int ks, long long r) {
+        const int k = ks % nyy;
         const bool upd = i >= 4 && i < nzz - 4 && j >= 4 && j < nxx - 4 && k >= 4 && k < nyy - 4;
-        const float v = vp[c];
-        out[c] = upd ? v * v * cvel : 0.0f;
-    }
+        const float v = vp[r * ldz + i];
+        out[r * ldz + i] = upd ? v * v * cvel : 0.0f;
+    });
 }
 
 // Range of a velocity model and its first value that is not a positive number.
@@ -570,13 +540,11 @@ __global__ void velocity_range_kernel(const float *__restrict__ v, long long n, 
 }
 
 // Largest |v| in a pitched field restricted to the real cells (CFL check).
-__global__ void max_abs_kernel(const float *__restrict__ v, long long n, int ldz, int nzz,
+__global__ void max_abs_kernel(const float *__restrict__ v, int nzz, int nxx, int nplane, int ldz,
                                unsigned int *__restrict__ out_bits)
 {
     float m = 0.0f;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
-         c += (long long)gridDim.x * blockDim.x)
-        if ((int)(c % ldz) < nzz) m = fmaxf(m, fabsf(v[c]));
+    for_cells(nzz, nxx, nplane, [&](int i, int, int, long long r) { m = fmaxf(m, fabsf(v[r * ldz + i])); });
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMax(out_bits, __float_as_uint(m));
 }

@@ -1107,7 +1107,8 @@ float device_max_abs(fwi_ctx *c, const float *v, long long n)
 {
     c->ubits.ensure(1);
     CK(cudaMemsetAsync(c->ubits.p, 0, sizeof(unsigned), c->stream));
-    max_abs_kernel<<<grid_blocks(n), 256, 0, c->stream>>>(v, n, c->ldz, c->nzz, c->ubits.p);
+    max_abs_kernel<<<grid_blocks(n), 256, 0, c->stream>>>(v, c->nzz, c->nxx, (int)(n / (c->ldz * (long long)c->nxx)),
+                                                          c->ldz, c->ubits.p);
     CK(cudaGetLastError());
     unsigned bits = 0;
     CK(cudaMemcpyAsync(&bits, c->ubits.p, sizeof bits, cudaMemcpyDeviceToHost, c->stream));
