@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kBrickThreads)
 
     int n = 0;  // blobs in the list
     for (int b0 = 0; b0 < nblob; b0 += kBrickThreads) {
-        // append the blobs of this round that reach the brick
+        // append the blobs of this pass that reach the brick
         Blob b;
         bool in = false;
         if (b0 + tid < nblob) {
