@@ -24,8 +24,7 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s cap on any device wait
 // Error bits the kernels raise in g_status (read back by the host).
 constexpr unsigned kErrTimeout = 1u;
 
-// Per-batch shot description, device resident so that a captured time loop
-// can be replayed for any batch of shots without re-capture.
+// Per-batch shot description, copied to the device once per batch.
 struct BatchInfo {
     int nshot;                    // shots in this batch
     int R;                        // receivers of all shots together
