@@ -56,7 +56,7 @@ def _stale(target: Path, sources: list[Path]) -> bool:
 def build_library(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> Path:
     LIB_DIR.mkdir(exist_ok=True)
     units = sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cpp"))
-    srcs = units + sorted(CSRC.glob("*.cuh")) + [ROOT / "include" / "fwi3d.h"]
+    srcs = units + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [ROOT / "include" / "fwi3d.h"]
     if force or ptxas_info or _stale(LIB, srcs):
         cmd = [nvcc(), *ARCH, *NVCC_FLAGS, "-shared", "-o", str(LIB), *map(str, units)]
         if ptxas_info:

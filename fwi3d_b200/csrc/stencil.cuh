@@ -35,6 +35,7 @@
 #include <type_traits>
 
 #include "device.cuh"
+#include "loop_order.h"
 
 namespace fwi {
 
@@ -221,6 +222,9 @@ __device__ __forceinline__ void xz_d2(const float *H, q4 (&c)[T::R], q4 (&d)[T::
 // after the plane y + 4 of u^t has arrived, so the neighbours have stored
 // plane y + 4 of step t-1 and therefore read all of plane y.  A halo box also
 // covers corner cells of diagonal neighbours, which the stencil never uses.
+// Receiver samples are a reader of their own, beside the stencil: the
+// publisher keeps its lead over them within kSampleLead planes.  (The rules
+// are in loop_order.h.)
 //
 // Warps of a CTA: NW compute warps; one producer (tickets, waits for the other
 // columns, TMA); one publisher (tells the other columns which planes are in
@@ -248,26 +252,6 @@ struct LoopShared {
     int abort;
 };
 
-struct Item {
-    int shot, t, col;
-};
-
-// Ticket order: shots in groups of `group` whose steps interleave, then step,
-// shot of the group, column.
-__device__ __forceinline__ Item item_of(long long ticket, int nshot, int group, int nsteps, int ncol)
-{
-    const long long per_group = (long long)nsteps * ncol * group;
-    const int first = (int)(ticket / per_group) * group;
-    const long long r = ticket % per_group;
-    const int per_step = min(group, nshot - first) * ncol;
-    Item it;
-    it.t = (int)(r / per_step);
-    const int q = (int)(r - (long long)it.t * per_step);
-    it.shot = first + q / ncol;
-    it.col = q % ncol;
-    return it;
-}
-
 __device__ __forceinline__ bool aborted(const int *flag) { return *(const volatile int *)flag != 0; }
 
 __device__ __forceinline__ void loop_fail(int *flag)
@@ -288,21 +272,6 @@ __device__ __forceinline__ bool wait_shared(const int *p, int v, const int *abor
             __nanosleep(64);
         }
         if (aborted(abort_flag) || global_ns() - t0 > kWaitLimitNs) return false;
-    }
-}
-
-// The columns whose progress an item waits for: lane 0 its own, lanes 1..4 the
-// neighbours along z and x that exist; the other lanes wait for nothing.
-__device__ __forceinline__ int dependency_column(int lane, int col, int ntz, int ncol)
-{
-    const int zt = col % ntz;
-    switch (lane) {
-    case 0: return col;
-    case 1: return zt > 0 ? col - 1 : -1;
-    case 2: return zt < ntz - 1 ? col + 1 : -1;
-    case 3: return col >= ntz ? col - ntz : -1;
-    case 4: return col + ntz < ncol ? col + ntz : -1;
-    default: return -1;
     }
 }
 
@@ -381,8 +350,7 @@ __device__ __forceinline__ void loop_producer(LoopShared<NW> &sh, uint64_t *full
         const auto state = start(it);
         for (int p = 4; p < geo.nyy; ++p) {
             if (p > 4 && g >= SC) ok = mbar_wait(&done[cs], cph);
-            // (the last four planes are never written)
-            if (p < geo.nyy - 4) ok = wait_columns(dp, base + p + 1, seen, &sh.abort) && ok;
+            if (const int need = planes_awaited(p, geo.nyy)) ok = wait_columns(dp, base + need, seen, &sh.abort) && ok;
             if (!__all_sync(0xffffffffu, ok)) {
                 ok = false;
                 break;
@@ -409,11 +377,11 @@ __device__ __forceinline__ void loop_producer(LoopShared<NW> &sh, uint64_t *full
 
 // Publisher warp: follows the compute warps and tells the other columns which
 // planes of an item are stored.  start(it) returns the state of an item;
-// before(state, n) runs when the planes below n are stored and not yet
-// published, after(state, n) when they are published.
-template <int NW, class Start, class Before, class After>
+// work(state, n) does its work on the planes below n: before they are published
+// (LEAD 0), or after LEAD planes at most have been published without it.
+template <int LEAD, int NW, class Start, class Work>
 __device__ __forceinline__ void loop_publisher(LoopShared<NW> &sh, const LoopGeo &geo, const LoopProgress &prog,
-                                               int lane, Start start, Before before, After after)
+                                               int lane, Start start, Work work)
 {
     const int nstage = geo.nyy - 4;  // stages of an item: p = 4 .. nyy-1, y = p - 4
     // stages finished by every compute warp, once there are more than s; -1
@@ -442,16 +410,20 @@ __device__ __forceinline__ void loop_publisher(LoopShared<NW> &sh, const LoopGeo
         long long *dp = counter(prog, geo.ncol, it.shot, it.t, it.col);
         const long long base = (long long)it.t * geo.nyy;
         auto state = start(it);
-        int published = 4;  // the first four planes are never written
+        int published = 4, stored = 4;  // the first four planes are never written
         while (published < nstage) {
-            n = more_than(s0 + published);
-            if (n < 0) return;
-            published = min(n - s0, nstage);
-            before(state, published);
+            if (stored == published) {
+                n = more_than(s0 + published);
+                if (n < 0) return;
+                stored = min(n - s0, nstage);
+            }
+            published = next_publication(published, stored, LEAD);
+            const bool first = work_first(published, nstage, LEAD);
+            if (first) work(state, published);
             __syncwarp();
             if (lane == 0) st_release_gpu(dp, base + published);
             __syncwarp();
-            after(state, published);
+            if (!first) work(state, published);
         }
     }
 }
@@ -540,9 +512,9 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
                 }
             });
     } else if (warp == NW + 1) {
-        // After publishing: samples of the level the item stores, u^(t+1).
-        // Lane l holds entry u + l of the column's list, looked up ahead of
-        // its plane.
+        // Samples of the level the item stores, u^(t+1), a few planes behind the
+        // publication where they can be.  Lane l holds entry u + l of the
+        // column's list, looked up ahead of its plane.
         struct State {
             int u, last, sample, y, first, end;
             long long cell;
@@ -559,7 +531,7 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
                 st.end = a.rec.first[e + 1];
             }
         };
-        loop_publisher(
+        loop_publisher<kSampleLead>(
             sh, geo, a.prog, lane,
             [&](const Item &it) {
                 State st{0, 0, it.t + 1 - a.tlag, 0, 0, 0, 0, a.F[1 - (it.t & 1)]};
@@ -570,7 +542,6 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
                 load(st);
                 return st;
             },
-            [](State &, int) {},
             [&](State &st, int n) {
                 for (;;) {
                     const bool mine = st.y < n;
@@ -850,7 +821,7 @@ __global__ void __launch_bounds__(Loop<T, 2>::THREADS, CTAS)
                 st.f = f;
             }
         };
-        loop_publisher(
+        loop_publisher<0>(
             sh, geo, a.prog, lane,
             [&](const Item &it) {
                 State st{0, 0, 0, 0, 0.0f, nullptr, a.Rf[1 - (it.t & 1)]};
@@ -872,8 +843,7 @@ __global__ void __launch_bounds__(Loop<T, 2>::THREADS, CTAS)
                     load(st);
                     if (got < 32) break;
                 }
-            },
-            [](State &, int) {});
+            });
     } else {
         // ---- compute: the first NWF warps advance the source field and
         // accumulate, the others advance the adjoint field ----
