@@ -402,8 +402,11 @@ __device__ __forceinline__ void loop_publisher(LoopShared<NW> &sh, const LoopGeo
     for (int item = 0;; ++item) {
         const int s0 = item * nstage;
         int n = more_than(s0);
-        if (n < 0 || n == kNoMoreItems) return;
+        if (n < 0) return;
+        // (the compute warps can be through with the last items when the
+        // publisher still has some of them ahead, so the item says what is left)
         const long long tk = *(volatile long long *)&sh.item[item % kItemRing];
+        if (tk < 0) return;
         __syncwarp();
         if (lane == 0) st_release_cta(&sh.items_read, item + 1);
         const Item it = item_of(tk, geo.nshot, prog.shots, geo.nsteps, geo.ncol);
