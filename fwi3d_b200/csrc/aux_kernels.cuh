@@ -85,40 +85,59 @@ __global__ void start_source_kernel(float *__restrict__ A, long long vol, int ld
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint injection: Pr[cell] += idh3 * d(receiver) for every receiver on the
-// cell, time-reversed (inject_seismogram / inject_residuo,
-// src/migration/migration.cu:119-132, src/inversion/inversion.cu:385-398).
-// Receivers sharing a cell are added one after another in receiver order,
-// which keeps the sum deterministic where the reference uses atomicAdd.
+// Adjoint sources: the sum of idh3 * d(receiver) over the receivers on a cell
+// (inject_seismogram / inject_residuo, src/migration/migration.cu:119-132,
+// src/inversion/inversion.cu:385-398), in receiver order, which keeps it
+// deterministic where the reference uses atomicAdd.  Data [R][nt] -> [nt][ncell]
+// in the order of the cell lists, 32x32 tiles through shared memory; the
+// receivers of cell u are rid[first[u]] .. rid[first[u+1]-1].
 // ---------------------------------------------------------------------------
-__global__ void inject_adjoint_kernel(float *__restrict__ Pr, const BatchInfo *__restrict__ bi,
-                                      const long long *__restrict__ cell,
-                                      const int *__restrict__ first, const int *__restrict__ rid,
-                                      const float *__restrict__ data_tm, int sample, float idh3)
+__global__ void gather_data_kernel(const float *__restrict__ in, int nt, int ncell, const int *__restrict__ first,
+                                   const int *__restrict__ rid, float idh3, float *__restrict__ out)
 {
-    const int ncell = bi->ncell, R = bi->R;
-    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < ncell; u += gridDim.x * blockDim.x) {
-        float v = Pr[cell[u]];
-        for (int k = first[u]; k < first[u + 1]; ++k)
-            v += idh3 * data_tm[(long long)sample * R + rid[k]];
-        Pr[cell[u]] = v;
-    }
-}
-
-// [rows][cols] -> [cols][rows], 32x32 tiles through shared memory.
-__global__ void transpose_kernel(const float *__restrict__ in, long long rows, long long cols,
-                                 float *__restrict__ out)
-{
-    __shared__ float t[32][33];
-    const long long r0 = (long long)blockIdx.y * 32, c0 = (long long)blockIdx.x * 32;
+    __shared__ float tile[32][33];
+    const int u0 = blockIdx.x * 32, t0 = blockIdx.y * 32;
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const long long r = r0 + k, c = c0 + threadIdx.x;
-        if (r < rows && c < cols) t[k][threadIdx.x] = in[r * cols + c];
+        const int u = u0 + k, t = t0 + threadIdx.x;
+        if (u < ncell && t < nt) {
+            float v = 0.0f;
+            for (int q = first[u]; q < first[u + 1]; ++q) v += idh3 * in[(long long)rid[q] * nt + t];
+            tile[k][threadIdx.x] = v;
+        }
     }
     __syncthreads();
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const long long c = c0 + k, r = r0 + threadIdx.x;
-        if (r < rows && c < cols) out[c * rows + r] = t[threadIdx.x][k];
+        const int t = t0 + k, u = u0 + threadIdx.x;
+        if (u < ncell && t < nt) out[(long long)t * ncell + u] = tile[threadIdx.x][k];
+    }
+}
+
+// Adjoint source of step 0, before the time loop adds the others.
+__global__ void inject_adjoint_kernel(float *__restrict__ Pr, const BatchInfo *__restrict__ bi,
+                                      const long long *__restrict__ cell, const float *__restrict__ data)
+{
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < bi->ncell; u += gridDim.x * blockDim.x)
+        Pr[cell[u]] += data[u];
+}
+
+// Samples of the receiver cells [nt][ncell] -> seismograms [R][nt].  The
+// reference records P after its in-place damping (src/modeling/modeling.cu:378,
+// 391-392), so every receiver has its factor (1 without a damping boundary).
+__global__ void scatter_seis_kernel(const float *__restrict__ in, int nt, int ncell, const int *__restrict__ first,
+                                    const int *__restrict__ rid, const float *__restrict__ damp, float *__restrict__ out)
+{
+    __shared__ float tile[32][33];
+    const int u0 = blockIdx.x * 32, t0 = blockIdx.y * 32;
+    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+        const int t = t0 + k, u = u0 + threadIdx.x;
+        if (u < ncell && t < nt) tile[k][threadIdx.x] = in[(long long)t * ncell + u];
+    }
+    __syncthreads();
+    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+        const int u = u0 + k, t = t0 + threadIdx.x;
+        if (u < ncell && t < nt)
+            for (int q = first[u]; q < first[u + 1]; ++q)
+                out[(long long)rid[q] * nt + t] = damp[rid[q]] * tile[threadIdx.x][k];
     }
 }
 

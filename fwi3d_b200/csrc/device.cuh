@@ -33,15 +33,11 @@ struct BatchInfo {
     int src[kMaxBatch][3];        // source cell (i=z, j=x, k=y), padded indices
 };
 
-// Receivers of a batch by the column of the tiling that owns their cells:
-// entry u of column (shot, col) is one distinct cell, sorted by y plane; its
-// receivers are rid[first[u]] .. rid[first[u+1]-1].
+// Distinct receiver cells of a batch, sorted by the column (shot, col) of the
+// tiling that owns them and by y plane.
 struct CellLists {
-    const int *col_first;         // [shots * columns + 1] first entry of each column
-    const long long *cell;        // batch-flat cell index
-    const int *y;                 // y plane of the cell
-    const int *first;             // [entries + 1]
-    const int *rid;
+    const int *below;             // [shots * columns][nyy + 1] place in the list of a column's first cell at or above a plane
+    const long long *cell;        // [ncell] batch-flat cell index
 };
 
 // Progress of the items of a time-loop kernel: an item is one step of one
@@ -73,8 +69,7 @@ struct FwdArgs {
     const float *wavelet;         // [nt]
     const BatchInfo *binfo;
     CellLists rec;
-    const float *rec_damp;        // [R] damping at the receiver (1 without ABC)
-    float *seis_tm;               // [nt][R] time-major seismograms
+    float *seis_tm;               // [nt][ncell] samples of the receiver cells
     LoopProgress prog;
 };
 
@@ -99,7 +94,7 @@ struct BwdArgs {
     const float *wavelet;
     const BatchInfo *binfo;
     CellLists inj;
-    const float *data_tm;         // [nt][R] observed data or residuals, time-major
+    const float *data_tm;         // [nt][ncell] adjoint sources of the receiver cells
     LoopProgress prog;
 };
 

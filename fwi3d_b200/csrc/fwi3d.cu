@@ -294,7 +294,7 @@ struct fwi_ctx {
     DevBuf<float> seis_tm, data_tm, raw;
     DevBuf<long long> inj_cell;
     DevBuf<float> rec_damp;
-    DevBuf<int> inj_first, inj_rid, inj_y, col_first;
+    DevBuf<int> inj_first, inj_rid, inj_below;
     DevBuf<unsigned long long> ticket;
     DevBuf<long long> progress;
     DevBuf<BatchInfo> binfo;
@@ -436,12 +436,12 @@ void ensure_fields(fwi_ctx *c, bool adjoint)
 
 // Per-batch shot tables: sources, receiver damping and the distinct receiver
 // cells with their receivers, listed by the column of the tiling that owns
-// them and within a column by (y, x, z).
+// them and within a column by (y, x, z).  below: see CellLists.
 struct BatchTables {
     BatchInfo info{};
     std::vector<float> damp;
     std::vector<long long> ucell;
-    std::vector<int> ufirst, urid, uy, col_first;
+    std::vector<int> ufirst, urid, below;
     std::vector<int> shot_nrec;
 };
 
@@ -472,18 +472,18 @@ BatchTables build_batch(fwi_ctx *c, const int *shots, int n, int tz, int tx)
     std::vector<int> order(t.info.R);
     for (int r = 0; r < t.info.R; ++r) order[r] = r;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key[a] < key[b]; });
-    t.col_first.assign((size_t)n * ncol + 1, 0);
+    t.below.assign((size_t)n * ncol * (c->nyy + 1), 0);
     for (int q = 0; q < t.info.R; ++q) {
         const int r = order[q];
         if (t.ucell.empty() || t.ucell.back() != cell[r]) {
             t.ucell.push_back(cell[r]);
             t.ufirst.push_back(q);
-            t.uy.push_back((int)(cell[r] % c->vol / ((long long)c->ldz * c->nxx)));
-            ++t.col_first[key[r] / c->vol + 1];
+            const long long y = cell[r] % c->vol / ((long long)c->ldz * c->nxx);
+            ++t.below[key[r] / c->vol * (c->nyy + 1) + y + 1];
         }
         t.urid.push_back(r);
     }
-    for (size_t q = 1; q < t.col_first.size(); ++q) t.col_first[q] += t.col_first[q - 1];
+    for (size_t q = 1; q < t.below.size(); ++q) t.below[q] += t.below[q - 1];
     t.ufirst.push_back(t.info.R);
     t.info.ncell = (int)t.ucell.size();
     return t;
@@ -491,7 +491,7 @@ BatchTables build_batch(fwi_ctx *c, const int *shots, int n, int tz, int tx)
 
 CellLists cell_lists(const fwi_ctx *c)
 {
-    return {c->col_first.p, c->inj_cell.p, c->inj_y.p, c->inj_first.p, c->inj_rid.p};
+    return {c->inj_below.p, c->inj_cell.p};
 }
 
 void upload_batch(fwi_ctx *c, const BatchTables &t)
@@ -499,21 +499,19 @@ void upload_batch(fwi_ctx *c, const BatchTables &t)
     const int R = std::max(t.info.R, 1);
     c->rec_damp.ensure(R);
     c->inj_cell.ensure(R);
-    c->inj_y.ensure(R);
     c->inj_first.ensure(R + 1);
     c->inj_rid.ensure(R);
-    c->col_first.ensure(t.col_first.size());
+    c->inj_below.ensure(t.below.size());
     const size_t need = (size_t)c->p.nt * R;
     c->seis_tm.ensure(need);
     c->data_tm.ensure(need);
     c->raw.ensure(need);
     c->binfo.ensure(1);
     CK(cudaMemcpyAsync(c->binfo.p, &t.info, sizeof(BatchInfo), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->col_first.p, t.col_first.data(), t.col_first.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->inj_below.p, t.below.data(), t.below.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     if (t.info.R) {
         CK(cudaMemcpyAsync(c->rec_damp.p, t.damp.data(), t.info.R * sizeof(float), cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemcpyAsync(c->inj_cell.p, t.ucell.data(), t.ucell.size() * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
-        CK(cudaMemcpyAsync(c->inj_y.p, t.uy.data(), t.uy.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemcpyAsync(c->inj_first.p, t.ufirst.data(), t.ufirst.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemcpyAsync(c->inj_rid.p, t.urid.data(), t.urid.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     }
@@ -638,7 +636,6 @@ FwdLaunch make_fwd(fwi_ctx *c, int n, int tile, bool record)
     a.wavelet = c->wavelet.p;
     a.binfo = c->binfo.p;
     a.rec = cell_lists(c);
-    a.rec_damp = c->rec_damp.p;
     a.seis_tm = c->seis_tm.p;
     return L;
 }
@@ -705,13 +702,13 @@ void forward_loop(fwi_ctx *c, int n, bool record)
     CK(cudaEventRecord(c->ev[1], c->stream));
 }
 
-void backward_loop(fwi_ctx *c, int n, bool grad)
+void backward_loop(fwi_ctx *c, int n, int ncell, bool grad)
 {
     BwdLaunch L = make_bwd(c, n, tuned_bwd(c), grad);
     CK(cudaEventRecord(c->ev[2], c->stream));
     // adjoint source of step 0; the loop adds the others
-    inject_adjoint_kernel<<<64, 256, 0, c->stream>>>(c->Rf[0].p, c->binfo.p, c->inj_cell.p, c->inj_first.p,
-                                                     c->inj_rid.p, c->data_tm.p, c->p.nt - 1, c->idh3);
+    inject_adjoint_kernel<<<64, 256, 0, c->stream>>>(c->Rf[0].p, c->binfo.p, c->inj_cell.p,
+                                                     c->data_tm.p + (size_t)(c->p.nt - 1) * ncell);
     CK(cudaGetLastError());
     ++c->launches;
     launch_loop(c, L, n);
@@ -738,20 +735,22 @@ void require_ready(fwi_ctx *c)
     if (!c->have_geom) fail(FWI_ERR_STATE, "no geometry set");
 }
 
-// Device seismogram block [nt][R] -> Fortran per shot [R][nt] at dst.
-void seis_to_fortran(fwi_ctx *c, int R, float *dst)
+// Samples of a batch's receiver cells -> seismograms, Fortran per shot [R][nt], at dst.
+void seis_to_fortran(fwi_ctx *c, int ncell, float *dst)
 {
-    dim3 grid((R + 31) / 32, (c->p.nt + 31) / 32);
-    transpose_kernel<<<grid, dim3(32, 8), 0, c->stream>>>(c->seis_tm.p, c->p.nt, R, dst);
+    dim3 grid((ncell + 31) / 32, (c->p.nt + 31) / 32);
+    scatter_seis_kernel<<<grid, dim3(32, 8), 0, c->stream>>>(c->seis_tm.p, c->p.nt, ncell, c->inj_first.p, c->inj_rid.p,
+                                                             c->rec_damp.p, dst);
     CK(cudaGetLastError());
     ++c->launches;
 }
 
-// Fortran per shot [R][nt] at src (device) -> data_tm [nt][R].
-void data_from_fortran(fwi_ctx *c, int R, const float *src, cudaStream_t st = nullptr)
+// Fortran per shot [R][nt] at src (device) -> adjoint sources of the receiver cells.
+void data_from_fortran(fwi_ctx *c, int ncell, const float *src, cudaStream_t st = nullptr)
 {
-    dim3 grid((c->p.nt + 31) / 32, (R + 31) / 32);
-    transpose_kernel<<<grid, dim3(32, 8), 0, st ? st : c->stream>>>(src, R, c->p.nt, c->data_tm.p);
+    dim3 grid((ncell + 31) / 32, (c->p.nt + 31) / 32);
+    gather_data_kernel<<<grid, dim3(32, 8), 0, st ? st : c->stream>>>(src, c->p.nt, ncell, c->inj_first.p,
+                                                                      c->inj_rid.p, c->idh3, c->data_tm.p);
     CK(cudaGetLastError());
     ++c->launches;
 }
@@ -788,15 +787,15 @@ void model_impl(fwi_ctx *c, const int *shots, int nshots, float *out, bool out_i
             shot_pads(c, shots + s0, n, shots + s0 + n, std::min(c->B, nshots - s0 - n));
         update_coeff(c);
         const int R = t.info.R;
-        if (R) CK(cudaMemsetAsync(c->seis_tm.p, 0, (size_t)c->p.nt * R * sizeof(float), c->stream));
+        if (R) CK(cudaMemsetAsync(c->seis_tm.p, 0, (size_t)c->p.nt * t.info.ncell * sizeof(float), c->stream));
         start_forward(c, n);
         forward_loop(c, n, true);
         const size_t cnt = (size_t)c->p.nt * R;
         if (R) {
             if (out_is_device) {
-                seis_to_fortran(c, R, out + off);
+                seis_to_fortran(c, t.info.ncell, out + off);
             } else {
-                seis_to_fortran(c, R, c->raw.p);
+                seis_to_fortran(c, t.info.ncell, c->raw.p);
                 CK(cudaMemcpyAsync(out + off, c->raw.p, cnt * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
             }
         }
@@ -833,7 +832,7 @@ void migrate_impl(fwi_ctx *c, const int *shots, int nshots, const float *data, b
         bool data_on_side = false;
         if (R) {
             if (data_is_device) {
-                data_from_fortran(c, R, data + off);
+                data_from_fortran(c, t.info.ncell, data + off);
             } else {
                 // Host data: the forward pass does not read it, so its copy and
                 // transpose run beside that pass, once everything queued so far
@@ -842,7 +841,7 @@ void migrate_impl(fwi_ctx *c, const int *shots, int nshots, const float *data, b
                 CK(cudaStreamWaitEvent(c->copy_stream, c->ev_free, 0));
                 CK(cudaMemcpyAsync(c->raw.p, data + off, cnt * sizeof(float), cudaMemcpyHostToDevice,
                                    c->copy_stream));
-                data_from_fortran(c, R, c->raw.p, c->copy_stream);
+                data_from_fortran(c, t.info.ncell, c->raw.p, c->copy_stream);
                 CK(cudaEventRecord(c->ev_data, c->copy_stream));
                 data_on_side = true;
             }
@@ -853,7 +852,7 @@ void migrate_impl(fwi_ctx *c, const int *shots, int nshots, const float *data, b
         CK(cudaMemsetAsync(c->Rf[0].p, 0, bytes, c->stream));
         CK(cudaMemsetAsync(c->Rf[1].p, 0, bytes, c->stream));
         if (data_on_side) CK(cudaStreamWaitEvent(c->stream, c->ev_data, 0));
-        backward_loop(c, n, grad);
+        backward_loop(c, n, t.info.ncell, grad);
         check_status(c);
         float ms = 0;
         CK(cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
@@ -1361,8 +1360,7 @@ int fwi_destroy(fwi_ctx *c)
     c->inj_cell.release();
     c->inj_first.release();
     c->inj_rid.release();
-    c->inj_y.release();
-    c->col_first.release();
+    c->inj_below.release();
     c->ticket.release();
     c->progress.release();
     c->binfo.release();

@@ -309,6 +309,50 @@ __device__ __forceinline__ int stages_done(const LoopShared<NW> &sh, int lane)
     return __reduce_min_sync(0xffffffffu, v);
 }
 
+// The receiver cells of a column in plane order, for the warp that follows the
+// planes.  Lane l holds cell u + l of the list and the list's place at plane
+// base + l, both fetched ahead of the planes.
+struct CellCursor {
+    const int *below;             // null: nothing to do
+    const long long *cells;
+    int u, last, base, ahead, nyy;
+    long long cell;
+
+    __device__ __forceinline__ void open(const CellLists &lists, int column, int planes, int lane)
+    {
+        cells = lists.cell;
+        below = lists.below + (long long)column * (planes + 1);
+        nyy = planes;
+        base = 0;
+        ahead = below[min(lane, nyy)];
+        u = __shfl_sync(0xffffffffu, ahead, 0);
+        last = below[nyy];
+        if (u == last) below = nullptr;
+        fetch(lane);
+    }
+    __device__ __forceinline__ void fetch(int lane)
+    {
+        if (u + lane < last) cell = cells[u + lane];
+    }
+    // End of the list's part below plane n.
+    __device__ __forceinline__ int end_below(int n, int lane)
+    {
+        if (n - base > 31) {
+            base = n;
+            ahead = below[min(n + lane, nyy)];
+        }
+        return __shfl_sync(0xffffffffu, ahead, n - base);
+    }
+};
+
+// Further cells of a plane are taken in bursts of kBurst per lane, whose loads
+// are in flight together: a warp that takes 32 at a time is latency-bound, and
+// with it the steps that wait for its publications.  201^3 cells with a 50-cell
+// pad, 404010 receivers on ten layers: forward 245 us a step by 32, 84 now (94
+// with 16 per lane; 61 without receivers), backward 279 and 137; receivers in
+// every cell of 44^3, 8-cell pad: forward 35 and 11, backward 162 and 13.
+constexpr int kBurst = 8;
+
 // What the roles of a CTA need to know of the loop.
 struct LoopGeo {
     int nshot, nsteps, ncol, ntz, nyy;
@@ -516,51 +560,43 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
             });
     } else if (warp == NW + 1) {
         // Samples of the level the item stores, u^(t+1), a few planes behind the
-        // publication where they can be.  Lane l holds entry u + l of the
-        // column's list, looked up ahead of its plane.
+        // publication where they can be.
         struct State {
-            int u, last, sample, y, first, end;
-            long long cell;
+            CellCursor at;
             const float *F;
+            float *dst;
         };
-        const int nrec = a.binfo->R;
-        auto load = [&](State &st) {
-            const int e = st.u + lane;
-            st.y = 0x7fffffff;
-            if (e < st.last) {
-                st.y = a.rec.y[e];
-                st.cell = a.rec.cell[e];
-                st.first = a.rec.first[e];
-                st.end = a.rec.first[e + 1];
-            }
-        };
+        const int ncell = a.binfo->ncell;
         loop_publisher<kSampleLead>(
             sh, geo, a.prog, lane,
             [&](const Item &it) {
-                State st{0, 0, it.t + 1 - a.tlag, 0, 0, 0, 0, a.F[1 - (it.t & 1)]};
-                if (st.sample > 0 && it.t + 1 < a.nsteps) {
-                    st.u = a.rec.col_first[it.shot * a.ncol + it.col];
-                    st.last = a.rec.col_first[it.shot * a.ncol + it.col + 1];
+                const int sample = it.t + 1 - a.tlag;
+                State st;
+                st.at.below = nullptr;
+                if (sample > 0 && it.t + 1 < a.nsteps) {
+                    st.at.open(a.rec, it.shot * a.ncol + it.col, a.nyy, lane);
+                    st.F = a.F[1 - (it.t & 1)];
+                    st.dst = a.seis_tm + (long long)sample * ncell;
                 }
-                load(st);
                 return st;
             },
             [&](State &st, int n) {
-                for (;;) {
-                    const bool mine = st.y < n;
-                    const int got = __popc(__ballot_sync(0xffffffffu, mine));
-                    if (got == 0) break;
-                    if (mine) {
-                        const float v = __ldcg(st.F + st.cell);
-                        for (int k = st.first; k < st.end; ++k) {
-                            const int r = a.rec.rid[k];
-                            a.seis_tm[(long long)st.sample * nrec + r] = a.rec_damp[r] * v;
-                        }
-                    }
-                    st.u += got;
-                    load(st);
-                    if (got < 32) break;
+                if (!st.at.below) return;
+                const int end = st.at.end_below(n, lane);
+                if (st.at.u == end) return;
+                if (st.at.u + lane < end) st.dst[st.at.u + lane] = __ldcg(st.F + st.at.cell);
+                for (int e0 = st.at.u + 32 + lane; e0 < end; e0 += 32 * kBurst) {
+                    float v[kBurst];
+#pragma unroll
+                    for (int k = 0; k < kBurst; ++k)
+                        if (e0 + 32 * k < end) v[k] = __ldcg(st.F + st.at.cells[e0 + 32 * k]);
+#pragma unroll
+                    for (int k = 0; k < kBurst; ++k)
+                        if (e0 + 32 * k < end) st.dst[e0 + 32 * k] = v[k];
                 }
+                __syncwarp();
+                st.at.u = end;
+                st.at.fetch(lane);
             });
     } else {
         // ---- compute ----
@@ -800,52 +836,53 @@ __global__ void __launch_bounds__(Loop<T, 2>::THREADS, CTAS)
                 }
             });
     } else if (warp == NW + 1) {
-        // Before publishing: the adjoint source of step t+1 (inject_seismogram
-        // / inject_residuo, src/migration/migration.cu:119-132,
-        // src/inversion/inversion.cu:385-398) is added to the level the item
-        // stores.  Lane l holds entry u + l of the column's list, with the sum
-        // of its receivers in receiver order, loaded ahead of its plane.
+        // Before publishing: the adjoint source of step t+1 is added to the level
+        // the item stores.  Lane l has that of its cell at hand, too.
         struct State {
-            int u, last, y;
-            long long cell;
-            float f;
-            const float *d;
+            CellCursor at;
+            const float *src;
             float *Pr;
+            float f;
         };
-        const int nrec = a.binfo->R;
-        auto load = [&](State &st) {
-            const int e = st.u + lane;
-            st.y = 0x7fffffff;
-            if (e < st.last) {
-                st.y = a.inj.y[e];
-                st.cell = a.inj.cell[e];
-                float f = 0.0f;
-                for (int k = a.inj.first[e]; k < a.inj.first[e + 1]; ++k) f += a.idh3 * st.d[a.inj.rid[k]];
-                st.f = f;
-            }
+        const int ncell = a.binfo->ncell;
+        auto fetch = [&](State &st) {
+            st.at.fetch(lane);
+            if (st.at.u + lane < st.at.last) st.f = st.src[st.at.u + lane];
         };
         loop_publisher<0>(
             sh, geo, a.prog, lane,
             [&](const Item &it) {
-                State st{0, 0, 0, 0, 0.0f, nullptr, a.Rf[1 - (it.t & 1)]};
+                State st;
+                st.at.below = nullptr;
                 if (it.t + 1 < a.nt) {
-                    st.u = a.inj.col_first[it.shot * a.ncol + it.col];
-                    st.last = a.inj.col_first[it.shot * a.ncol + it.col + 1];
-                    st.d = a.data_tm + (long long)(a.nt - 2 - it.t) * nrec;
+                    st.Pr = a.Rf[1 - (it.t & 1)];
+                    st.src = a.data_tm + (long long)(a.nt - 2 - it.t) * ncell;
+                    st.at.open(a.inj, it.shot * a.ncol + it.col, a.nyy, lane);
+                    fetch(st);
                 }
-                load(st);
                 return st;
             },
             [&](State &st, int n) {
-                for (;;) {
-                    const bool mine = st.y < n;
-                    const int got = __popc(__ballot_sync(0xffffffffu, mine));
-                    if (got == 0) break;
-                    if (mine) red_add(st.Pr + st.cell, st.f);
-                    st.u += got;
-                    load(st);
-                    if (got < 32) break;
+                if (!st.at.below) return;
+                const int end = st.at.end_below(n, lane);
+                if (st.at.u == end) return;
+                if (st.at.u + lane < end) red_add(st.Pr + st.at.cell, st.f);
+                for (int e0 = st.at.u + 32 + lane; e0 < end; e0 += 32 * kBurst) {
+                    float f[kBurst];
+                    long long cell[kBurst];
+#pragma unroll
+                    for (int k = 0; k < kBurst; ++k)
+                        if (e0 + 32 * k < end) {
+                            f[k] = st.src[e0 + 32 * k];
+                            cell[k] = st.at.cells[e0 + 32 * k];
+                        }
+#pragma unroll
+                    for (int k = 0; k < kBurst; ++k)
+                        if (e0 + 32 * k < end) red_add(st.Pr + cell[k], f[k]);
                 }
+                __syncwarp();
+                st.at.u = end;
+                fetch(st);
             });
     } else {
         // ---- compute: the first NWF warps advance the source field and
