@@ -70,6 +70,37 @@ __global__ void sum_slots_kernel(float *__restrict__ acc, long long vol, int nsl
     }
 }
 
+// Accumulators of one time loop: z x x x y cells of the box per shot with z pitch
+// ld, image and illumination by blockIdx.y, times kAccScale.  A value that is not
+// finite has left the range that the scale leaves and sets *over.
+__global__ void check_loop_sums_kernel(const float *__restrict__ sums, long long n, unsigned *__restrict__ over)
+{
+    bool bad = false;
+    const float4 *s = reinterpret_cast<const float4 *>(sums);
+    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n / 4; c += (long long)gridDim.x * blockDim.x) {
+        const float4 v = s[c];
+        bad |= !isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z) || !isfinite(v.w);
+    }
+    if (bad) *over = 1u;
+}
+
+// Adds them to the accumulators, whose box starts at `box`, unless *over, and
+// leaves them at 0.
+__global__ void fold_loop_sums_kernel(float *__restrict__ sums, long long to_illum, int ld, int nx, int ny, int nshot,
+                                      float *__restrict__ image, float *__restrict__ illum, long long box,
+                                      long long vol, int ldz, int nxx, const unsigned *__restrict__ over)
+{
+    sums += blockIdx.y * to_illum;
+    float *acc = (blockIdx.y ? illum : image) + box;
+    const bool drop = *over != 0u;
+    for_cells(ld, nx, ny * nshot, [&](int i, int j, int ks, long long r) {
+        const float v = sums[r * ld + i];
+        if (v == 0.0f) return;
+        if (!drop) acc[ks / ny * vol + ((long long)(ks % ny) * nxx + j) * ldz + i] += v * (1.0f / kAccScale);
+        sums[r * ld + i] = 0.0f;
+    });
+}
+
 // First source sample of every shot: A[src] = idh3 * w[0]
 // (src/modeling/modeling.cu:347-348 at t = 0).
 __global__ void start_source_kernel(float *__restrict__ A, long long vol, int ldz, int nxx,

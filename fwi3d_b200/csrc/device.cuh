@@ -19,6 +19,10 @@ constexpr float W4 = 0.001785714285f;
 
 constexpr int kMaxBatch = 64;      // shots per launch
 constexpr int kMaxPad = 1024;      // largest pad width the damper table holds
+// Image and illumination accumulate in reductions, which take what is below
+// 2^-126 for 0.  Times 2^24 an addend that FP32 holds, the least being 2^-149, stays
+// above that, and what a sum loses is below half of the least.
+constexpr float kAccScale = 0x1p24f;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s cap on any device wait
 
 // Error bits the kernels raise in g_status (read back by the host).
@@ -79,7 +83,7 @@ struct BwdArgs {
     long long vol;
     int ntz, ncol;
     int nsteps, nt;               // N = nt + tlag, wavelet and data length
-    float gscale;                 // 1/dt (gradient imaging condition)
+    float gscale;                 // acc_scale / dt (gradient imaging condition)
     float idh3;
     int subtract_src;             // remove the source while rebuilding Ps
     int vel_slots;                // 1: every shot reads velocity slot 0; B: shot s reads slot s
@@ -89,8 +93,13 @@ struct BwdArgs {
     int s0;                       // F[s0] holds the older of the two forward levels
     float *F[2];                  // source field: step t reads F[(s0 + t) & 1], overwrites the other
     float *Rf[2];                 // adjoint field: step t reads Rf[t & 1], overwrites the other
-    float *image;                 // image or gradient accumulator (batch base)
-    float *illum;                 // illumination accumulator (batch base)
+    float *image;                 // image or gradient accumulator, of cell (0, 0, 0) of the first shot
+    long long to_illum;           // from there to the illumination
+    int acc_ld;                   // pitches of the accumulators: x rows,
+    long long acc_plane;          // y planes
+    long long acc_shot;           // and shots
+    float acc_scale;              // what is added is scaled by this
+    int acc_direct;               // loads and stores instead of reductions in L2
     const float *wavelet;
     const BatchInfo *binfo;
     CellLists inj;

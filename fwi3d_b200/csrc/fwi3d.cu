@@ -313,6 +313,10 @@ struct fwi_ctx {
     bool shot_rbc = false;
     fwi_rbc shot_rbc_params{};
     uint64_t shot_rbc_seed = 0;
+    // [image, illumination][B] sums of one backward loop over the accumulated box;
+    // empty where memory is short
+    DevBuf<float> loop_sums;
+    DevBuf<unsigned> over;    // they have left their range
     bool acc_dirty = false;
 
     // geometry (padded grid indices)
@@ -419,6 +423,25 @@ float host_cerjan(const fwi_ctx *c, int i, int j, int k)
     return s2 - 5.0f;
 }
 
+// The cells whose image and illumination accumulate, in padded indices.
+struct AccBox {
+    int z0, z1, x0, x1, y0, y1;
+    int nx() const { return x1 - x0; }
+    int ny() const { return y1 - y0; }
+    // z extent from and to quads
+    int zq() const { return z0 & ~3; }
+    int ld() const { return ((z1 + 3) & ~3) - zq(); }
+    long long size() const { return (long long)ld() * nx() * ny(); }
+};
+
+AccBox acc_box(const fwi_ctx *c)
+{
+    if (c->p.flags & FWI_FLAG_PAD_ACCUMULATE)  // every updated cell
+        return {4, c->nzz - 4, 4, c->nxx - 4, 4, c->nyy - 4};
+    const int nb = c->g.nb;  // the physical box, the only cells that the post-processing reads
+    return {nb, nb + c->g.nz, nb, nb + c->g.nx, nb, nb + c->g.ny};
+}
+
 void ensure_fields(fwi_ctx *c, bool adjoint)
 {
     const size_t n = (size_t)c->B * c->vol;
@@ -432,6 +455,26 @@ void ensure_fields(fwi_ctx *c, bool adjoint)
             CK(cudaMemsetAsync(c->acc_ill.p, 0, n * sizeof(float), c->stream));
         }
     }
+}
+
+// Whether the backward loop sums into loop_sums.  It does without where memory is
+// short (what a context needs later, three volumes at most beside the data, goes
+// first), and where the illumination would leave the range that the scale
+// leaves: a field of 8 times the source's amplitude over all steps.  That takes
+// cells below 2.5 mm.
+bool use_loop_sums(fwi_ctx *c)
+{
+    const double amp = 8.0 * 1e5 * c->idh3;
+    if (amp * amp * c->nsteps * kAccScale > 1e38) return false;
+    c->over.ensure(1);
+    if (c->loop_sums.p) return true;
+    const size_t n = 2 * c->B * acc_box(c).size();
+    size_t free_bytes = 0, total = 0;
+    CK(cudaMemGetInfo(&free_bytes, &total));
+    if (free_bytes < (n + 3 * (size_t)c->vol) * sizeof(float) + (1ull << 30)) return false;
+    c->loop_sums.ensure(n);
+    CK(cudaMemsetAsync(c->loop_sums.p, 0, n * sizeof(float), c->stream));
+    return true;
 }
 
 // Per-batch shot tables: sources, receiver damping and the distinct receiver
@@ -640,7 +683,7 @@ FwdLaunch make_fwd(fwi_ctx *c, int n, int tile, bool record)
     return L;
 }
 
-BwdLaunch make_bwd(fwi_ctx *c, int n, int tile, bool grad)
+BwdLaunch make_bwd(fwi_ctx *c, int n, int tile, bool grad, bool sums)
 {
     BwdLaunch L;
     L.k = bwd_kernel(tile, grad, (c->p.flags & FWI_FLAG_GRAD_DY) != 0);
@@ -656,17 +699,28 @@ BwdLaunch make_bwd(fwi_ctx *c, int n, int tile, bool grad)
         a.Rf[b] = c->Rf[b].p;
     }
     L.m.mv = make_map(c->vc.p, c->nzz, c->nxx, c->nyy, c->ldz, c->vel_slots, L.k.tz, L.k.tx);
-    if (c->p.flags & FWI_FLAG_PAD_ACCUMULATE) {  // every updated cell
-        a.acc_z0 = a.acc_x0 = a.acc_y0 = 4;
-        a.acc_z1 = c->nzz - 4;
-        a.acc_x1 = c->nxx - 4;
-        a.acc_y1 = c->nyy - 4;
-    } else {  // the physical box, the only cells that the post-processing reads
-        a.acc_z0 = a.acc_x0 = a.acc_y0 = c->g.nb;
-        a.acc_z1 = c->g.nb + c->g.nz;
-        a.acc_x1 = c->g.nb + c->g.nx;
-        a.acc_y1 = c->g.nb + c->g.ny;
+    const AccBox box = acc_box(c);
+    a.acc_z0 = box.z0;
+    a.acc_z1 = box.z1;
+    a.acc_x0 = box.x0;
+    a.acc_x1 = box.x1;
+    a.acc_y0 = box.y0;
+    a.acc_y1 = box.y1;
+    if (sums) {
+        a.acc_ld = box.ld();
+        a.acc_plane = (long long)box.ld() * box.nx();
+        a.acc_shot = box.size();
+        a.image = c->loop_sums.p - box.y0 * a.acc_plane - (long long)box.x0 * box.ld() - box.zq();
+        a.to_illum = c->B * box.size();
+    } else {
+        a.acc_ld = c->ldz;
+        a.acc_plane = (long long)c->ldz * c->nxx;
+        a.acc_shot = c->vol;
+        a.image = c->acc_img.p;
+        a.to_illum = c->acc_ill.p - c->acc_img.p;
     }
+    a.acc_scale = sums ? kAccScale : 1.0f;
+    a.acc_direct = !sums;
     a.nzz = c->nzz;
     a.nxx = c->nxx;
     a.nyy = c->nyy;
@@ -674,14 +728,12 @@ BwdLaunch make_bwd(fwi_ctx *c, int n, int tile, bool grad)
     a.vol = c->vol;
     a.nsteps = c->nsteps;
     a.nt = c->p.nt;
-    a.gscale = 1.0f / c->p.dt;
+    a.gscale = a.acc_scale / c->p.dt;
     a.idh3 = c->idh3;
     a.subtract_src = (c->p.flags & FWI_FLAG_SUBTRACT_SOURCE) ? 1 : 0;
     a.vel_slots = c->vel_slots;
     // the forward pass leaves u^N in F[N%2] and u^{N-1} in F[1-N%2]
     a.s0 = 1 - (c->nsteps & 1);
-    a.image = c->acc_img.p;
-    a.illum = c->acc_ill.p;
     a.wavelet = c->wavelet.p;
     a.binfo = c->binfo.p;
     a.inj = cell_lists(c);
@@ -702,9 +754,28 @@ void forward_loop(fwi_ctx *c, int n, bool record)
     CK(cudaEventRecord(c->ev[1], c->stream));
 }
 
-void backward_loop(fwi_ctx *c, int n, int ncell, bool grad)
+// The sums of a backward loop join the accumulators, unless they have left their
+// range: then *over is set and the loop counts as not done.
+void fold_loop_sums(fwi_ctx *c, int n)
 {
-    BwdLaunch L = make_bwd(c, n, tuned_bwd(c), grad);
+    const AccBox box = acc_box(c);
+    const long long start = ((long long)box.y0 * c->nxx + box.x0) * c->ldz + box.zq(), to_illum = c->B * box.size();
+    CK(cudaMemsetAsync(c->over.p, 0, sizeof(unsigned), c->stream));
+    for (int q = 0; q < 2; ++q)
+        check_loop_sums_kernel<<<grid_blocks(n * box.size() / 4), 256, 0, c->stream>>>(c->loop_sums.p + q * to_illum,
+                                                                                      n * box.size(), c->over.p);
+    dim3 grid(grid_blocks(n * box.size()), 2);
+    fold_loop_sums_kernel<<<grid, 256, 0, c->stream>>>(c->loop_sums.p, to_illum, box.ld(), box.nx(), box.ny(), n,
+                                                       c->acc_img.p, c->acc_ill.p, start, c->vol, c->ldz, c->nxx,
+                                                       c->over.p);
+    CK(cudaGetLastError());
+    c->launches += 3;
+}
+
+// sums: into loop_sums, else into the accumulators themselves.
+void backward_loop(fwi_ctx *c, int n, int ncell, bool grad, bool sums)
+{
+    BwdLaunch L = make_bwd(c, n, tuned_bwd(c), grad, sums);
     CK(cudaEventRecord(c->ev[2], c->stream));
     // adjoint source of step 0; the loop adds the others
     inject_adjoint_kernel<<<64, 256, 0, c->stream>>>(c->Rf[0].p, c->binfo.p, c->inj_cell.p,
@@ -712,6 +783,7 @@ void backward_loop(fwi_ctx *c, int n, int ncell, bool grad)
     CK(cudaGetLastError());
     ++c->launches;
     launch_loop(c, L, n);
+    if (sums) fold_loop_sums(c, n);
     CK(cudaEventRecord(c->ev[3], c->stream));
 }
 
@@ -846,19 +918,25 @@ void migrate_impl(fwi_ctx *c, const int *shots, int nshots, const float *data, b
                 data_on_side = true;
             }
         }
-        start_forward(c, n);
-        forward_loop(c, n, false);
-        const size_t bytes = (size_t)n * c->vol * sizeof(float);
-        CK(cudaMemsetAsync(c->Rf[0].p, 0, bytes, c->stream));
-        CK(cudaMemsetAsync(c->Rf[1].p, 0, bytes, c->stream));
-        if (data_on_side) CK(cudaStreamWaitEvent(c->stream, c->ev_data, 0));
-        backward_loop(c, n, t.info.ncell, grad);
-        check_status(c);
-        float ms = 0;
-        CK(cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
-        f_ms += ms;
-        CK(cudaEventElapsedTime(&ms, c->ev[2], c->ev[3]));
-        b_ms += ms;
+        bool sums = use_loop_sums(c);
+        for (bool done = false; !done; sums = false) {
+            start_forward(c, n);
+            forward_loop(c, n, false);
+            const size_t bytes = (size_t)n * c->vol * sizeof(float);
+            CK(cudaMemsetAsync(c->Rf[0].p, 0, bytes, c->stream));
+            CK(cudaMemsetAsync(c->Rf[1].p, 0, bytes, c->stream));
+            if (data_on_side) CK(cudaStreamWaitEvent(c->stream, c->ev_data, 0));
+            backward_loop(c, n, t.info.ncell, grad, sums);
+            unsigned over = 0;
+            if (sums) CK(cudaMemcpyAsync(&over, c->over.p, sizeof over, cudaMemcpyDeviceToHost, c->stream));
+            check_status(c);
+            done = !over;
+            float ms = 0;
+            CK(cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
+            f_ms += ms;
+            CK(cudaEventElapsedTime(&ms, c->ev[2], c->ev[3]));
+            b_ms += ms;
+        }
         off += cnt;
         c->acc_dirty = true;
     }
@@ -1353,6 +1431,8 @@ int fwi_destroy(fwi_ctx *c)
     for (auto &f : c->Rf) f.release();
     c->acc_img.release();
     c->acc_ill.release();
+    c->loop_sums.release();
+    c->over.release();
     c->seis_tm.release();
     c->data_tm.release();
     c->raw.release();
@@ -1813,6 +1893,7 @@ int fwi_autotune(fwi_ctx *c)
         require_ready(c);
         const bool adj = c->p.boundary == FWI_BOUNDARY_RBC;
         ensure_fields(c, adj);
+        const bool sums = adj && use_loop_sums(c);
         std::vector<int> one(1, 0);
         BatchTables t = build_batch(c, one.data(), 1, 4, 4);
         t.info.nshot = c->B;  // every slot busy, like a full batch
@@ -1849,7 +1930,7 @@ int fwi_autotune(fwi_ctx *c)
             for (int pass = 0; pass < kPasses; ++pass)
                 for (int tile = 0; tile < kNumTiles; ++tile) {
                     if (backward) {
-                        BwdLaunch L = make_bwd(c, c->B, tile, false);
+                        BwdLaunch L = make_bwd(c, c->B, tile, false, sums);
                         ms[tile] = std::min(ms[tile], timed(L));
                     } else {
                         FwdLaunch L = make_fwd(c, c->B, tile, false);
@@ -1869,6 +1950,7 @@ int fwi_autotune(fwi_ctx *c)
             const size_t bytes = (size_t)c->B * c->vol * sizeof(float);
             CK(cudaMemsetAsync(c->acc_img.p, 0, bytes, c->stream));
             CK(cudaMemsetAsync(c->acc_ill.p, 0, bytes, c->stream));
+            if (c->loop_sums.p) CK(cudaMemsetAsync(c->loop_sums.p, 0, c->loop_sums.n * sizeof(float), c->stream));
         }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
