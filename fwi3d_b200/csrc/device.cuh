@@ -162,16 +162,20 @@ __device__ __forceinline__ void st_release_gpu(long long *p, long long v)
     asm volatile("st.release.gpu.global.s64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-__device__ __forceinline__ int ld_acquire_cta(const int *p)
+template <class T>
+__device__ __forceinline__ T ld_acquire_cta(const T *p)
 {
-    int v;
-    asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
+    static_assert(sizeof(T) == 4, "32-bit counters");
+    T v;
+    asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
     return v;
 }
 
-__device__ __forceinline__ void st_release_cta(int *p, int v)
+template <class T>
+__device__ __forceinline__ void st_release_cta(T *p, T v)
 {
-    asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_addr(p)), "r"(v) : "memory");
+    static_assert(sizeof(T) == 4, "32-bit counters");
+    asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(p)), "r"(v) : "memory");
 }
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)

@@ -271,7 +271,10 @@ __device__ __forceinline__ void xz_d2(const float *H, q4 (&c)[T::R], q4 (&d)[T::
 // only zeros and are not loaded.
 // ---------------------------------------------------------------------------
 constexpr int kItemRing = 4;      // items described in shared memory at once
-constexpr int kNoMoreItems = 0x7fffffff;
+// Stages are counted modulo 2^32 and compared by differences, since a CTA of a
+// very long loop takes more than 2^31; starting here, every loop wraps.
+constexpr unsigned kFirstStage = 0u - 1000u;
+constexpr unsigned kNoMoreItems = 1u << 30;   // added to the count of a warp that is through
 
 // FIELDS: fields that advance side by side, each with its own compute warps.
 template <class T, int FIELDS>
@@ -285,7 +288,7 @@ struct Loop {
 template <int NW>
 struct LoopShared {
     long long item[kItemRing];    // tickets of the items in flight, -1 ends
-    int staged[NW];               // stages finished by each compute warp
+    unsigned staged[NW];          // stages finished by each compute warp, from kFirstStage on
     int items_read;               // items the publisher has looked up
     int abort;
 };
@@ -338,12 +341,12 @@ __device__ __forceinline__ bool wait_columns(const long long *p, long long need,
     return true;
 }
 
-// Smallest number of stages that the compute warps have finished.
+// Smallest number of stages beyond s0 that the compute warps have finished.
 template <int NW>
-__device__ __forceinline__ int stages_done(const LoopShared<NW> &sh, int lane)
+__device__ __forceinline__ int stages_done(const LoopShared<NW> &sh, unsigned s0, int lane)
 {
     int v = kNoMoreItems;
-    for (int w = lane; w < NW; w += 32) v = min(v, ld_acquire_cta(&sh.staged[w]));
+    for (int w = lane; w < NW; w += 32) v = min(v, (int)(ld_acquire_cta(&sh.staged[w]) - s0));
     return __reduce_min_sync(0xffffffffu, v);
 }
 
@@ -407,7 +410,8 @@ __device__ __forceinline__ void loop_producer(LoopShared<NW> &sh, uint64_t *full
 {
     constexpr int SC = SH - 4;
     const long long total = (long long)geo.nshot * geo.nsteps * geo.ncol;
-    int hs = 0, cs = 0, cph = 1, g = 0;  // cph: parity of the previous use of done[cs]
+    int hs = 0, cs = 0, cph = 1;  // cph: parity of the previous use of done[cs]
+    long long g = 0;              // stages issued
     bool ok = true;
     for (int item = 0; ok; ++item) {
         unsigned long long tk = 0;
@@ -450,8 +454,8 @@ __device__ __forceinline__ void loop_producer(LoopShared<NW> &sh, uint64_t *full
         loop_fail(&sh.abort);  // (the compute warps wait for the same stage and give up as well)
         // no copy may land after the CTA has gone: only the newest use of
         // each slot can still be in flight
-        for (int k = 1; k <= min(g, SH); ++k) {
-            const int st = g - k;
+        for (int k = 1; k <= SH && k <= g; ++k) {
+            const long long st = g - k;
             mbar_wait(&full[st % SH], (st / SH) & 1);
         }
     }
@@ -466,25 +470,24 @@ __device__ __forceinline__ void loop_publisher(LoopShared<NW> &sh, const LoopGeo
                                                int lane, Start start, Work work)
 {
     const int nstage = geo.nyy - 4;  // stages of an item: p = 4 .. nyy-1, y = p - 4
-    // stages finished by every compute warp, once there are more than s; -1
-    // when the wait gave up
+    // stages of the item finished by every compute warp, once there are more
+    // than s; -1 when the wait gave up
+    unsigned s0 = kFirstStage;  // stages before the item
     auto more_than = [&](int s) {
-        int n = stages_done(sh, lane);
+        int n = stages_done(sh, s0, lane);
         if (n > s) return n;
         const uint64_t t0 = global_ns();
         for (;;) {
             for (int i = 0; i < 64; ++i) {
                 __nanosleep(20);
-                if ((n = stages_done(sh, lane)) > s) return n;
+                if ((n = stages_done(sh, s0, lane)) > s) return n;
             }
             const bool late = aborted(&sh.abort) || global_ns() - t0 > 2 * kWaitLimitNs;
             if (__any_sync(0xffffffffu, late)) return -1;
         }
     };
-    for (int item = 0;; ++item) {
-        const int s0 = item * nstage;
-        int n = more_than(s0);
-        if (n < 0) return;
+    for (int item = 0;; ++item, s0 += nstage) {
+        if (more_than(0) < 0) return;
         // (the compute warps can be through with the last items when the
         // publisher still has some of them ahead, so the item says what is left)
         const long long tk = *(volatile long long *)&sh.item[item % kItemRing];
@@ -498,9 +501,9 @@ __device__ __forceinline__ void loop_publisher(LoopShared<NW> &sh, const LoopGeo
         int published = 4, stored = 4;  // the first four planes are never written
         while (published < nstage) {
             if (stored == published) {
-                n = more_than(s0 + published);
+                const int n = more_than(published);
                 if (n < 0) return;
-                stored = min(n - s0, nstage);
+                stored = min(n, nstage);
             }
             published = next_publication(published, stored, LEAD);
             const bool first = work_first(published, nstage, LEAD);
@@ -555,7 +558,7 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
     if constexpr (ABC) {
         for (int i = tid; i < a.nb; i += Loop<T, 1>::THREADS) b1s[i] = a.b1d[i];
     }
-    if (tid < NW) sh.staged[tid] = 0;
+    if (tid < NW) sh.staged[tid] = kFirstStage;
     if (tid == 0) {
         sh.items_read = 0;
         sh.abort = 0;
@@ -641,7 +644,8 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
         const int ct = min(tid, T::NT - 1);  // the last warp's spare lanes repeat its last thread
         const int lz = ct % T::TZ4, lx = ct / T::TZ4 * R;
         const int ho = (lx + 4) * T::HZ + 4 + 4 * lz, co = lx * T::TZ + 4 * lz;
-        int hs = 0, hph = 0, cs = 0, g = 0;
+        int hs = 0, hph = 0, cs = 0;
+        unsigned g = kFirstStage;  // stages finished
         for (int item = 0;; ++item) {
             bool ok = __all_sync(0xffffffffu, mbar_wait(&full[hs], hph) && !aborted(&sh.abort));
             if (!ok) {
@@ -651,7 +655,7 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
             const long long tk = *(volatile long long *)&sh.item[item % kItemRing];
             if (tk < 0) {
                 __syncwarp();
-                if (lane == 0) st_release_cta(&sh.staged[warp], kNoMoreItems);
+                if (lane == 0) st_release_cta(&sh.staged[warp], g + kNoMoreItems);
                 break;
             }
             const Item it = item_of(tk, geo.nshot, a.prog.shots, a.nsteps, a.ncol);
@@ -828,7 +832,7 @@ __global__ void __launch_bounds__(Loop<T, 2>::THREADS, CTAS)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (status_failed()) return;
-    if (tid < NW) sh.staged[tid] = 0;
+    if (tid < NW) sh.staged[tid] = kFirstStage;
     if (tid == 0) {
         sh.items_read = 0;
         sh.abort = 0;
@@ -934,7 +938,8 @@ __global__ void __launch_bounds__(Loop<T, 2>::THREADS, CTAS)
             const int ct = min(ft, T::NT - 1);  // the last warp's spare lanes repeat its last thread
             const int lz = ct % T::TZ4, lx = ct / T::TZ4 * R;
             const int ho = (lx + 4) * T::HZ + 4 + 4 * lz, co = lx * T::TZ + 4 * lz;
-            int hs = 0, hph = 0, cs = 0, g = 0;
+            int hs = 0, hph = 0, cs = 0;
+            unsigned g = kFirstStage;  // stages finished
             for (int item = 0;; ++item) {
                 bool ok = __all_sync(0xffffffffu, mbar_wait(&full[hs], hph) && !aborted(&sh.abort));
                 if (!ok) {
@@ -944,7 +949,7 @@ __global__ void __launch_bounds__(Loop<T, 2>::THREADS, CTAS)
                 const long long tk = *(volatile long long *)&sh.item[item % kItemRing];
                 if (tk < 0) {
                     __syncwarp();
-                    if (lane == 0) st_release_cta(&sh.staged[warp], kNoMoreItems);
+                    if (lane == 0) st_release_cta(&sh.staged[warp], g + kNoMoreItems);
                     break;
                 }
                 const Item it = item_of(tk, geo.nshot, a.prog.shots, a.nsteps, a.ncol);
