@@ -609,15 +609,26 @@ struct BwdLaunch {
     BwdArgs a;
 };
 
+int z_tiles(const fwi_ctx *c, const KInfo &k) { return (c->nzz - 8 + k.tz - 1) / k.tz; }
+int columns(const fwi_ctx *c, const KInfo &k) { return z_tiles(c, k) * ((c->nxx - 8 + k.tx - 1) / k.tx); }
+int progress_ring(const fwi_ctx *c) { return c->nyy / 4 + 3; }
+
+// Counters for the loops of a call, before the first of them: a buffer that
+// grew between two loops would wait for the one that runs.
+void reserve_progress(fwi_ctx *c, int n, int ncol)
+{
+    c->ticket.ensure(1);
+    c->progress.ensure((size_t)n * progress_ring(c) * ncol * kCounterStride);
+}
+
 // Columns, progress counters and grid of a time loop over n shots: one wave of
 // resident CTAs at most.
 template <class L>
 void plan_loop(fwi_ctx *c, L &l, int n)
 {
     prepare_kernel(l.k);
-    const int ntz = (c->nzz - 8 + l.k.tz - 1) / l.k.tz, ntx = (c->nxx - 8 + l.k.tx - 1) / l.k.tx;
-    l.a.ntz = ntz;
-    l.a.ncol = ntz * ntx;
+    l.a.ntz = z_tiles(c, l.k);
+    l.a.ncol = columns(c, l.k);
     int per_sm = 0, dev = 0, sms = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, l.k.fn, l.k.threads, l.k.smem));
     CK(cudaGetDevice(&dev));
@@ -627,13 +638,12 @@ void plan_loop(fwi_ctx *c, L &l, int n)
     // before at four planes at least, and in practice at about twelve
     const int steps = std::max(1, (c->nyy - 8) / 12);
     LoopProgress &p = l.a.prog;
-    p.ring = c->nyy / 4 + 3;
+    p.ring = progress_ring(c);
     // one shot after the other keeps its fields in L2 as far as they fit; as
     // many side by side as it takes to occupy the GPU
     p.shots = std::min(n, std::max(1, (ctas + l.a.ncol * steps - 1) / (l.a.ncol * steps)));
     l.grid = dim3(std::min<long long>(ctas, (long long)p.shots * l.a.ncol * (c->nyy / 4 + 1)));
-    c->ticket.ensure(1);
-    c->progress.ensure((size_t)n * p.ring * l.a.ncol * kCounterStride);
+    reserve_progress(c, n, l.a.ncol);
     p.ticket = c->ticket.p;
     p.done = c->progress.p;
 }
@@ -919,6 +929,7 @@ void migrate_impl(fwi_ctx *c, const int *shots, int nshots, const float *data, b
             }
         }
         bool sums = use_loop_sums(c);
+        reserve_progress(c, c->B, std::max(columns(c, k), columns(c, fwd_kernel(tuned_fwd(c), false))));
         for (bool done = false; !done; sums = false) {
             start_forward(c, n);
             forward_loop(c, n, false);
