@@ -267,6 +267,7 @@ struct fwi_ctx {
     fwi_params p{};
     int nzz = 0, nxx = 0, nyy = 0, ldz = 0;
     long long vol = 0;  // elements of one pitched field
+    long long rows() const { return (long long)nxx * nyy; }  // z rows of one field
     float idh2 = 0, idh3 = 0;
     int tlag = 0, nsteps = 0;
     int B = 1;  // batch capacity
@@ -361,6 +362,9 @@ int grid_blocks(long long n, int threads = 256)
     long long b = (n + threads - 1) / threads;
     return (int)std::max(1LL, std::min(b, 148LL * 16));
 }
+
+// For the kernels built on for_cells: 8 warps a block, a warp to a z row.
+int row_blocks(long long rows) { return grid_blocks(rows, 8); }
 
 void check_status(fwi_ctx *c)
 {
@@ -774,7 +778,7 @@ void fold_loop_sums(fwi_ctx *c, int n)
     for (int q = 0; q < 2; ++q)
         check_loop_sums_kernel<<<grid_blocks(n * box.size() / 4), 256, 0, c->stream>>>(c->loop_sums.p + q * to_illum,
                                                                                       n * box.size(), c->over.p);
-    dim3 grid(grid_blocks(n * box.size()), 2);
+    dim3 grid(row_blocks((long long)n * box.nx() * box.ny()), 2);
     fold_loop_sums_kernel<<<grid, 256, 0, c->stream>>>(c->loop_sums.p, to_illum, box.ld(), box.nx(), box.ny(), n,
                                                        c->acc_img.p, c->acc_ill.p, start, c->vol, c->ldz, c->nxx,
                                                        c->over.p);
@@ -847,8 +851,8 @@ void update_coeff(fwi_ctx *c)
     if (c->vc.n < n) {
         c->vc.ensure(n);
     }
-    coeff_kernel<<<grid_blocks((long long)n), 256, 0, c->stream>>>(c->vp.p, c->vc.p, c->nzz, c->nxx, c->nyy, c->ldz,
-                                                                   c->vel_slots, c->p.dt * c->p.dt * c->idh2);
+    coeff_kernel<<<row_blocks(c->rows() * c->vel_slots), 256, 0, c->stream>>>(
+        c->vp.p, c->vc.p, c->nzz, c->nxx, c->nyy, c->ldz, c->vel_slots, c->p.dt * c->p.dt * c->idh2);
     CK(cudaGetLastError());
     ++c->launches;
 }
@@ -1208,8 +1212,8 @@ float device_max_abs(fwi_ctx *c, const float *v, long long n)
 {
     c->ubits.ensure(1);
     CK(cudaMemsetAsync(c->ubits.p, 0, sizeof(unsigned), c->stream));
-    max_abs_kernel<<<grid_blocks(n), 256, 0, c->stream>>>(v, c->nzz, c->nxx, (int)(n / (c->ldz * (long long)c->nxx)),
-                                                          c->ldz, c->ubits.p);
+    max_abs_kernel<<<row_blocks(n / c->ldz), 256, 0, c->stream>>>(
+        v, c->nzz, c->nxx, (int)(n / (c->ldz * (long long)c->nxx)), c->ldz, c->ubits.p);
     CK(cudaGetLastError());
     unsigned bits = 0;
     CK(cudaMemcpyAsync(&bits, c->ubits.p, sizeof bits, cudaMemcpyDeviceToHost, c->stream));
@@ -1514,8 +1518,8 @@ int fwi_set_velocity(fwi_ctx *c, const float *vp)
     if (!c || !vp) return FWI_ERR_ARG;
     return guarded(c, [&] {
         stage_velocity(c, vp, (size_t)c->g.nz * c->g.nx * c->g.ny);
-        pad_edges_kernel<<<grid_blocks(c->vol), 256, 0, c->stream>>>(c->stage.p, c->g.nz, c->g.nx, c->g.ny, c->g.nb,
-                                                                     c->nzz, c->nxx, c->nyy, c->ldz, c->vp.p);
+        pad_edges_kernel<<<row_blocks(c->rows()), 256, 0, c->stream>>>(c->stage.p, c->g.nz, c->g.nx, c->g.ny, c->g.nb,
+                                                                       c->nzz, c->nxx, c->nyy, c->ldz, c->vp.p);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(c->vp_clean.p, c->vp.p, c->vol * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -1530,8 +1534,8 @@ int fwi_set_padded_velocity(fwi_ctx *c, const float *vpp)
     if (!c || !vpp) return FWI_ERR_ARG;
     return guarded(c, [&] {
         stage_velocity(c, vpp, (size_t)c->nzz * c->nxx * c->nyy);
-        dense_to_pitched_kernel<<<grid_blocks(c->vol), 256, 0, c->stream>>>(c->stage.p, c->nzz, c->nxx, c->nyy,
-                                                                            c->ldz, c->vp.p);
+        dense_to_pitched_kernel<<<row_blocks(c->rows()), 256, 0, c->stream>>>(c->stage.p, c->nzz, c->nxx, c->nyy,
+                                                                              c->ldz, c->vp.p);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(c->vp_clean.p, c->vp.p, c->vol * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -1547,8 +1551,8 @@ int fwi_get_padded_velocity(fwi_ctx *c, float *vpp)
     return guarded(c, [&] {
         const size_t n = (size_t)c->nzz * c->nxx * c->nyy;
         c->stage.ensure(n);
-        pitched_to_dense_kernel<<<grid_blocks(n), 256, 0, c->stream>>>(c->vp.p, c->nzz, c->nxx, c->nyy, c->ldz,
-                                                                       c->stage.p);
+        pitched_to_dense_kernel<<<row_blocks(c->rows()), 256, 0, c->stream>>>(c->vp.p, c->nzz, c->nxx, c->nyy, c->ldz,
+                                                                              c->stage.p);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(vpp, c->stage.p, n * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -1735,8 +1739,8 @@ int fwi_get_accumulators(fwi_ctx *c, float *img, float *ill)
         const float *srcs[2] = {c->acc_img.p, c->acc_ill.p};
         for (int q = 0; q < 2; ++q) {
             if (!outs[q]) continue;
-            pitched_to_dense_kernel<<<grid_blocks(n), 256, 0, c->stream>>>(srcs[q], c->nzz, c->nxx, c->nyy, c->ldz,
-                                                                           c->post.p);
+            pitched_to_dense_kernel<<<row_blocks(c->rows()), 256, 0, c->stream>>>(srcs[q], c->nzz, c->nxx, c->nyy, c->ldz,
+                                                                                  c->post.p);
             CK(cudaGetLastError());
             CK(cudaMemcpyAsync(outs[q], c->post.p, n * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
             CK(cudaStreamSynchronize(c->stream));
@@ -1755,8 +1759,8 @@ int fwi_get_accumulators_dev(fwi_ctx *c, float *d_img, float *d_ill)
         const float *srcs[2] = {c->acc_img.p, c->acc_ill.p};
         for (int q = 0; q < 2; ++q) {
             if (!outs[q]) continue;
-            pitched_to_dense_kernel<<<grid_blocks(n), 256, 0, c->stream>>>(srcs[q], c->nzz, c->nxx, c->nyy, c->ldz,
-                                                                           outs[q]);
+            pitched_to_dense_kernel<<<row_blocks(c->rows()), 256, 0, c->stream>>>(srcs[q], c->nzz, c->nxx, c->nyy, c->ldz,
+                                                                                  outs[q]);
             CK(cudaGetLastError());
             c->launches += 1;
         }
@@ -1774,8 +1778,8 @@ int fwi_set_accumulators_dev(fwi_ctx *c, const float *d_img, const float *d_ill)
         float *dsts[2] = {c->acc_img.p, c->acc_ill.p};
         for (int q = 0; q < 2; ++q) {
             if (!ins[q]) continue;
-            dense_to_pitched_kernel<<<grid_blocks(c->vol), 256, 0, c->stream>>>(ins[q], c->nzz, c->nxx, c->nyy,
-                                                                                c->ldz, dsts[q]);
+            dense_to_pitched_kernel<<<row_blocks(c->rows()), 256, 0, c->stream>>>(ins[q], c->nzz, c->nxx, c->nyy,
+                                                                                  c->ldz, dsts[q]);
             CK(cudaGetLastError());
             c->launches += 1;
         }
@@ -1790,8 +1794,8 @@ int fwi_rtm_image(fwi_ctx *c, float *image)
         fold_accumulators(c);
         const long long n = (long long)c->g.nz * c->g.nx * c->g.ny;
         c->post.ensure(std::max<size_t>(n, (size_t)c->nzz * c->nxx * c->nyy));
-        rtm_image_kernel<<<grid_blocks(n), 256, 0, c->stream>>>(c->acc_img.p, c->acc_ill.p, c->g.nz, c->g.nx, c->g.ny,
-                                                                c->g.nb, c->nxx, c->ldz, c->idh2, c->post.p);
+        rtm_image_kernel<<<row_blocks((long long)c->g.nx * c->g.ny), 256, 0, c->stream>>>(
+            c->acc_img.p, c->acc_ill.p, c->g.nz, c->g.nx, c->g.ny, c->g.nb, c->nxx, c->ldz, c->idh2, c->post.p);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(image, c->post.p, n * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -1809,9 +1813,9 @@ int fwi_gradient_post(fwi_ctx *c, float zmask, float *grad, float *gmax)
         c->ubits.ensure(1);
         CK(cudaMemsetAsync(c->ubits.p, 0, sizeof(unsigned), c->stream));
         const int imask = (int)(zmask / c->g.dh);
-        grad_post_kernel<<<grid_blocks(n), 256, 0, c->stream>>>(c->acc_img.p, c->acc_ill.p, c->g.nz, c->g.nx, c->g.ny,
-                                                                c->g.nb, c->nxx, c->ldz, c->idh2, imask, c->post.p,
-                                                                c->ubits.p);
+        grad_post_kernel<<<row_blocks((long long)c->g.nx * c->g.ny), 256, 0, c->stream>>>(
+            c->acc_img.p, c->acc_ill.p, c->g.nz, c->g.nx, c->g.ny, c->g.nb, c->nxx, c->ldz, c->idh2, imask, c->post.p,
+            c->ubits.p);
         scale_by_inverse_kernel<<<grid_blocks(n), 256, 0, c->stream>>>(c->post.p, n, c->ubits.p);
         CK(cudaGetLastError());
         c->launches += 2;
