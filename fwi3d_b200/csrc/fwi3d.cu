@@ -1188,12 +1188,28 @@ BlobSet make_blobs(BlobKey k)
     return out;
 }
 
-// Uploads a velocity model into `stage` and checks it there: every value a
-// positive number; the range goes to vmin, vmax.  The context's model does not
-// change before the check has passed.
+// Models below this size are checked on the host: the GPU takes 20 us to answer,
+// the host 3 ns a value.
+constexpr size_t kHostCheck = 15000;
+
+// Uploads a velocity model into `stage` and checks it: every value a positive
+// number; the range goes to vmin, vmax.  The context's model does not change
+// before the check has passed.
 void stage_velocity(fwi_ctx *c, const float *vp, size_t n)
 {
     c->stage.ensure(n);
+    if (n < kHostCheck) {
+        float lo = INFINITY, hi = 0.0f;
+        for (size_t i = 0; i < n; ++i) {
+            if (!std::isfinite(vp[i]) || vp[i] <= 0) fail(FWI_ERR_NUMERIC, "velocity[%zu] = %g is not a positive number", i, vp[i]);
+            lo = std::min(lo, vp[i]);
+            hi = std::max(hi, vp[i]);
+        }
+        CK(cudaMemcpyAsync(c->stage.p, vp, n * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+        c->vmin = lo;
+        c->vmax = hi;
+        return;
+    }
     c->vrange.ensure(1);
     VelocityRange r{~0ull, 0x7f800000u, 0u};
     CK(cudaMemcpyAsync(c->stage.p, vp, n * sizeof(float), cudaMemcpyHostToDevice, c->stream));
