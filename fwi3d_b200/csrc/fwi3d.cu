@@ -1115,7 +1115,7 @@ std::vector<float> poisson_points(float xm, float ym, float zm, float r, const f
         }
     };
     std::mt19937_64 ahead = rng;
-    auto cur = std::make_unique<Chunk>(), next = std::make_unique<Chunk>();
+    std::unique_ptr<Chunk> cur(new Chunk), next;  // (not cleared)
     std::future<void> filling;
     int used = 0;
     long long picks = 0;
@@ -1130,6 +1130,7 @@ std::vector<float> poisson_points(float xm, float ym, float zm, float r, const f
             }
             picks += cur->n;
             if (picks >= kPicks) {
+                if (!next) next.reset(new Chunk);
                 next->n = kPicks;
                 filling = std::async(std::launch::async, fill, next.get(), &ahead);
             }
