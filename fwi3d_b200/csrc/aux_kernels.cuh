@@ -294,8 +294,8 @@ __device__ __forceinline__ float4 load4(const float *__restrict__ p, long long q
 // what counts is bytes in flight: each thread has kQuads independent quads of
 // both inputs outstanding.  45.6 M residual samples with the residual stored:
 // the whole call takes 0.101 ms (0.160 ms with scalar loads, two blocks per SM,
-// a second launch for the total and a copy of it).  The order of the sum depends on n and the grid alone, not on the
-// alignment.
+// a second launch for the total and a copy of it).  The order of the sum depends
+// on n and the grid alone, not on the alignment.
 constexpr int kQuads = 4;
 
 // res = obs - cal (FP32, as the reference stores it) and sum(res^2) in FP64

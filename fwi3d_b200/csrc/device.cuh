@@ -365,24 +365,4 @@ __device__ __forceinline__ int pad_depth(int i, int n, int nb)
     return i < nb ? i : (i >= n - nb ? n - 1 - i : -1);
 }
 
-// Cerjan factor of a cell from the 1-D table, bit-identical to the reference's
-// b2d/b3d tables (src/modeling/modeling.cu:101-127): the 2-D entry is
-// (b1[a] + b1[b]) - 1 and the 3-D entry ((B(z,x) + B(x,y)) + B(z,y)) - 5 with
-// B(p,q) = b1[p] + b1[q], all in FP32 in that order.
-__device__ __forceinline__ float cerjan(const float *b1, int dz, int dx, int dy)
-{
-    const int n = (dz >= 0) + (dx >= 0) + (dy >= 0);
-    if (n == 0) return 1.0f;
-    if (n == 1) return b1[dz >= 0 ? dz : (dx >= 0 ? dx : dy)];
-    if (n == 2) {
-        const int u = dz >= 0 ? dz : dx;
-        const int v = dy >= 0 ? dy : dx;
-        return __fsub_rn(__fadd_rn(b1[u], b1[v]), 1.0f);
-    }
-    const float bzx = __fadd_rn(b1[dz], b1[dx]);
-    const float bxy = __fadd_rn(b1[dx], b1[dy]);
-    const float bzy = __fadd_rn(b1[dz], b1[dy]);
-    return __fsub_rn(__fadd_rn(__fadd_rn(bzx, bxy), bzy), 5.0f);
-}
-
 }  // namespace fwi
