@@ -1410,6 +1410,14 @@ int fwi_tile_shape(int tile, int *tz, int *tx)
     return FWI_OK;
 }
 
+int fwi_backward_tile_shape(int tile, int *tz, int *tx)
+{
+    if (tile < 0 || tile >= kNumTiles || !tz || !tx) return FWI_ERR_ARG;
+    *tz = 4 * kBwdTiles[tile].tz4;
+    *tx = kBwdTiles[tile].tx;
+    return FWI_OK;
+}
+
 int fwi_create(const fwi_grid *grid, const fwi_params *params, fwi_ctx **out)
 {
     if (!grid || !params || !out) return FWI_ERR_ARG;

@@ -93,6 +93,7 @@ SIGNATURES = {
     "fwi_autotune": (_i, [_p]),
     "fwi_num_tiles": (_i, [_ip]),
     "fwi_tile_shape": (_i, [_i, _ip, _ip]),
+    "fwi_backward_tile_shape": (_i, [_i, _ip, _ip]),
 }
 
 
@@ -513,13 +514,15 @@ def residual_noalloc(d_obs: int, d_cal: int, n: int, d_res: int, d_sum_sq: int, 
         raise FwiError(st, "fwi_residual_noalloc failed (n above NOALLOC_MAX_N or a CUDA error)")
 
 
-def tile_table() -> list[tuple[int, int]]:
+def tile_table(backward: bool = False) -> list[tuple[int, int]]:
+    """Shapes (z cells, x rows) of the forward or the backward kernel's tiles."""
     lib = load()
+    shape = lib.fwi_backward_tile_shape if backward else lib.fwi_tile_shape
     n = C.c_int()
     lib.fwi_num_tiles(C.byref(n))
     out = []
     for t in range(n.value):
         tz, tx = C.c_int(), C.c_int()
-        lib.fwi_tile_shape(t, C.byref(tz), C.byref(tx))
+        shape(t, C.byref(tz), C.byref(tx))
         out.append((tz.value, tx.value))
     return out

@@ -22,6 +22,9 @@
  *   - One context per host thread; calls on one context are not re-entrant.
  *     Each context owns one CUDA stream (or uses the one set with
  *     fwi_set_stream).
+ *   - The time loop of a batch of shots is one kernel on all SMs, for
+ *     milliseconds to minutes.  Work on other streams of the GPU, other contexts'
+ *     included, runs before or after it.
  *   - The library keeps per-device state for the life of the process (kernel
  *     attributes, grid sizes, the no-alloc scratch address); cudaDeviceReset
  *     while it is loaded is not supported.
@@ -270,14 +273,15 @@ int fwi_last_timing(fwi_ctx *ctx, float *fwd_ms, float *bwd_ms);
 /* Kernel launches issued by the library since creation (the time loop of a
  * batch is one launch). */
 int fwi_launch_count(fwi_ctx *ctx, int64_t *count);
-/* Stencil tile chosen by the autotuner for the forward and backward kernels
- * (index into the compiled tile table; -1 = not tuned yet). */
+/* Stencil tiles chosen by the autotuner for the forward and backward kernels
+ * (indices into their tables of fwi_num_tiles() shapes; -1 = not tuned yet). */
 int fwi_get_tiles(fwi_ctx *ctx, int *fwd_tile, int *bwd_tile);
 int fwi_set_tiles(fwi_ctx *ctx, int fwd_tile, int bwd_tile);
 int fwi_autotune(fwi_ctx *ctx);
 int fwi_num_tiles(int *n);
-/* Cells of a forward tile (the backward kernel has shapes of its own). */
+/* Cells of a tile of the forward and of the backward kernel. */
 int fwi_tile_shape(int tile, int *tz, int *tx);
+int fwi_backward_tile_shape(int tile, int *tz, int *tx);
 
 #ifdef __cplusplus
 }
