@@ -526,8 +526,8 @@ __device__ __forceinline__ void loop_publisher(LoopShared<NW> &sh, const LoopGeo
 //       that are never updated, which keeps those cells at 0.
 // Bound: shared-memory wavefronts (70 % of the L1 pipe: 10 halo rows read for
 // 8 cells) together with HBM.  301^3 cells, random pad, one shot, per step:
-// 86.5 us as one launch per step with a register queue per cell, 60.1 us now;
-// 13.3 bytes per cell from HBM instead of 14.9, since a plane that one step
+// 86.1 us as one launch per step with a register queue per cell, 60.7 us now;
+// 13.7 bytes per cell from HBM instead of 14.9, since a plane that one step
 // stores is often still in L2 when the next reads it; 16 bytes per cell at the
 // 6.55 TB/s of a copy take 67 us.  Small grids were bound by the launches and
 // by few planes per CTA: 56 x 60 x 58 cells with the Cerjan pad 29 us, now 6.2 us.
@@ -806,11 +806,11 @@ __global__ void __launch_bounds__(Loop<T, 1>::THREADS, CTAS)
 // 14 loads per 4 cells (301^3 cells, 4 shots: 0.694 ms per step, by field
 // 0.665, with the accumulators out of shared memory 0.573 and the ring that
 // this makes room for 0.543).
-// Bound: HBM.  301^3 cells, random pad, one shot: 32.8 bytes per cell and step
+// Bound: HBM.  301^3 cells, random pad, one shot: 32.1 bytes per cell and step
 // at 6.5 TB/s, the rate of a copy (the old levels and the coefficients arrive
 // in 148 x 8 boxes, the halos of the two fields are read 2.1 times, from L2).
 // 185 us per step as one launch per step, 136 us now; 88^3 cells,
-// 4 shots: 35 and 11.7 us.
+// 4 shots: 35 and 12.1 us.
 // ---------------------------------------------------------------------------
 struct BwdMaps {
     CUtensorMap mhs[2], mhr[2], mcs[2], mcr[2], mv;
