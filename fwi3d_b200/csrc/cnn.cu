@@ -653,15 +653,18 @@ __global__ void __launch_bounds__(wg::THREADS, wg::CTAS_PER_SM)
 // Fixed-order sums of the per-CTA partials of a layer's weight and bias
 // gradients, times `scale`: out[i] = scale * sum_b part[b][i].  A block is 32
 // entries x 8 slices of b; slice y sums b = y, y+8, ... in order, then the
-// eight slice sums are added in order.  The last block has the biases.
+// eight slice sums are added in order.  The last block has the biases.  *status:
+// what g_cnn_status says after the kernels before; a copy, since another network's
+// call may raise or clear it while the step goes on.
 constexpr int RED_X = 32, RED_Y = 8;
 constexpr int RED_WBLOCKS = (WSZ + RED_X - 1) / RED_X;
 
 __global__ void __launch_bounds__(RED_X * RED_Y)
     reduce_partials_kernel(const float *__restrict__ wpart, const float *__restrict__ bpart, int nb, float scale,
-                           float *__restrict__ gw, float *__restrict__ gb)
+                           float *__restrict__ gw, float *__restrict__ gb, unsigned *__restrict__ status)
 {
     __shared__ float red[RED_Y][RED_X];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *status = *(volatile unsigned int *)&g_cnn_status;
     const bool weights = blockIdx.x < RED_WBLOCKS;
     const float *part = weights ? wpart : bpart;
     float *out = weights ? gw : gb;
@@ -759,8 +762,8 @@ __global__ void sum_f64_kernel(const double *__restrict__ p, int n, double *__re
 // Adam on the FP32 master weights (Kingma & Ba, 2015), then the BF16 copies:
 // forward layout [t][co][ci] and the data-gradient layout [t][ci][co].  The
 // mask keeps the padding channels of the first and last layer at zero.  One
-// launch updates every layer (blockIdx.y); it changes nothing once a kernel of
-// the step has given up a wait.
+// launch updates every layer (blockIdx.y), or none once a wait of the step has
+// given up.
 struct AdamLayer {
     float *w, *gw, *mw, *vw, *mask, *b, *gb, *mb, *vb;
     __nv_bfloat16 *wb, *wt;
@@ -768,12 +771,13 @@ struct AdamLayer {
 };
 struct AdamArgs {
     AdamLayer layer[NL];
+    const unsigned *status;
     float lr, b1, b2, eps, c1, c2;
 };
 
 __global__ void adam_kernel(const __grid_constant__ AdamArgs a)
 {
-    if (*(volatile unsigned int *)&g_cnn_status) return;
+    if (*a.status) return;
     const AdamLayer &l = a.layer[blockIdx.y];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < WSZ) {
@@ -822,6 +826,11 @@ struct Buf {
 
 }  // namespace
 
+struct StepResult {
+    double sum;       // of squares, the loss
+    unsigned status;  // see reduce_partials_kernel
+};
+
 struct fwi_cnn {
     Geo g{};
     cudaStream_t stream = nullptr;
@@ -832,7 +841,8 @@ struct fwi_cnn {
     Buf<__nv_bfloat16> act[NL];  // act[0] input, act[l] = output of layer l-1 (l = 1..3)
     Buf<__nv_bfloat16> dg[2];    // data gradients, ping-pong
     Buf<float> pred, partial, bpartial;
-    Buf<double> lpart, lsum;
+    Buf<double> lpart;
+    Buf<StepResult> result;
     int adam_step = 0;
     std::string err;
 };
@@ -1023,7 +1033,7 @@ int launch_wgrad(fwi_cnn *n, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, fl
     wgrad_tc_kernel<<<grid, wg::THREADS, wg::SMEM, n->stream>>>(mx, mdy, a);
     CNN_CK(cudaGetLastError());
     reduce_partials_kernel<<<RED_WBLOCKS + 1, RED_X * RED_Y, 0, n->stream>>>(n->partial.p, n->bpartial.p, grid, scale,
-                                                                            gw, gb);
+                                                                            gw, gb, &n->result.p->status);
     CNN_CK(cudaGetLastError());
     return FWI_OK;
 }
@@ -1063,7 +1073,7 @@ int ensure_volume(fwi_cnn *n, int nz, int nx, int ny)
     CNN_CK(n->gw.ensure((size_t)NL * WSZ));
     CNN_CK(n->gb.ensure((size_t)NL * CH));
     CNN_CK(n->lpart.ensure(1024));
-    CNN_CK(n->lsum.ensure(1));
+    CNN_CK(n->result.ensure(1));
     return FWI_OK;
 }
 
@@ -1151,7 +1161,7 @@ int fwi_cnn_destroy(fwi_cnn *n)
     n->partial.release();
     n->bpartial.release();
     n->lpart.release();
-    n->lsum.release();
+    n->result.release();
     delete n;
     return FWI_OK;
 }
@@ -1233,7 +1243,7 @@ int fwi_cnn_train_step(fwi_cnn *n, int nz, int nx, int ny, const float *d_in, co
     // by V (loss scaling) and scaled back in the weight gradients
     const int lblk = 1024;
     mse_kernel<<<lblk, 256, 0, n->stream>>>(g, n->pred.p, d_target, 1.0f, n->dg[0].p, n->lpart.p);
-    sum_f64_kernel<<<1, 32, 0, n->stream>>>(n->lpart.p, lblk, n->lsum.p);
+    sum_f64_kernel<<<1, 32, 0, n->stream>>>(n->lpart.p, lblk, &n->result.p->sum);
     // (d, not d/V: the parameter gradients are scaled by 1/V as they are summed)
     const float inv = 1.0f / (float)V;
     int cur = 0;
@@ -1251,6 +1261,7 @@ int fwi_cnn_train_step(fwi_cnn *n, int nz, int nx, int ny, const float *d_in, co
     if (lr > 0) {
         const int step = n->adam_step + 1;
         AdamArgs a;
+        a.status = &n->result.p->status;
         a.lr = lr;
         a.b1 = 0.9f;
         a.b2 = 0.999f;
@@ -1263,8 +1274,8 @@ int fwi_cnn_train_step(fwi_cnn *n, int nz, int nx, int ny, const float *d_in, co
         adam_kernel<<<dim3((WSZ + 255) / 256, NL), 256, 0, n->stream>>>(a);
     }
     CNN_CK(cudaGetLastError());
-    double lsum = 0.0;
-    CNN_CK(cudaMemcpyAsync(&lsum, n->lsum.p, sizeof(double), cudaMemcpyDeviceToHost, n->stream));
+    StepResult r{};
+    CNN_CK(cudaMemcpyAsync(&r, n->result.p, sizeof r, cudaMemcpyDeviceToHost, n->stream));
     if (grad_w)
         CNN_CK(cudaMemcpyAsync(grad_w, n->gw.p, (size_t)NL * WSZ * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
     if (grad_b)
@@ -1272,8 +1283,12 @@ int fwi_cnn_train_step(fwi_cnn *n, int nz, int nx, int ny, const float *d_in, co
     CNN_CK(cudaStreamSynchronize(n->stream));
     st = check_cnn_status(n);
     if (st != FWI_OK) return st;
+    if (r.status) {  // cleared by another network's call, whose wait it may have been
+        n->err = "convolution kernel: a bounded wait gave up";
+        return FWI_ERR_TIMEOUT;
+    }
     if (lr > 0) ++n->adam_step;
-    if (loss) *loss = 0.5 * lsum / (double)V;
+    if (loss) *loss = 0.5 * r.sum / (double)V;
     return FWI_OK;
 }
 
