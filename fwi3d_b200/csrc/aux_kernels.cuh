@@ -123,25 +123,31 @@ __global__ void start_source_kernel(float *__restrict__ A, long long vol, int ld
 // src/inversion/inversion.cu:385-398), in receiver order, which keeps it
 // deterministic where the reference uses atomicAdd.  Data [R][nt] -> [nt][ncell]
 // in the order of the cell lists, 32x32 tiles through shared memory; the
-// receivers of cell u are rid[first[u]] .. rid[first[u+1]-1].
+// receivers of cell u are rid[first[u]] .. rid[first[u+1]-1].  A grid has 65535
+// blocks along the times, which go on beyond 2097120 of them.
 // ---------------------------------------------------------------------------
 __global__ void gather_data_kernel(const float *__restrict__ in, int nt, int ncell, const int *__restrict__ first,
                                    const int *__restrict__ rid, float idh3, float *__restrict__ out)
 {
     __shared__ float tile[32][33];
-    const int u0 = blockIdx.x * 32, t0 = blockIdx.y * 32;
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int u = u0 + k, t = t0 + threadIdx.x;
-        if (u < ncell && t < nt) {
-            float v = 0.0f;
-            for (int q = first[u]; q < first[u + 1]; ++q) v += idh3 * in[(long long)rid[q] * nt + t];
-            tile[k][threadIdx.x] = v;
+    const int u0 = blockIdx.x * 32;
+    for (long long t0 = blockIdx.y * 32; t0 < nt; t0 += gridDim.y * 32) {
+        for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+            const long long t = t0 + threadIdx.x;
+            const int u = u0 + k;
+            if (u < ncell && t < nt) {
+                float v = 0.0f;
+                for (int q = first[u]; q < first[u + 1]; ++q) v += idh3 * in[(long long)rid[q] * nt + t];
+                tile[k][threadIdx.x] = v;
+            }
         }
-    }
-    __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int t = t0 + k, u = u0 + threadIdx.x;
-        if (u < ncell && t < nt) out[(long long)t * ncell + u] = tile[threadIdx.x][k];
+        __syncthreads();
+        for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+            const long long t = t0 + k;
+            const int u = u0 + threadIdx.x;
+            if (u < ncell && t < nt) out[t * ncell + u] = tile[threadIdx.x][k];
+        }
+        __syncthreads();
     }
 }
 

@@ -834,7 +834,7 @@ void seis_to_fortran(fwi_ctx *c, int ncell, float *dst)
 // Fortran per shot [R][nt] at src (device) -> adjoint sources of the receiver cells.
 void data_from_fortran(fwi_ctx *c, int ncell, const float *src, cudaStream_t st = nullptr)
 {
-    dim3 grid((ncell + 31) / 32, (c->p.nt + 31) / 32);
+    dim3 grid((ncell + 31) / 32, std::min((c->p.nt + 31) / 32, 65535));
     gather_data_kernel<<<grid, dim3(32, 8), 0, st ? st : c->stream>>>(src, c->p.nt, ncell, c->inj_first.p,
                                                                       c->inj_rid.p, c->idh3, c->data_tm.p);
     CK(cudaGetLastError());
