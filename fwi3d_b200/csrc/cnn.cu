@@ -1281,9 +1281,11 @@ int fwi_cnn_train_step(fwi_cnn *n, int nz, int nx, int ny, const float *d_in, co
     if (grad_b)
         CNN_CK(cudaMemcpyAsync(grad_b, n->gb.p, (size_t)NL * CH * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
     CNN_CK(cudaStreamSynchronize(n->stream));
-    st = check_cnn_status(n);
-    if (st != FWI_OK) return st;
-    if (r.status) {  // cleared by another network's call, whose wait it may have been
+    // the copy that the weights went by: what g_cnn_status says by now can be
+    // another network's
+    if (r.status) {
+        st = check_cnn_status(n);
+        if (st != FWI_OK) return st;
         n->err = "convolution kernel: a bounded wait gave up";
         return FWI_ERR_TIMEOUT;
     }
