@@ -1070,8 +1070,6 @@ int ensure_volume(fwi_cnn *n, int nz, int nx, int ny)
     CNN_CK(n->pred.ensure(g.V));
     CNN_CK(n->partial.ensure((size_t)kMaxPartials * WSZ));
     CNN_CK(n->bpartial.ensure((size_t)kMaxPartials * CH));
-    CNN_CK(n->gw.ensure((size_t)NL * WSZ));
-    CNN_CK(n->gb.ensure((size_t)NL * CH));
     CNN_CK(n->lpart.ensure(1024));
     CNN_CK(n->result.ensure(1));
     return FWI_OK;
@@ -1108,6 +1106,7 @@ int fwi_cnn_create(uint64_t seed, fwi_cnn **out)
     fwi_cnn *n = new fwi_cnn();
     std::mt19937_64 rng(seed);
     int st = FWI_OK;
+    if (n->gw.ensure((size_t)NL * WSZ) != cudaSuccess || n->gb.ensure((size_t)NL * CH) != cudaSuccess) st = FWI_ERR_ALLOC;
     for (int l = 0; l < NL && st == FWI_OK; ++l) {
         // He initialisation over the real fan-in, zero on padding channels
         std::normal_distribution<float> N(0.0f, std::sqrt(2.0f / (TAPS * CIN[l])));
