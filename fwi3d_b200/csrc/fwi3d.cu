@@ -1310,12 +1310,16 @@ void pad_slot(fwi_ctx *c, const fwi_rbc *rbc, uint64_t seed, int slot)
     d.ensure(bs.size());
     CK(cudaMemcpyAsync(d.p, bs.data(), bs.size() * sizeof(Blob), cudaMemcpyHostToDevice, c->stream));
     // bricks of 16 x 16 rows, or of 8 x 8 where those would not occupy the GPU
-    // (88^3 cells: 0.98 -> 0.43 ms a call)
+    // (88^3 cells: 0.98 -> 0.43 ms a call), or of 4 x 4 where there would not be
+    // two for every SM (the kernel on 20^3 and 56^3 cells: 13.0 and 41.2 us with 8 x 8,
+    // 5.5 and 15.6 with 4 x 4; 5.3 and 23.5 with a thread per cell)
     int edge = 16;
     auto bricks = [&] {
         return dim3((c->nzz + kBrickZ - 1) / kBrickZ, (c->nxx + edge - 1) / edge, (c->nyy + edge - 1) / edge);
     };
-    if ((long long)bricks().x * bricks().y * bricks().z < 8 * 148) edge = 8;
+    auto count = [&] { return (long long)bricks().x * bricks().y * bricks().z; };
+    if (count() < 8 * 148) edge = 8;
+    if (count() < 2 * 148) edge = 4;
     rbc_blobs_kernel<<<bricks(), kBrickThreads, 0, c->stream>>>(dst, c->nzz, c->nxx, c->nyy, c->ldz, c->g.nb, c->g.dh,
                                                                 d.p, (int)bs.size(), vlo, vhi, edge, edge);
     CK(cudaGetLastError());
