@@ -16,15 +16,18 @@ namespace fwi {
 // 732 us.  Rows shorter than a warp leave lanes idle, which costs less than
 // the divisions (88^3 cells: no difference), given a grid by rows: with one by
 // cells, warps took several short rows in turn (image of 5^3 cells, the call:
-// 32 us, 23 now).
-template <class F>
+// 32 us, 23 now).  LANES 256: a block to a row, for few and long rows, where the
+// passes of a warp over its row wait for one another (image kernel, 500 x 16 x 16
+// cells: 14.5 us with warps, 4.1 with blocks; 4.0 with a thread per cell).  Parts of
+// rows to a warp take a division more (201^3 cells: 33 us, 48 with it).
+template <int LANES = 32, class F>
 __device__ __forceinline__ void for_cells(int nz, int nx, int ny, F f)
 {
-    const long long rows = (long long)nx * ny, step = (long long)gridDim.x * (blockDim.x / 32);
-    for (long long r = blockIdx.x * (long long)(blockDim.x / 32) + threadIdx.x / 32; r < rows; r += step) {
+    const long long rows = (long long)nx * ny, step = (long long)gridDim.x * (blockDim.x / LANES);
+    for (long long r = blockIdx.x * (long long)(blockDim.x / LANES) + threadIdx.x / LANES; r < rows; r += step) {
         const int k = (int)(r / nx), j = (int)(r - (long long)k * nx);
 #pragma unroll 4
-        for (int i = threadIdx.x % 32; i < nz; i += 32) f(i, j, k, r);
+        for (int i = threadIdx.x % LANES; i < nz; i += LANES) f(i, j, k, r);
     }
 }
 
@@ -191,11 +194,12 @@ __global__ void scatter_seis_kernel(const float *__restrict__ in, int nt, int nc
 // project defines it as 0.
 __device__ __forceinline__ float ratio(float a, float ill) { return ill != 0.0f ? a / ill : 0.0f; }
 
+template <int LANES>
 __global__ void rtm_image_kernel(const float *__restrict__ img, const float *__restrict__ ill,
                                  int nz, int nx, int ny, int nb, int nxx, int ldz, float idh2,
                                  float *__restrict__ out)
 {
-    for_cells(nz, nx, ny, [&](int i, int j, int k, long long r) {
+    for_cells<LANES>(nz, nx, ny, [&](int i, int j, int k, long long r) {
         float v = 0.0f;
         if (i > 0 && i < nz - 1) {
             const long long p = (i + nb) + (long long)(j + nb) * ldz + (long long)(k + nb) * ldz * nxx;
@@ -212,12 +216,13 @@ __global__ void rtm_image_kernel(const float *__restrict__ img, const float *__r
 // and the running max |g| (src/inversion/inversion.cu:142-165).  max|g| of
 // non-negative floats is taken with an integer atomicMax on their bits, which
 // is exact and order independent.
+template <int LANES>
 __global__ void grad_post_kernel(const float *__restrict__ g, const float *__restrict__ ill, int nz,
                                  int nx, int ny, int nb, int nxx, int ldz, float idh2, int imask,
                                  float *__restrict__ out, unsigned int *__restrict__ gmax_bits)
 {
     float lmax = 0.0f;
-    for_cells(nz, nx, ny, [&](int i, int j, int k, long long r) {
+    for_cells<LANES>(nz, nx, ny, [&](int i, int j, int k, long long r) {
         float v = 0.0f;
         if (i > imask && i < nz - 1) {
             const long long p = (i + nb) + (long long)(j + nb) * ldz + (long long)(k + nb) * ldz * nxx;

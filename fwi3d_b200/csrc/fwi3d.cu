@@ -367,6 +367,10 @@ int grid_blocks(long long n, int threads = 256)
 // For the kernels built on for_cells: 8 warps a block, a warp to a z row.
 int row_blocks(long long rows) { return grid_blocks(rows, 8); }
 
+// Whether a z row should have a block instead: for rows of more than two passes of
+// a warp, of which there are fewer than 8 to an SM.
+bool few_long_rows(int nz, long long rows) { return nz > 64 && rows < 8 * 148; }
+
 void check_status(fwi_ctx *c)
 {
     CK(cudaStreamSynchronize(c->stream));
@@ -1828,7 +1832,9 @@ int fwi_rtm_image(fwi_ctx *c, float *image)
         fold_accumulators(c);
         const long long n = (long long)c->g.nz * c->g.nx * c->g.ny;
         c->post.ensure(std::max<size_t>(n, (size_t)c->nzz * c->nxx * c->nyy));
-        rtm_image_kernel<<<row_blocks((long long)c->g.nx * c->g.ny), 256, 0, c->stream>>>(
+        const long long rows = (long long)c->g.nx * c->g.ny;
+        const bool few = few_long_rows(c->g.nz, rows);
+        (few ? rtm_image_kernel<256> : rtm_image_kernel<32>)<<<few ? (int)rows : row_blocks(rows), 256, 0, c->stream>>>(
             c->acc_img.p, c->acc_ill.p, c->g.nz, c->g.nx, c->g.ny, c->g.nb, c->nxx, c->ldz, c->idh2, c->post.p);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(image, c->post.p, n * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
@@ -1847,7 +1853,9 @@ int fwi_gradient_post(fwi_ctx *c, float zmask, float *grad, float *gmax)
         c->ubits.ensure(1);
         CK(cudaMemsetAsync(c->ubits.p, 0, sizeof(unsigned), c->stream));
         const int imask = (int)(zmask / c->g.dh);
-        grad_post_kernel<<<row_blocks((long long)c->g.nx * c->g.ny), 256, 0, c->stream>>>(
+        const long long rows = (long long)c->g.nx * c->g.ny;
+        const bool few = few_long_rows(c->g.nz, rows);
+        (few ? grad_post_kernel<256> : grad_post_kernel<32>)<<<few ? (int)rows : row_blocks(rows), 256, 0, c->stream>>>(
             c->acc_img.p, c->acc_ill.p, c->g.nz, c->g.nx, c->g.ny, c->g.nb, c->nxx, c->ldz, c->idh2, imask, c->post.p,
             c->ubits.p);
         scale_by_inverse_kernel<<<grid_blocks(n), 256, 0, c->stream>>>(c->post.p, n, c->ubits.p);
