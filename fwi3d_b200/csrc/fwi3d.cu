@@ -1973,12 +1973,12 @@ int fwi_autotune(fwi_ctx *c)
         t.info.ncell = 0;
         upload_batch(c, t);
         update_coeff(c);
-        // Each tile is timed over kSteps steps after a warm launch, in two
+        // Each tile is timed over kSteps steps after a warm launch of a few, in two
         // passes (the SM clock moves under the power cap during a sweep), and
         // keeps its faster pass.  The heuristic default stays unless another
         // beats it by more than 1 %: a short window can favour whatever ran
         // while the clock was high.
-        constexpr int kSteps = 32, kPasses = 2;
+        constexpr int kWarm = 8, kSteps = 32, kPasses = 2;
         cudaEvent_t e0, e1;
         CK(cudaEventCreate(&e0));
         CK(cudaEventCreate(&e1));
@@ -1986,9 +1986,10 @@ int fwi_autotune(fwi_ctx *c)
             float ms[kNumTiles];
             std::fill(ms, ms + kNumTiles, 1e30f);
             auto timed = [&](auto &L) {
-                L.a.nsteps = std::min(kSteps, c->nsteps);
+                L.a.nsteps = std::min(kWarm, c->nsteps);
                 L.a.nt = 0;  // no sources, no adjoint data
                 launch_loop(c, L, c->B);
+                L.a.nsteps = std::min(kSteps, c->nsteps);
                 CK(cudaEventRecord(e0, c->stream));
                 launch_loop(c, L, c->B);
                 CK(cudaEventRecord(e1, c->stream));
